@@ -17,6 +17,7 @@
 // Newton-refined hardware reciprocal instead of five IEEE divisions).  Its kernels
 // live in namespace vx::fast64 and its launcher is launch_fct64_substep_fast.
 #include <cuda_runtime.h>
+#include "div64.cuh"
 #include "fast64.cuh"
 #include "vx_kernels.hpp"
 
@@ -33,54 +34,61 @@ namespace VX_FCT64_NS {
 
 using P64 = PatchT<double>;
 
-// WENO-type upwind face value (Rectangle.cpp:980-1030; identical values to
-// Rectangle.cpp:943-977).  f1..f4 are the four cells left-to-right around the face.
-__device__ __forceinline__ double weno_face(double f1, double f2, double f3, double f4, bool right) {
-    const double c6 = 1.0 / 6;
-    const double c43 = 4.0 / 3;
-    double fL = c6 * (-f1 + 5 * f2 + 2 * f3);
-    double fR = c6 * (2 * f2 + 5 * f3 - f4);
-    double AL = f1 - 2 * f2 + f3;
-    double BL = f3 - f1;
-    double AR = f2 - 2 * f3 + f4;
-    double BR = f4 - f2;
-    double bL = c43 * (AL * AL) + 0.5 * AL * BL + 0.25 * (BL * BL);
-    double bR = c43 * (AR * AR) - 0.5 * AR * BR + 0.25 * (BR * BR);
-    const double mm = 1.0e-10;
-#ifdef VX_FP64_FAST
-    // oL / (oL + oR) with o = 0.5 / (mm + b)^2 is dR^2 / (dL^2 + dR^2), d = mm + b
-    const double dL = mm + bL, dR = mm + bR;
-    double wL = (dR * dR) * rcp_nr(dL * dL + dR * dR);
-    double wR = 1.0 - wL;
-#else
-    double oL = 0.5 / ((mm + bL) * (mm + bL));
-    double oR = 0.5 / ((mm + bR) * (mm + bR));
-    double wL = oL / (oL + oR);
-    double wR = oR / (oL + oR);
-#endif
-    double wL0 = wL * (0.75 + wL * (wL - 0.5));
-    double wR0 = wR * (0.75 + wR * (wR - 0.5));
-    double pick;
-    if (right) pick = (wL0 > wR0) ? wL0 : wR0;
-    else pick = (wL0 < wR0) ? wL0 : wR0;
-#ifdef VX_FP64_FAST
-    double fwl = pick * rcp_nr(wL0 + wR0);
-#else
-    double fwl = pick / (wL0 + wR0);
-#endif
-    double fwr = 1 - fwl;
-    return fwl * fL + fwr * fR;
+// The four cells around a face where the reconstruction needs no weights.
+// 2: all are +0.0, and so is the face value (every term of weno_face is +0.0).
+// 1: every |f| < 1e-14.  The smoothness indicators are then below 27 max|f|^2 < 2.7e-27,
+//    less than half an ulp of the regulariser 1e-10 they are added to, so both sums equal
+//    it, wL = wR = 0.5, the mapped weights are 0.375 and the face weight is 0.375 / 0.75 =
+//    0.5 exactly, whichever way the wind blows.
+// 0: anything else (NaN and infinities included).
+// f is a phase-space density in SI units, 1e46 or so where there is plasma: a thermal
+// distribution falls below 1e-14 at 17 thermal widths, so most of the momentum range of a
+// base patch is on one of the two short paths (4096 x 512, 1 keV: 60 % of it).  A warp is
+// 32 neighbouring p of one row, so whole warps take it: decided with integer compares
+// on the high words, off the FP64 unit that bounds these kernels.
+__device__ __forceinline__ int weno_void(double f1, double f2, double f3, double f4) {
+    const unsigned h1 = (unsigned)__double2hiint(f1), h2 = (unsigned)__double2hiint(f2);
+    const unsigned h3 = (unsigned)__double2hiint(f3), h4 = (unsigned)__double2hiint(f4);
+    constexpr unsigned kTiny = 0x3d06849bu;  // high word of 1e-14 (1e-14 = 0x3d06849b86a12b9b)
+    const unsigned m = max(max(h1 & 0x7fffffffu, h2 & 0x7fffffffu), max(h3 & 0x7fffffffu, h4 & 0x7fffffffu));
+    if (m >= kTiny) return 0;
+    const unsigned any = h1 | h2 | h3 | h4 | (unsigned)__double2loint(f1) | (unsigned)__double2loint(f2) |
+                         (unsigned)__double2loint(f3) | (unsigned)__double2loint(f4);
+    return any == 0 ? 2 : 1;
 }
 
-// Both upwind choices of weno_face at once (the smoothness weights do not depend on the
-// velocity): out_right / out_left are weno_face(..., true) / weno_face(..., false), bit
-// for bit.
-__device__ __forceinline__ void weno_face_both(double f1, double f2, double f3, double f4, double &out_right,
-                                               double &out_left) {
+// a > b and a < b for the mapped weights (positive, or NaN): on the bit patterns, where
+// any NaN makes the face value NaN whichever weight is picked.
+__device__ __forceinline__ bool wgt(double a, double b) {
+    return __double_as_longlong(a) > __double_as_longlong(b);
+}
+
+// WENO-type upwind face value (Rectangle.cpp:980-1030; identical values to
+// Rectangle.cpp:943-977).  f1..f4 are the four cells left-to-right around the face.  The
+// smoothness weights do not depend on the velocity, so both upwind choices come out of one
+// evaluation (BOTH: out_right with the larger mapped weight, out_left with the smaller);
+// otherwise out_right is the choice for `right`.
+// In the FP64 form its quotients go through div64.cuh (the two of a weight pair share a
+// reciprocal): one FP64 instruction of this kernel costs 4.5 us per RK stage on the 4096 x
+// 512 two-level workload, an IEEE division about sixteen of them, a reciprocal three and
+// each quotient three more.
+template <bool BOTH>
+__device__ __forceinline__ void weno_values(double f1, double f2, double f3, double f4, bool right,
+                                            double &out_right, double &out_left) {
+    const int none = weno_void(f1, f2, f3, f4);
+    if (none == 2) {
+        out_right = 0.0;
+        out_left = 0.0;
+        return;
+    }
     const double c6 = 1.0 / 6;
     const double c43 = 4.0 / 3;
     double fL = c6 * (-f1 + 5 * f2 + 2 * f3);
     double fR = c6 * (2 * f2 + 5 * f3 - f4);
+    if (none == 1) {
+        out_right = out_left = 0.5 * fL + 0.5 * fR;
+        return;
+    }
     double AL = f1 - 2 * f2 + f3;
     double BL = f3 - f1;
     double AR = f2 - 2 * f3 + f4;
@@ -88,31 +96,54 @@ __device__ __forceinline__ void weno_face_both(double f1, double f2, double f3, 
     double bL = c43 * (AL * AL) + 0.5 * AL * BL + 0.25 * (BL * BL);
     double bR = c43 * (AR * AR) - 0.5 * AR * BR + 0.25 * (BR * BR);
     const double mm = 1.0e-10;
-#ifdef VX_FP64_FAST
     const double dL = mm + bL, dR = mm + bR;
-    double wL = (dR * dR) * rcp_nr(dL * dL + dR * dR);
-    double wR = 1.0 - wL;
+    double wL, wR;
+#ifdef VX_FP64_FAST
+    // oL / (oL + oR) with o = 0.5 / (mm + b)^2 is dR^2 / (dL^2 + dR^2)
+    wL = (dR * dR) * rcp_nr(dL * dL + dR * dR);
+    wR = 1.0 - wL;
+    constexpr bool plain = true;
 #else
-    double oL = 0.5 / ((mm + bL) * (mm + bL));
-    double oR = 0.5 / ((mm + bR) * (mm + bR));
-    double wL = oL / (oL + oR);
-    double wR = oR / (oL + oR);
+    // within 1e-10 .. 1e95 every intermediate of the short quotients is a normal number
+    const bool plain = (unsigned)__double2hiint(dL) < 0x53a00000u && (unsigned)__double2hiint(dR) < 0x53a00000u;
+    if (plain) {
+        const double oL = 0.5 * rcp_rn(dL * dL), oR = 0.5 * rcp_rn(dR * dR);
+        const double so = oL + oR, y = rcp_ulp(so);
+        wL = div_rn(oL, so, y);
+        wR = div_rn(oR, so, y);
+    } else {
+        const double oL = 0.5 / (dL * dL), oR = 0.5 / (dR * dR);
+        wL = oL / (oL + oR);
+        wR = oR / (oL + oR);
+    }
 #endif
     double wL0 = wL * (0.75 + wL * (wL - 0.5));
     double wR0 = wR * (0.75 + wR * (wR - 0.5));
-    const double pr = (wL0 > wR0) ? wL0 : wR0, pl = (wL0 < wR0) ? wL0 : wR0;
+    const double pr = wgt(wL0, wR0) ? wL0 : wR0, pl = wgt(wR0, wL0) ? wL0 : wR0;
+    const double sw = wL0 + wR0;
 #ifdef VX_FP64_FAST
-    const double inv = rcp_nr(wL0 + wR0);  // one reciprocal for both choices
-    double fwl = pr * inv;
-    out_right = fwl * fL + (1 - fwl) * fR;
-    fwl = pl * inv;
-    out_left = fwl * fL + (1 - fwl) * fR;
+    const double inv = rcp_nr(sw);
+    auto quot = [&](double a) { return a * inv; };
 #else
-    double fwl = pr / (wL0 + wR0);
-    out_right = fwl * fL + (1 - fwl) * fR;
-    fwl = pl / (wL0 + wR0);
-    out_left = fwl * fL + (1 - fwl) * fR;
+    // the mapped weights sum to 0.75 .. 1.25, each 0 .. 1.25: below 1e-250 (a weight of a
+    // face between regions 1e60 apart) the residual would leave the normal range
+    const double inv = rcp_ulp(sw);
+    auto quot = [&](double a) {
+        return (plain && (unsigned)__double2hiint(a) >= 0x0c000000u) ? div_rn(a, sw, inv) : a / sw;
+    };
 #endif
+    const double w = quot(BOTH || right ? pr : pl);
+    out_right = w * fL + (1 - w) * fR;
+    if (BOTH) {
+        const double v = quot(pl);
+        out_left = v * fL + (1 - v) * fR;
+    }
+}
+
+__device__ __forceinline__ double weno_face(double f1, double f2, double f3, double f4, bool right) {
+    double v = 0.0, unused = 0.0;
+    weno_values<false>(f1, f2, f3, f4, right, v, unused);
+    return v;
 }
 
 __device__ __forceinline__ double vmax(double a, double b) { return (a > b) ? a : b; }
@@ -202,7 +233,7 @@ __global__ void k64_faces(const P64 *patches, const TileRef *tiles, const RunFie
     // choice.
     if ((part & 4) && i >= -1 && i <= P.nx && j >= 0 && j <= P.np) {
         double vr, vl;
-        weno_face_both(f[pidx(i, j - 2, pit)], f[pidx(i, j - 1, pit)], f[id], f[pidx(i, j + 1, pit)], vr, vl);
+        weno_values<true>(f[pidx(i, j - 2, pit)], f[pidx(i, j - 1, pit)], f[id], f[pidx(i, j + 1, pit)], true, vr, vl);
         P.fp[id] = vr;
         P.Rp[id] = vl;
     }
@@ -281,28 +312,57 @@ __global__ void k64_limR(const P64 *patches, const TileRef *tiles) {
     double dxi = DX[id], dxn = DX[id + pit], dpi = DP[id], dpn = DP[id + 1];
     double Pp = vmax0(dxi) - vmin0(dxn) + vmax0(dpi) - vmin0(dpn);
     double Pm = vmax0(dxn) - vmin0(dxi) + vmax0(dpn) - vmin0(dpi);
-    double c0 = f0[id], c2 = f2[id];
-    double w1ma = vmax(c0, c2);
-    double w2ma = vmax(f0[id + pit], f2[id + pit]);
-    double w3ma = vmax(f0[id - pit], f2[id - pit]);
-    double w4ma = vmax(f0[id + 1], f2[id + 1]);
-    double w5ma = vmax(f0[id - 1], f2[id - 1]);
-    double wMax = vmax(w1ma, vmax(w2ma, vmax(w3ma, vmax(w4ma, w5ma))));
-    double w1mi = vmin(c0, c2);
-    double w2mi = vmin(f0[id + pit], f2[id + pit]);
-    double w3mi = vmin(f0[id - pit], f2[id - pit]);
-    double w4mi = vmin(f0[id + 1], f2[id + 1]);
-    double w5mi = vmin(f0[id - 1], f2[id - 1]);
-    double wMin = vmin(w1mi, vmin(w2mi, vmin(w3mi, vmin(w4mi, w5mi))));
-    double Qm = -wMin + c2;
-    double Qp = wMax - c2;
-    // min(1, Q/P) is 1 whenever Q >= P and P is finite: the quotient (Q infinite
-    // included) is then >= 1 however it rounds.  Every other case, NaN and infinite P
-    // among them, takes the division as written.  Most cells of a smooth solution take
-    // the first branch and skip the division (about ten FP64 instructions).
-    constexpr double kMaxFinite = 1.7976931348623157e308;
-    P.Rp[id] = gt0(Pp) ? ((Qp >= Pp && Pp <= kMaxFinite) ? 1.0 : vmin(1.0, Qp / Pp)) : 0.0;
-    P.Rm[id] = gt0(Pm) ? ((Qm >= Pm && Pm <= kMaxFinite) ? 1.0 : vmin(1.0, Qm / Pm)) : 0.0;
+    const bool up = gt0(Pp), um = gt0(Pm);
+    double rp = 0.0, rm = 0.0;
+    if (up || um) {  // no antidiffusive flux touches the cell otherwise: both are 0
+        const double v[10] = {f0[id],       f2[id],       f0[id + pit], f2[id + pit], f0[id - pit],
+                              f2[id - pit], f0[id + 1],   f2[id + 1],   f0[id - 1],   f2[id - 1]};
+        const double c2 = v[1];
+        // f is not negative (the limiter's purpose), and non-negative doubles order as
+        // their bit patterns: the eighteen compares of the extrema leave the FP64 unit
+        // (one FP64 instruction of this kernel is 4.5 us per stage on the 4096 x 512
+        // workload).  A negative value, -0 or NaN among the ten takes the general path.
+        long long hi = 0, lo = 0x7FF0000000000000LL;
+        int sign = 0;
+#pragma unroll
+        for (int k = 0; k < 10; k++) {
+            const long long b = __double_as_longlong(v[k]);
+            sign |= __double2hiint(v[k]);
+            hi = b > hi ? b : hi;
+            lo = b < lo ? b : lo;
+        }
+        double wMax, wMin;
+        if (sign >= 0 && hi <= 0x7FF0000000000000LL) {
+            wMax = __longlong_as_double(hi);
+            wMin = __longlong_as_double(lo);
+        } else {
+            wMax = vmax(vmax(v[0], v[1]), vmax(vmax(v[2], v[3]), vmax(vmax(v[4], v[5]), vmax(vmax(v[6], v[7]), vmax(v[8], v[9])))));
+            wMin = vmin(vmin(v[0], v[1]), vmin(vmin(v[2], v[3]), vmin(vmin(v[4], v[5]), vmin(vmin(v[6], v[7]), vmin(v[8], v[9])))));
+        }
+        const double Qm = -wMin + c2;
+        const double Qp = wMax - c2;
+        // min(1, Q/P) is 1 whenever Q >= P and P is finite: the quotient (Q infinite
+        // included) is then >= 1 however it rounds; P > 0, so Q >= P is a compare of the
+        // bit patterns once Q's sign is known.  Every other case, NaN and infinite P
+        // among them, takes the division as written.  Most cells of a smooth solution
+        // skip the division.
+        auto ratio = [](double Q, double P) {
+            const long long q = __double_as_longlong(Q), p = __double_as_longlong(P);
+            if (q >= p && p < 0x7FF0000000000000LL && q <= 0x7FF0000000000000LL) return 1.0;
+            return vmin(1.0, Q / P);
+        };
+        if (up) rp = ratio(Qp, Pp);
+        if (um) rm = ratio(Qm, Pm);
+    }
+    P.Rp[id] = rp;
+    P.Rm[id] = rm;
+}
+
+// vmin for limiter values (not negative, or NaN) on the bit patterns: b where either is NaN
+__device__ __forceinline__ double vmin_r(double a, double b) {
+    const long long p = __double_as_longlong(a), q = __double_as_longlong(b);
+    if ((p | q) < 0) return vmin(a, b);
+    return (p < q && q <= 0x7FF0000000000000LL) ? a : b;
 }
 
 // Limiter coefficients on interior faces, 1 elsewhere (Rectangle.cpp:1581-1594).
@@ -313,8 +373,9 @@ __global__ void k64_limC(const P64 *patches, const TileRef *tiles) {
     double cx = 1.0, cp = 1.0;
     if (i >= 1 && i < P.nx && j >= 0 && j < P.np) {
         const double *Rp = P.Rp, *Rm = P.Rm;
-        cx = gt0(P.FxDS[id]) ? vmin(Rp[id], Rm[id - pit]) : vmin(Rp[id - pit], Rm[id]);
-        cp = gt0(P.FpDS[id]) ? vmin(Rp[id], Rm[id - 1]) : vmin(Rp[id - 1], Rm[id]);
+        const bool ux = gt0(P.FxDS[id]), up = gt0(P.FpDS[id]);
+        cx = vmin_r(Rp[ux ? id : id - pit], Rm[ux ? id - pit : id]);
+        cp = vmin_r(Rp[up ? id : id - 1], Rm[up ? id - 1 : id]);
     }
     P.Cx[id] = cx;
     P.Cp[id] = cp;
