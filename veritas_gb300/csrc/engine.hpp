@@ -172,7 +172,7 @@ public:
     DevBuf dBy, dBz, dEy, dEz, dAy, dAz, dasq, dphi, dcharge, dJ, dneut, defin, dex0, dasq32, defin32, dacell32;
     RunFields F{};
     PoissonLU lu;
-    DevBuf dlu_perm, dlb_band, dlb_fptr, dlb_fcol, dlb_fval, dlb_slot, dlb_sload, dlb_take, dub_band, dub_diag, dub_rdiag, dub_rdlo, dub_fptr, dub_fcol,
+    DevBuf dlu_perm, dlb_band, dlb_fptr, dlb_fcol, dlb_fval, dlb_slot, dlb_sload, dlb_take, dub_band, dub_diag, dub_sweep, dub_fptr, dub_fcol,
         dub_fval;
     LUDev ludev{};
     std::vector<int> pipe_rfc;  // per row: first forward chunk reading it (empty: no pipelined solve)

@@ -351,46 +351,42 @@ __device__ __forceinline__ double efield_at(const double *phi, int n, double fco
 }
 
 // One block per run.  The triangular solves are linear recurrences; to keep the
-// reference's rounding they run in one thread in the order of the column-oriented
-// dgetrs (entries ascending in column for L, descending for U).  FP64 dependent latency
-// (~64 cycles per add/mul, ~550 per IEEE division on this part) makes the chain length
-// the cost, so the factors are stored in band form: four coefficients per row for the
-// columns next to the diagonal (exact zeros where the factor has none — subtracting a
-// zero product never changes a partial sum, which is never -0 here) plus a short list of
-// "far" entries that precede the band in the summation order.  Only the product with the
-// previous row's value sits on the critical path.  Back substitution divides with
-// Markstein's sequence (q = s*y, r = s - q*u exactly, q' = q + r*y with y = RN(1/u));
-// after each chunk the whole block checks every quotient against the IEEE quotient and
-// the chunk is redone with IEEE division if any differs, so the result is always the
-// dgetrs rounding.
+// reference's rounding they run in the order of the column-oriented dgetrs (entries
+// ascending in column for L, descending for U), one warp each, chunk by chunk of 256 rows
+// staged in shared memory by the other warps.  FP64 dependent latency (~65 cycles per
+// add/mul/fma, ~550 per IEEE division on this part, 37 per 64-bit shuffle) makes the chain
+// length the cost, so the factors are stored in band form (exact zeros where the factor
+// has none — subtracting a zero product never changes a partial sum, which is never -0
+// here) and only the operations that need the previous row's value sit on the chain.
 constexpr int kPoisRows = kPoisRowsHost;     // rows per chunk
 constexpr int kPoisLA = 4;                   // look-ahead rows staged with each chunk
 constexpr int kPoisBuf = kPoisRows + kPoisLA;
-constexpr int kPoisFar = 2048;               // far entries per staged chunk
 
-struct PoisBandChunk {
+// Lower factor: staged rows of one chunk.
+struct PoisFwdChunk {
     int a;                                    // first staged row
     double c[4][kPoisBuf];                    // band coefficients, c[d-1][row - a]
-    double diag[kPoisBuf], rdiag[kPoisBuf], rdlo[kPoisBuf];  // U only
-    double num[kPoisRows], rhs[kPoisRows];    // backward: numerators, chunk right-hand sides
-    double slotc[4][kPoisBuf];                // forward: accumulator-lane coefficients per step
-    int sload[4][kPoisBuf];                   // forward: row taken up by each slot at each step
-    int take[kPoisBuf];                       // forward: slot finishing row step+4
-    int fptr[kPoisBuf + 1];
-    int fcol[kPoisFar];
-    double fval[kPoisFar];
+    double slotc[4][kPoisBuf];                // accumulator-lane coefficients per step
+    int sload[4][kPoisBuf];                   // row taken up by each slot at each step
+    int take[kPoisBuf];                       // slot finishing row step+4
+};
+// Upper factor: rows r0 - kPoisLA .. of a chunk starting at row r0 (zeros below row 0).
+struct PoisBwdChunk {
+    double2 c[4][kPoisBuf];                   // {u_{d+1}, d == 0 ? y : 1} of each row; c[3][0] = {0, 1}
+    float2 lo[kPoisBuf];                      // FP32 {yl, u1}
+    double diag[kPoisRows], rhs[kPoisRows];   // u_ii and the right-hand sides
+};
+union PoisChunk {
+    PoisFwdChunk f;
+    PoisBwdChunk b;
 };
 
-// Stage rows [a, b) (clamped to [0, n)) of a band factor into B with threads
-// [t0, t0+nt).  Returns whether the far entries fit.
-__device__ bool pois_stage_band(PoisBandChunk &B, const BandFactor &F, int a, int b, int n, int t0, int nt,
-                                bool upper) {
+// Stage rows [a, b) (clamped to [0, n)) of the lower factor into B with threads
+// t, t + nt, ...
+__device__ void pois_stage_fwd(PoisFwdChunk &B, const BandFactor &F, int a, int b, int n, int t, int nt) {
     a = max(a, 0);
     b = min(b, n);
     const int cnt = b - a;
-    const int f0 = F.fptr[a], f1 = F.fptr[b];
-    const bool fits = (f1 - f0) <= kPoisFar;
-    const int t = (int)threadIdx.x - t0;
     if (t == 0) B.a = a;
     for (int k = t; k < cnt; k += nt) {
         const int r = a + k;
@@ -398,11 +394,6 @@ __device__ bool pois_stage_band(PoisBandChunk &B, const BandFactor &F, int a, in
         B.c[1][k] = F.band[4 * r + 1];
         B.c[2][k] = F.band[4 * r + 2];
         B.c[3][k] = F.band[4 * r + 3];
-        if (upper) {
-            B.diag[k] = F.diag[r];
-            B.rdiag[k] = F.rdiag[r];
-            B.rdlo[k] = F.rdiag_lo[r];
-        }
         for (int sl = 0; sl < F.nslots; sl++) {
             B.slotc[sl][k] = F.slot_coef[(size_t)sl * n + r];
             B.sload[sl][k] = F.slot_load[(size_t)sl * n + r];
@@ -419,146 +410,74 @@ __device__ bool pois_stage_band(PoisBandChunk &B, const BandFactor &F, int a, in
         }
         B.take[k] = -1;
     }
-    for (int k = t; k <= cnt; k += nt) B.fptr[k] = F.fptr[a + k] - f0;
-    if (fits)
-        for (int e = f0 + t; e < f1; e += nt) {
-            B.fcol[e - f0] = F.fcol[e];
-            B.fval[e - f0] = F.fval[e];
-        }
-    return fits;
 }
 
 // Right-hand side of row r with its far entries subtracted in summation order.
-template <bool FAR_SMEM>
-__device__ __forceinline__ double pois_far(const PoisBandChunk &B, const BandFactor &F, const double *x, int r) {
-    const int k = r - B.a;
+__device__ __forceinline__ double pois_far(const BandFactor &F, const double *x, int r) {
     double s = x[r];
-    const int gbase = FAR_SMEM ? 0 : F.fptr[B.a];
-    for (int e = B.fptr[k]; e < B.fptr[k + 1]; e++) {
-        const int col = FAR_SMEM ? B.fcol[e] : F.fcol[gbase + e];
-        const double v = FAR_SMEM ? B.fval[e] : F.fval[gbase + e];
-        s = s - x[col] * v;
-    }
+    for (int e = F.fptr[r]; e < F.fptr[r + 1]; e++) s = s - x[F.fcol[e]] * F.fval[e];
     return s;
 }
 
-// Software-pipelined substitution on lanes 0..3 of warp 0.  Row i's sum is
-// ((((Fb - x4 c4) - x3 c3) - x2 c2) - x1 c1), x_d the solution d rows back (forward) or
-// ahead (backward), Fb the right-hand side minus its far entries.  Lane L holds the
-// partial sum of row i+L (forward) / i-L (backward), already reduced by every term but
-// the one with x_{i-1} (x_{i+1}); when that value arrives, each lane subtracts its own
-// product in the same two warp instructions, lane 0's result is x_i (before the division
-// backward), and the partials shift down one lane while lane 3 takes up the next row's
-// right-hand side.  On this part each FP64 warp instruction occupies the sub-partition's
-// FP64 unit for tens of cycles whatever the number of active lanes, so the lanes carry
-// the independent work for free.
-template <bool FAR_SMEM>
-__device__ void pois_fwd_chunk(const PoisBandChunk &B, const BandFactor &F, int r0, int cnt, int n, double *x,
-                               double &V, double &w1) {
-    const unsigned full = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    const int L = lane < 4 ? lane : 3;
-    const int slot = lane - 4;  // lanes 4..7: accumulators of the rows with far terms
-    const bool is_slot = slot >= 0 && slot < F.nslots;
-    const bool slots = F.nslots >= 0;
-    // Operands of row r0 + q, loaded one row ahead so their shared-memory latency overlaps
-    // the previous row's multiply-subtract.
-    auto fetch = [&](int q, double &coef, int &ld, double &fb, int &tk) {
-        const int i = r0 + q;
-        const int k = i - B.a;
-        coef = 0.0;
-        ld = -1;
-        if (lane < 4) coef = (i + L < n) ? B.c[L][k + L] : 0.0;
-        else if (is_slot) {
-            ld = B.sload[slot][k];
-            coef = B.slotc[slot][k];
+// Rows lo .. hi-1 of a factor one after another on one thread, every operation as dgetrs
+// has it: the upper factor's first rows, a chunk whose quotients did not all come out
+// (far = false: the far entries are subtracted already), and factors whose far entries do
+// not fit the sweeps' forms.
+template <bool UPPER>
+__device__ __noinline__ void pois_rows_plain(const BandFactor &F, int lo, int hi, int n, double *x, bool far) {
+    for (int q = 0; q < hi - lo; q++) {
+        const int i = UPPER ? hi - 1 - q : lo + q;
+        double s = far ? pois_far(F, x, i) : x[i];
+        for (int d = 4; d >= 1; d--) {
+            const int c = UPPER ? i + d : i - d;
+            if (c >= 0 && c < n) s = s - x[c] * F.band[4 * i + d - 1];
         }
-        fb = 0.0;
-        if (slots && lane == 3 && i + 4 < n) fb = x[i + 4];
-        tk = slots ? B.take[k] : -1;
-    };
-    double coef, fb;
-    int ld, tk;
-    fetch(0, coef, ld, fb, tk);
-    for (int q = 0; q < cnt; q++) {
-        const int i = r0 + q;
-        if (ld >= 0) V = x[ld];  // a slot takes up a new row's right-hand side
-        if (!slots && lane == 3 && i + 4 < n) fb = pois_far<FAR_SMEM>(B, F, x, i + 4);
-        const double nv = V - w1 * coef;
-        double coef_n = 0.0, fb_n = 0.0;
-        int ld_n = -1, tk_n = -1;
-        if (q + 1 < cnt) fetch(q + 1, coef_n, ld_n, fb_n, tk_n);
-        const double xi = __shfl_sync(full, nv, 0);
-        const double up = __shfl_down_sync(full, nv, 1);
-        if (slots) {
-            const double fin = __shfl_sync(full, nv, 4 + (tk >= 0 ? tk : 0));
-            if (tk >= 0) fb = fin;
-        }
-        V = (lane == 3) ? fb : (is_slot ? nv : up);
-        if (lane == 0) x[i] = xi;
-        if (!slots) __syncwarp();  // lane 3 reads x[i] when it gathers a later row's far entries
-        w1 = xi;
-        coef = coef_n;
-        fb = fb_n;
-        ld = ld_n;
-        tk = tk_n;
+        x[i] = UPPER ? s / F.diag[i] : s;
     }
 }
 
-template <bool FAR_SMEM, bool IEEE>
-__device__ void pois_bwd_chunk(PoisBandChunk &B, const BandFactor &F, int r0, int cnt, double *x, double &V,
-                               double &w1, bool far_done) {
-    const unsigned full = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    const int L = lane < 4 ? lane : 3;
-    auto fetch = [&](int qq, double &coef, double &fb, double &u, double &y) {
-        const int i = r0 + qq;
-        const int k = i - B.a;
-        coef = (i - L >= 0) ? B.c[L][k - L] : 0.0;
-        fb = (far_done && lane == 3 && i - 4 >= 0) ? x[i - 4] : 0.0;
-        u = B.diag[k];
-        y = B.rdiag[k];
-    };
-    double coef, fb, u, y;
-    fetch(cnt - 1, coef, fb, u, y);
-    for (int qq = cnt - 1; qq >= 0; qq--) {
-        const int i = r0 + qq;
-        if (!far_done && lane == 3 && i - 4 >= 0) fb = pois_far<FAR_SMEM>(B, F, x, i - 4);
-        const double nv = V - w1 * coef;
-        double coef_n = 0.0, fb_n = 0.0, u_n = 1.0, y_n = 1.0;
-        if (qq > 0) fetch(qq - 1, coef_n, fb_n, u_n, y_n);
-        const double up = __shfl_down_sync(full, nv, 1);
-        double xi = 0.0;
-        if (lane == 0) {
-            if (IEEE) {
-                xi = nv / u;
-            } else {
-                B.num[qq] = nv;
-                xi = __fma_rn(nv, y, __dmul_rn(nv, B.rdlo[i - B.a]));
-            }
-            x[i] = xi;
-        }
-        xi = __shfl_sync(full, xi, 0);
-        if (!far_done) __syncwarp();  // lane 3 reads x[i] when it gathers a later row's far entries
-        V = (lane == 3) ? fb : up;
-        w1 = xi;
-        coef = coef_n;
-        fb = fb_n;
-        u = u_n;
-        y = y_n;
+// Stage the chunk of rows [r0, r1) of the upper factor and subtract the rows' far terms
+// (their solution values are known): threads t of nt; those with t2 >= 0 (of nt2) do the
+// FP64 work.
+__device__ void pois_stage_bwd(PoisBwdChunk &B, const BandFactor &F, int r0, int r1, double *x, int t, int nt, int t2,
+                               int nt2) {
+    const int base = r0 - kPoisLA, rows = r1 - base;
+    for (int k = t; k < rows; k += nt) {
+        double v[kBwdCols] = {0.0, 0.0, 0.0, 0.0, 0.0};
+        if (base + k >= 0)
+            for (int c = 0; c < kBwdCols; c++) v[c] = F.sweep[(size_t)(base + k) * kBwdCols + c];
+        B.c[0][k] = make_double2(v[0], v[3]);
+        B.c[1][k] = make_double2(v[1], 1.0);
+        B.c[2][k] = make_double2(v[2], 1.0);
+        B.lo[k] = make_float2(__int_as_float(__double2loint(v[4])), __int_as_float(__double2hiint(v[4])));
+        if (k >= kPoisLA) B.diag[k - kPoisLA] = F.diag[base + k];
     }
+    if (t == 0) B.c[3][0] = make_double2(0.0, 1.0);
+    if (t2 >= 0)
+        for (int k = t2; k < r1 - r0; k += nt2) {
+            const double v = pois_far(F, x, r0 + k);
+            x[r0 + k] = v;
+            B.rhs[k] = v;
+        }
 }
 
-// Steady-state forms of the two chunk loops (every far term handled by accumulator
-// lanes or by the parallel pass): each lane walks its own coefficient stream with a
-// pointer, the shift and the slot hand-over are one shuffle with a per-lane source, and
-// no branch depends on the lane.  The operands of the next row are loaded at the top of
-// each row, ahead of its multiply: the warp issues in order, and a load placed after the
-// previous row's shuffle-dependent store would add its shared-memory latency to every row
-// of the chain (forward 282 -> 242 cycles per row, step 28.4 -> 27.1 ms).  The look-ahead
-// reads at most two rows past the chunk: the staged look-ahead rows, or past n the
-// neutral entries pois_stage_band writes there (zero coefficients, no slot row).
-__device__ void pois_fwd_fast(const PoisBandChunk &B, const BandFactor &F, int r0, int cnt, int n, double *x,
+// Forward sweep of one chunk, software-pipelined on lanes 0..7 of warp 0.  Row i's sum is
+// ((((Fb - x4 c4) - x3 c3) - x2 c2) - x1 c1), x_d the solution d rows back, Fb the
+// right-hand side minus its far entries (finished by the accumulator lanes 4..7).  Lane L <
+// 4 holds the partial sum of row i+L, already reduced by every term but the one with
+// x_{i-1}; when that value arrives, each lane subtracts its own product in the same two
+// warp instructions, lane 0's result is x_i, and the partials shift down one lane while
+// lane 3 takes up the next row's right-hand side.  On this part each FP64 warp instruction
+// occupies the sub-partition's FP64 unit for tens of cycles whatever the number of active
+// lanes, so the lanes carry the independent work for free.  Each lane walks its own
+// coefficient stream with a pointer, the shift and the slot hand-over are one shuffle with
+// a per-lane source, and no branch depends on the lane.  The operands of the next row are
+// loaded at the top of each row, ahead of its multiply: the warp issues in order, and a
+// load placed after the previous row's shuffle-dependent store would add its shared-memory
+// latency to every row of the chain.  The look-ahead reads at most two rows past the
+// chunk: the staged look-ahead rows, or past n the neutral entries pois_stage_fwd writes
+// there (zero coefficients, no slot row).  206 cycles per row.
+__device__ void pois_fwd_fast(const PoisFwdChunk &B, const BandFactor &F, int r0, int cnt, int n, double *x,
                               double &V, double &w1) {
     // Only lanes 0..7 (band lanes 0..3, accumulator lanes 4..7) run the recurrence.
     constexpr unsigned act = 0xffu;
@@ -616,52 +535,75 @@ __device__ void pois_fwd_fast(const PoisBandChunk &B, const BandFactor &F, int r
     }
 }
 
-__device__ void pois_bwd_fast(PoisBandChunk &B, int r0, int cnt, double *x, double &V, double &w1) {
-    // Lanes 0..3 run the multiply-subtract and lane 0 alone the quotient (the same
-    // instructions on four lanes made the backward sweep 40 % slower); the other lanes
-    // leave V and w1 unused.
-    constexpr unsigned act = 0xfu;
+// FP32 neighbours of doubles, on the integer units: d2f truncates a double (its exponent is
+// taken modulo 2^8: garbage beyond FP32's range), f2d is exact for normal floats.
+__device__ __forceinline__ float d2f_bits(double d) {
+    const unsigned hi = __double2hiint(d), lo = __double2loint(d);
+    const unsigned w = __funnelshift_l(lo, hi, 3) ^ 0x40000000u;
+    return __uint_as_float((w & 0x7fffffffu) | (hi & 0x80000000u));
+}
+__device__ __forceinline__ double f2d_bits(float f) {
+    const unsigned u = __float_as_uint(f);
+    return __hiloint2double((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + 0x38000000u), u << 29);
+}
+
+// Backward sweep of one chunk: rows r0 + cnt - 1 down to r0, on lanes 0..7 of warp 0.
+// Row k is x_k = a_k / u0, a_k = ((B_k - u3 x_{k+3}) - u2 x_{k+2}) - u1 x_{k+1} (the upper
+// factor has three columns beside the diagonal).  Lane L < 3 holds the partial sum of row
+// k - L, already reduced by every term but the one with x_{k+1}; each lane subtracts its
+// own product in the same two warp instructions, and a third, fma(a, y, t), makes lane 0's
+// sum x_k (y the rounded reciprocal of u0) and leaves the others as they are (y = 1, t =
+// -0); one shuffle spreads x_k, one moves the partials down a lane.  t is a_k times the
+// reciprocal's low part, at most half an ulp of x_k; ten of its digits are enough, so it
+// is formed in FP32 from the truncated s_k - u1 x_{k+1}, on units the chain does not use,
+// while the product and the difference run.  The quotient is then within 2^-20 ulp of the
+// true one before its rounding (FP32's range holds t down to x = 1e-21: below, above FP32's
+// range and at 0 it is simply wrong); the block checks every row against IEEE division
+// afterwards and has the chunk redone if any differs, so the result is always the dgetrs
+// rounding.  What bounds it is latency: three dependent FP64 instructions (63 cycles each)
+// and the shuffles behind them, 250 cycles per row (an fma more for t, and its lane 0
+// select: 320).
+__device__ void pois_bwd_fast(const PoisBwdChunk &B, int r0, int cnt, double *x) {
+    constexpr unsigned act = 0xffu;
     const int lane = threadIdx.x & 31;
-    if (lane >= 4) return;
-    const int L = lane;
-    const int kl = r0 + cnt - 1 - B.a;  // buffer row of the chunk's last (first processed) row
-    const double *cp = &B.c[L][kl - L];
-    const double *yp = &B.rdiag[kl];
-    const double *lp = &B.rdlo[kl];
-    const int ilast = r0 + cnt - 1;
-    double coef = (ilast - L < 0) ? 0.0 : cp[0];
-    double y = yp[0], ylo = lp[0];
-    cp--;
-    yp--;
-    lp--;
-    double fb = (lane == 3 && ilast - 4 >= 0) ? x[ilast - 4] : 0.0;
-    for (int qq = cnt - 1; qq >= 0; qq--) {
-        const int i = r0 + qq;
-        // row i-1's operands (kPoisLA rows are staged below the chunk); x[i - 5] is still
-        // the right-hand side
-        const double coef_n = (i - 1 - L >= 0) ? cp[0] : 0.0;
-        const double y_n = qq > 0 ? yp[0] : 0.0, ylo_n = qq > 0 ? lp[0] : 0.0;
-        const double fb_n = (lane == 3 && i - 5 >= 0) ? x[i - 5] : 0.0;
-        cp--;
-        yp--;
-        lp--;
-        const double nv = V - w1 * coef;
-        const double up = __shfl_down_sync(act, nv, 1, 4);
-        // quotient from the reciprocal split into high and low parts: within 2^-105 of
-        // nv/u before the final rounding; the chunk check catches the rare wrong rounding
-        double q1 = 0.0;
-        if (lane == 0) {
-            q1 = __fma_rn(nv, y, __dmul_rn(nv, ylo));
-            B.num[qq] = nv;
-            x[i] = q1;
-        }
-        const double xi = __shfl_sync(act, q1, 0, 4);
-        V = (lane == 3) ? fb : up;
-        w1 = xi;
-        coef = coef_n;
-        y = y_n;
-        ylo = ylo_n;
-        fb = fb_n;
+    if (lane >= 8) return;
+    const int k0 = r0 + cnt - 1, q0 = cnt - 1 + kPoisLA;  // first row and its buffer row
+    const bool is0 = lane == 0, is2 = lane == 2;
+    const int src = lane < 7 ? lane + 1 : 7;
+    const double2 *pc = lane < 3 ? &B.c[lane][q0 - lane] : &B.c[3][0];
+    const int sc = lane < 3 ? 1 : 0;
+    // lane 2: the right-hand sides, from row k0 - 2 down (rows below the chunk are not read);
+    // the others: the FP32 pair of the row
+    const double *pl = is2 ? x + k0 - 2 : reinterpret_cast<const double *>(&B.lo[q0]);
+    int left = is2 ? cnt - 2 : 0x7fffffff;
+    double X = x[k0 + 1], V = 0.0;
+    {
+        const double x2 = x[k0 + 2], x3 = x[k0 + 3];
+        if (is0) V = (x[k0] - x3 * B.c[2][q0].x) - x2 * B.c[1][q0].x;
+        if (lane == 1 && cnt > 1) V = x[k0 - 1] - x2 * B.c[2][q0 - 1].x;
+        if (is2 && cnt > 2) V = x[k0 - 2];
+    }
+    double2 c = *pc;
+    double l = left > 0 ? *pl : 0.0;
+#pragma unroll 2
+    for (int q = cnt - 1; q >= 0; q--) {
+        pc -= sc;
+        pl--;
+        left--;
+        const double2 c_n = *pc;
+        const double l_n = left > 0 ? *pl : 0.0;
+        const double m = __dmul_rn(X, c.x);
+        const float yl = __int_as_float(__double2loint(l)), u1 = __int_as_float(__double2hiint(l));
+        const float tf = yl * (d2f_bits(V) - u1 * d2f_bits(X));
+        const double t = is0 ? f2d_bits(tf) : -0.0;
+        const double a = __dsub_rn(V, m);
+        const double r = __fma_rn(a, c.y, t);
+        X = __shfl_sync(act, r, 0, 8);
+        const double down = __shfl_sync(act, r, src, 8);
+        V = is2 ? l_n : down;
+        if (is0) x[r0 + q] = r;
+        c = c_n;
+        l = l_n;
     }
 }
 
@@ -749,7 +691,7 @@ __device__ void pipe_rows(const PipeLaunch &K, int run, int c, double *x, int t,
 template <bool XS, bool PIPE>
 __device__ __forceinline__ void poisson_solve(const PoissonLaunch &L, unsigned char *smem_raw, double *x,
                                               const PipeLaunch *K) {
-    PoisBandChunk *buf = (PoisBandChunk *)smem_raw;  // two chunk buffers, then the solution vector
+    PoisChunk *buf = (PoisChunk *)smem_raw;  // two chunk buffers, then the solution vector
     __shared__ int s_bad;
     const int run = blockIdx.x;
     RunFields &F = L.fields[run];
@@ -778,119 +720,86 @@ __device__ __forceinline__ void poisson_solve(const PoissonLaunch &L, unsigned c
     if (PIPE && K->trace && run == 0 && threadIdx.x == 0) K->trace[1 + 2 * K->trace_nch] = clock64();
     const int lane = threadIdx.x & 31;
     // ---- forward: rows ascending; chunk c stages rows [c*R, c*R + R + LA)
-    {
-        double V = 0.0, w1 = 0.0;
-        bool fit_cur = pois_stage_band(buf[0], lu.L, 0, kPoisBuf, n, 0, blockDim.x, false);
+    if (!PIPE && lu.L.nslots < 0) {
         __syncthreads();
-        if (threadIdx.x < 32 && lane < 4 && lane < n)
-            V = fit_cur ? pois_far<true>(buf[0], lu.L, x, lane) : pois_far<false>(buf[0], lu.L, x, lane);
-
-        if (PIPE) {
-            // warp 0 sweeps, the others stage the next chunk and gather its rows: two
-            // loops with one block barrier per chunk each, so that the sweep's loop holds
-            // only the sweep's values (the accumulator-lane form: the host pipelines only
-            // factors that have it)
-            if (threadIdx.x < 32) {
-                for (int c = 0; c < nchunks; c++) {
-                    const int r0 = c * kPoisRows;
-                    pois_fwd_fast(buf[c & 1], lu.L, r0, min(kPoisRows, n - r0), n, x, V, w1);
-                    __syncthreads();
-                    if (trace) trace[1 + c] = tick();
-                }
-            } else {
-                for (int c = 0; c + 1 < nchunks; c++) {
-                    const int r1 = (c + 1) * kPoisRows;
-                    pois_stage_band(buf[(c + 1) & 1], lu.L, r1, r1 + kPoisBuf, n, 32, blockDim.x - 32, false);
-                    // the rows chunk c+1 reads first, while warp 0 sweeps chunk c (it reads
-                    // and writes only rows first read by chunks up to c)
-                    pipe_rows(*K, run, c + 1, x, threadIdx.x - 32, blockDim.x - 32, 1, true);
-                    __syncthreads();
-                }
-                __syncthreads();  // the last chunk's
+        if (threadIdx.x == 0) pois_rows_plain<false>(lu.L, 0, n, n, x, true);
+        __syncthreads();
+    } else {
+        double V = 0.0, w1 = 0.0;
+        pois_stage_fwd(buf[0].f, lu.L, 0, kPoisBuf, n, threadIdx.x, blockDim.x);
+        __syncthreads();
+        if (threadIdx.x < 32 && lane < 4 && lane < n) V = pois_far(lu.L, x, lane);
+        // warp 0 sweeps, the others stage the next chunk (pipelined: and gather its rows):
+        // two loops with one block barrier per chunk each, so that the sweep's loop holds
+        // only the sweep's values (the host pipelines only factors with accumulator lanes)
+        if (threadIdx.x < 32) {
+            for (int c = 0; c < nchunks; c++) {
+                const int r0 = c * kPoisRows;
+                pois_fwd_fast(buf[c & 1].f, lu.L, r0, min(kPoisRows, n - r0), n, x, V, w1);
+                __syncthreads();
+                if (trace) trace[1 + c] = tick();
             }
-        }
-        for (int c = 0; !PIPE && c < nchunks; c++) {
-            const int r0 = c * kPoisRows, cnt = min(kPoisRows, n - r0);
-            PoisBandChunk &B = buf[c & 1];
-            bool fit_next = false;
-            if (c + 1 < nchunks) {
-                const int r1 = r0 + kPoisRows;
-                if (threadIdx.x >= 32)
-                    fit_next = pois_stage_band(buf[(c + 1) & 1], lu.L, r1, r1 + kPoisBuf, n, 32, blockDim.x - 32, false);
-                else
-                    fit_next = (lu.L.fptr[min(r1 + kPoisBuf, n)] - lu.L.fptr[r1]) <= kPoisFar;
+        } else {
+            for (int c = 0; c + 1 < nchunks; c++) {
+                const int r1 = (c + 1) * kPoisRows;
+                pois_stage_fwd(buf[(c + 1) & 1].f, lu.L, r1, r1 + kPoisBuf, n, threadIdx.x - 32, blockDim.x - 32);
+                // the rows chunk c+1 reads first, while warp 0 sweeps chunk c (it reads
+                // and writes only rows first read by chunks up to c)
+                if (PIPE) pipe_rows(*K, run, c + 1, x, threadIdx.x - 32, blockDim.x - 32, 1, true);
+                __syncthreads();
             }
-            if (threadIdx.x < 32) {
-                if (lu.L.nslots >= 0) pois_fwd_fast(B, lu.L, r0, cnt, n, x, V, w1);
-                else if (fit_cur) pois_fwd_chunk<true>(B, lu.L, r0, cnt, n, x, V, w1);
-                else pois_fwd_chunk<false>(B, lu.L, r0, cnt, n, x, V, w1);
-            }
-            fit_cur = fit_next;
-            __syncthreads();
-            if (trace) trace[1 + c] = tick();
+            __syncthreads();  // the last chunk's
         }
     }
     if (PIPE && K->trace && run == 0 && threadIdx.x == 0) K->trace[2 + 2 * K->trace_nch] = clock64();
-    // ---- backward: rows descending; chunk c stages rows [c*R - LA, c*R + R)
+    // ---- backward: the last rows (all of them if their far columns reach further down)
+    // one by one, then chunks of R rows, descending
     {
-        double V = 0.0, w1 = 0.0;
-        bool far_done = false;
-        const int clast = nchunks - 1;
-        int parity = 0;
-        bool fit_cur = pois_stage_band(buf[0], lu.U, clast * kPoisRows - kPoisLA, n, n, 0, blockDim.x, true);
-        __syncthreads();
-        if (threadIdx.x < 32 && lane < 4 && n - 1 - lane >= 0)
-            V = fit_cur ? pois_far<true>(buf[0], lu.U, x, n - 1 - lane) : pois_far<false>(buf[0], lu.U, x, n - 1 - lane);
-        for (int c = clast; c >= 0; c--) {
-            const int r0 = c * kPoisRows, cnt = min(kPoisRows, n - r0);
-            PoisBandChunk &B = buf[parity];
-            bool fit_next = false;
-            if (c > 0) {
-                const int r1 = (c - 1) * kPoisRows;
-                if (threadIdx.x >= 32)
-                    fit_next = pois_stage_band(buf[parity ^ 1], lu.U, r1 - kPoisLA, r1 + kPoisRows, n, 32, blockDim.x - 32, true);
-                else
-                    fit_next = (lu.U.fptr[r1 + kPoisRows] - lu.U.fptr[max(r1 - kPoisLA, 0)]) <= kPoisFar;
-            }
-            const double V0 = V, w10 = w1;
-            if (threadIdx.x < 32) {
-                if (threadIdx.x == 0) s_bad = 0;
-                for (int q = lane; q < cnt; q += 32) B.rhs[q] = x[r0 + q];
-                __syncwarp();
-                if (far_done) pois_bwd_fast(B, r0, cnt, x, V, w1);
-                else if (fit_cur) pois_bwd_chunk<true, false>(B, lu.U, r0, cnt, x, V, w1, far_done);
-                else pois_bwd_chunk<false, false>(B, lu.U, r0, cnt, x, V, w1, far_done);
-            }
-            __syncthreads();
-            // every Markstein quotient of the chunk against the IEEE quotient of its numerator
-            for (int q = threadIdx.x; q < cnt; q += blockDim.x) {
-                const double ieee = B.num[q] / B.diag[r0 + q - B.a];
-                if (__double_as_longlong(ieee) != __double_as_longlong(x[r0 + q])) s_bad = 1;
-            }
-            __syncthreads();
-            if (s_bad && threadIdx.x < 32) {
-                for (int q = lane; q < cnt; q += 32) x[r0 + q] = B.rhs[q];
-                __syncwarp();
-                V = V0;
-                w1 = w10;
-                if (fit_cur) pois_bwd_chunk<true, true>(B, lu.U, r0, cnt, x, V, w1, far_done);
-                else pois_bwd_chunk<false, true>(B, lu.U, r0, cnt, x, V, w1, far_done);
-            }
-            __syncthreads();
-            if (!far_done && c == clast && lu.U.far_pre_col == r0 && r0 > 4) {
-                // x_{r0..n-1} are final: subtract the far terms of every row below r0-4 at once
-                for (int r = threadIdx.x; r < r0 - 4; r += blockDim.x) {
-                    double v = x[r];
-                    for (int e = lu.U.fptr[r]; e < lu.U.fptr[r + 1]; e++) v = v - x[lu.U.fcol[e]] * lu.U.fval[e];
-                    x[r] = v;
-                }
-                far_done = true;
-            }
-            fit_cur = fit_next;
-            parity ^= 1;
-            __syncthreads();
-            if (trace) trace[1 + nchunks + (clast - c)] = tick();
+        const int t0 = lu.U.sweep ? lu.U.far_pre_col : 0;
+        if (threadIdx.x == 0) {
+            pois_rows_plain<true>(lu.U, t0, n, n, x, true);
+            s_bad = 0;
         }
+        __syncthreads();
+        const int nbwd = (t0 + kPoisRows - 1) / kPoisRows;
+        // FP64 work of the staging warps stays off warp 0's sub-partition (warps 4m)
+        const int wg = (int)threadIdx.x >> 5;
+        const int t2 = (wg & 3) == 0 ? -1 : ((wg >> 2) * 3 + (wg & 3) - 1) * 32 + lane;
+        const int nt2 = ((int)blockDim.x >> 7) * 3 * 32;
+        if (nbwd > 0)
+            pois_stage_bwd(buf[0].b, lu.U, max(t0 - kPoisRows, 0), t0, x, threadIdx.x, blockDim.x, t2, nt2);
+        __syncthreads();
+        for (int c = 0; c < nbwd; c++) {
+            const int r1 = t0 - c * kPoisRows, r0 = max(r1 - kPoisRows, 0), cnt = r1 - r0;
+            PoisBwdChunk &B = buf[c & 1].b;
+            if (threadIdx.x < 32) pois_bwd_fast(B, r0, cnt, x);
+            else if (r0 > 0)
+                pois_stage_bwd(buf[(c + 1) & 1].b, lu.U, max(r0 - kPoisRows, 0), r0, x, threadIdx.x - 32,
+                               blockDim.x - 32, t2, nt2);
+            __syncthreads();
+            // every row of the chunk with IEEE division, from the rows above it
+            for (int q = threadIdx.x; q < cnt; q += blockDim.x) {
+                const double *xr = x + r0 + q;
+                const int e = q + kPoisLA;
+                double s = B.rhs[q] - xr[3] * B.c[2][e].x;
+                s = s - xr[2] * B.c[1][e].x;
+                s = s - xr[1] * B.c[0][e].x;
+                if (__double_as_longlong(s / B.diag[q]) != __double_as_longlong(xr[0])) s_bad = 1;
+            }
+            __syncthreads();
+            if (s_bad) {  // uniform: redone in IEEE division (the next chunk's sweep reads x alone)
+                for (int q = threadIdx.x; q < cnt; q += blockDim.x) x[r0 + q] = B.rhs[q];
+                __syncthreads();
+                if (threadIdx.x == 0) {
+                    pois_rows_plain<true>(lu.U, r0, r1, n, x, false);
+                    s_bad = 0;
+                }
+                __syncthreads();
+            }
+            if (trace) trace[1 + nchunks + c] = tick();
+        }
+        if (trace)
+            for (int c = nbwd; c < nchunks; c++) trace[1 + nchunks + c] = tick();
     }
     if (in_smem)
         for (int i = threadIdx.x; i < n; i += blockDim.x) F.phi[i] = x[i];
@@ -908,7 +817,7 @@ __device__ __forceinline__ void poisson_solve(const PoissonLaunch &L, unsigned c
 __global__ void __launch_bounds__(1024, 1) k_poisson(PoissonLaunch L) {
     VX_PDL_WAIT();
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    if (L.x_in_smem) poisson_solve<true, false>(L, smem_raw, (double *)(smem_raw + 2 * sizeof(PoisBandChunk)), nullptr);
+    if (L.x_in_smem) poisson_solve<true, false>(L, smem_raw, (double *)(smem_raw + 2 * sizeof(PoisChunk)), nullptr);
     else poisson_solve<false, false>(L, smem_raw, L.fields[blockIdx.x].phi, nullptr);
 }
 
@@ -1057,7 +966,7 @@ __global__ void __launch_bounds__(1024, 1) k64_moments_poisson(PipeLaunch K) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     if ((int)blockIdx.x < K.P.nruns) {
         if (K.P.x_in_smem)
-            poisson_solve<true, true>(K.P, smem_raw, (double *)(smem_raw + 2 * sizeof(PoisBandChunk)), &K);
+            poisson_solve<true, true>(K.P, smem_raw, (double *)(smem_raw + 2 * sizeof(PoisChunk)), &K);
         else poisson_solve<false, true>(K.P, smem_raw, K.P.fields[blockIdx.x].phi, &K);
     } else if ((int)blockIdx.x < K.P.nruns + K.summers) {
         if (threadIdx.x < 4 * 32) pipe_summer(K, (int)threadIdx.x & 31);  // warps 0..3: one per sub-partition
@@ -1087,7 +996,7 @@ void launch_poisson(const PoissonLaunch &L) {
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     // the solution vector joins the two chunk buffers in shared memory when it fits
-    const int base = 2 * (int)sizeof(PoisBandChunk);
+    const int base = 2 * (int)sizeof(PoisChunk);
     P.x_in_smem = (L.maxn <= kPoisSmemMaxN && base + 8 * L.maxn <= max_smem) ? 1 : 0;
     const int smem = base + (P.x_in_smem ? 8 * L.maxn : 0);
     cudaFuncSetAttribute(k_poisson, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -1102,7 +1011,7 @@ void launch_moments_poisson64(const PipeLaunch &K0) {
     int max_smem = 0, dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    const int base = 2 * (int)sizeof(PoisBandChunk);
+    const int base = 2 * (int)sizeof(PoisChunk);
     K.P.x_in_smem = (K.P.maxn <= kPoisSmemMaxN && base + 8 * K.P.maxn <= max_smem) ? 1 : 0;
     const int smem_solve = base + (K.P.x_in_smem ? 8 * K.P.maxn : 0);
     const int smem = std::max(smem_solve, 16);

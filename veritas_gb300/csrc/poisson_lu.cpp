@@ -2,6 +2,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <map>
 #include <stdexcept>
 
@@ -219,8 +220,6 @@ PoissonLU::Band PoissonLU::upper_band() const {
     Band B;
     B.band.assign((size_t)4 * n, 0.0);
     B.diag = udiag;
-    B.rdiag = urdiag;
-    B.rdiag_lo = urdiag_lo;
     B.fptr.push_back(0);
     for (int i = 0; i < n; i++) {
         for (int e = uptr[i]; e < uptr[i + 1]; e++) {  // descending columns
@@ -234,15 +233,21 @@ PoissonLU::Band PoissonLU::upper_band() const {
         }
         B.fptr.push_back((int)B.fcol.size());
     }
-    // Far terms of the rows below the last 256-row chunk can be precomputed in parallel
-    // after that chunk when every such row's far columns lie inside it.
-    const int R = 256;
-    const int last = ((n + R - 1) / R - 1) * R;
-    bool ok = last > 4;
-    for (int i = 0; ok && i < last - 4; i++)
+    const int t0 = n - Band::kTail;
+    if (t0 < 1) return B;
+    for (int i = 0; i < t0; i++) {
+        if (B.band[4 * i + 3] != 0.0) return B;
         for (int e = B.fptr[i]; e < B.fptr[i + 1]; e++)
-            if (B.fcol[e] < last) ok = false;
-    B.far_pre_col = ok ? last : -1;
+            if (B.fcol[e] < t0) return B;
+    }
+    B.far_pre_col = t0;
+    B.sweep.resize((size_t)n * Band::kCols);
+    for (int i = 0; i < n; i++) {
+        const float lo[2] = {(float)urdiag_lo[i], (float)B.band[4 * i]};
+        double v[Band::kCols] = {B.band[4 * i], B.band[4 * i + 1], B.band[4 * i + 2], urdiag[i], 0.0};
+        std::memcpy(&v[4], lo, sizeof lo);
+        std::copy(v, v + Band::kCols, B.sweep.begin() + (size_t)i * Band::kCols);
+    }
     return B;
 }
 

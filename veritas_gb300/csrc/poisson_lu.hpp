@@ -30,7 +30,7 @@ struct PoissonLU {
     // Band form of the factors for the device (four columns either side of the
     // diagonal, the rest as "far" entries in summation order).
     struct Band {
-        std::vector<double> band, diag, rdiag, rdiag_lo, fval;
+        std::vector<double> band, diag, fval;
         std::vector<int> fptr, fcol;
         // Lower factor: the far terms of every row are accumulated by up to kMaxSlots
         // dedicated lanes.  At step i (when x_{i-1} has just been produced) slot s
@@ -42,9 +42,16 @@ struct PoissonLU {
         int nslots = 0;
         std::vector<double> slot_coef;
         std::vector<int> slot_load, take;
-        // Upper factor: rows below far_pre_row have all their far columns at or above
-        // far_pre_col, so their far terms can be subtracted in one parallel pass once the
-        // solution is known from far_pre_col up (-1: not possible).
+        // Upper factor: the far columns of every row below far_pre_col lie at or above it,
+        // and those rows have three columns beside the diagonal, so the device can solve
+        // the rows from far_pre_col up one by one, subtract the far terms of all others
+        // and run its three-instruction sweep over them.  sweep holds kCols columns of each
+        // row i: u1, u2, u3 (columns i+1 .. i+3), y = RN(1 / u_ii), and the pair of floats
+        // (1 / u_ii - y, u1) in the fifth's eight bytes.  Empty when a row does not fit
+        // (far_pre_col is then -1).
+        static constexpr int kCols = 5;
+        static constexpr int kTail = 8;  // rows solved one by one: the far columns are n-1 and n-2
+        std::vector<double> sweep;
         int far_pre_col = -1;
     };
     Band lower_band() const;

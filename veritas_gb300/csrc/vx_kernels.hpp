@@ -134,18 +134,18 @@ void launch_assemble(const AsmLaunch &A);
 // One triangular factor in band form (see k_poisson): band[4*i + d - 1] is the
 // coefficient of column i-d (L) or i+d (U), exact zero where the factor has none; the
 // far entries of row i are fcol/fval[fptr[i] .. fptr[i+1]) in summation order.
+constexpr int kBwdCols = 5;  // PoissonLU::Band::kCols
 struct BandFactor {
     const double *band;
     const double *diag;   // U: u_ii
-    const double *rdiag;  // U: RN(1/u_ii)
-    const double *rdiag_lo;  // U: 1/u_ii - RN(1/u_ii)
+    const double *sweep;  // U: kBwdCols columns per row (PoissonLU::Band::sweep), or null
     const int *fptr, *fcol;
     const double *fval;
-    int nslots;                // L: accumulator lanes in use (-1: far terms on lane 3)
+    int nslots;                // L: accumulator lanes in use (-1: the rows do not fit them)
     const double *slot_coef;   // L: [slot][step] coefficient of column step-1
     const int *slot_load;      // L: [slot][step] row whose right-hand side the slot takes up, or -1
     const int *take;           // L: [step] slot finishing row step+4, or -1
-    int far_pre_col;           // U: see PoissonLU::Band (-1: none)
+    int far_pre_col;           // U: see PoissonLU::Band (sweep not null)
 };
 
 struct LUDev {
