@@ -655,6 +655,8 @@ std::vector<double> Engine::profile_kernels(Run &run, int reps) {
     ml.nruns = (int)L.runs.size();
     ml.maxnf = L.maxnf;
     ml.fast = L.precision == kF64 ? L.fast64 : 0;
+    ml.screen = L.dmom_screen.as<unsigned>();
+    ml.maxnwin = L.mom_maxnwin;
     ml.acell = 0;  // as in a step's later stages: the Maxwell stage made the copy
     ml.stream = stream;
     time_it([&] { run_moments(L, ml); });
@@ -724,7 +726,10 @@ std::vector<double> Engine::profile_kernels(Run &run, int reps) {
         StageLaunches K = stage_launches(L);
         K.ml.acell = 0;
         PipeLaunch P = pipe_launch(L, K);
-        time_it([&] { launch_moments_poisson64(P); });
+        time_it([&] {
+            launch_mom_screen64(P.M);
+            launch_moments_poisson64(P);
+        });
         pipe_pending_ = true;
         // VX_TRACE_PIPE=1: when each forward chunk's rows were ready, when the sweeps ended
         // and when each chunk's last moment unit finished (ns from the solve's start)
@@ -735,6 +740,7 @@ std::vector<double> Engine::profile_kernels(Run &run, int reps) {
             P.trace = tr.as<unsigned long long>();
             P.trace_nch = nch;
             P.P.trace = tp.as<unsigned long long>();
+            launch_mom_screen64(P.M);
             launch_moments_poisson64(P);
             sync();
             std::vector<unsigned long long> a(3 + 2 * nch), b(2 * nch + 1);
@@ -1107,6 +1113,10 @@ void Engine::build_set(LaunchSet &L) {
         colidx.swap(ci2);
     }
     L.ncols = (int)colpatch.size();
+    if (L.precision == kF64) {
+        L.mom_maxnwin = (L.maxnp + kMomWindow - 1) / kMomWindow;
+        pk.reserve(L.dmom_screen, (size_t)(L.ncols / kMomCols) * L.mom_maxnwin * kMomScreen * sizeof(unsigned));
+    }
     build_pipe_tables(L, colpatch, colidx, pk);
     lap("units");
     // lvl_ptr is absolute; lvl_off points at each run's block.
@@ -1253,11 +1263,12 @@ void Engine::build_pipe_tables(LaunchSet &L, const std::vector<int> &colpatch, c
     pk.put(L.dpipe_grow, grow);
     L.dpipe_scratch = DevBuf((size_t)nitems * kPipeItemDoubles * sizeof(double));
     L.dpipe_state = DevBuf((size_t)(kPipeDone + L.pipe_ndone + 2 * nunits) * sizeof(unsigned));  // zeroed
-    // summing warps, four per block: each unit's sums take about 64 cycles per FP64 add on
-    // their sub-partition; enough blocks that they keep up with the column warps
-    long long adds = 0;
-    for (int t = 0; t < nunits; t++) adds += (long long)(item0[t + 1] - item0[t]) * 2 * kMomWindow;
-    L.pipe_summers = (int)std::min<long long>(8, std::max<long long>(1, (adds * 64 / 4 + 1200000 - 1) / 1200000));
+    // Summing warps, four per block, each with an FP64 unit to itself (64 cycles per add).
+    // Eight blocks per run let the sums keep ahead of the forward sweep's 200 cycles per row;
+    // with fewer the sweep waits for them (4096 x 512 two-level step 39.5 / 25.6 / 18.6 /
+    // 15.9 / 15.9 ms with 1 / 2 / 4 / 8 / 12 blocks, 2048 x 256 7.2 / 5.2 / 4.4 / 4.2 / 4.2
+    // ms).  A small set has no use for more warps than units.
+    L.pipe_summers = std::max(1, std::min({8 * (int)L.runs.size(), 24, (nunits + 3) / 4}));
     if (!pipe_err_.p) pipe_err_ = DevBuf(sizeof(int));
     L.pipe = true;
 }
@@ -1293,6 +1304,8 @@ StageLaunches Engine::stage_launches(LaunchSet &L) {
     ml.nruns = (int)L.runs.size();
     ml.maxnf = L.maxnf;
     ml.fast = L.precision == kF64 ? L.fast64 : 0;
+    ml.screen = L.dmom_screen.as<unsigned>();
+    ml.maxnwin = L.mom_maxnwin;
     ml.stream = stream;
     al.patches = L.dpatch.p;
     al.lvl_ptr = L.dlvl_ptr.as<int>();
@@ -1350,7 +1363,7 @@ void Engine::record_step(LaunchSet &L) {
         ml.acell = s == 0;
         run_moments(L, ml);
         launch_assemble(al);
-        launches += (L.precision == kF32 && s == 0) ? 3 : 2;
+        launches += (L.precision == kF32 && s != 0) ? 2 : 3;  // FP64: with the moments' screen
         // the Poisson solve (and E_x) runs beside the x-direction face work, which does
         // not read E_x; the p-direction faces wait for both
         VX_CUDA(cudaEventRecord(ev_fork, stream));
@@ -1441,6 +1454,7 @@ void Engine::record_step(LaunchSet &L) {
 PipeLaunch Engine::pipe_launch(LaunchSet &L, const StageLaunches &K) {
     PipeLaunch P{};
     P.M = K.ml;
+    P.M.priority = prio_hi_;
     P.A = K.al;
     P.P = K.pl;
     P.P.stream = stream;
@@ -1476,6 +1490,7 @@ void Engine::record_pipe_stage(LaunchSet &L, StageLaunches &K, int s, int &launc
     const PipeLaunch P = pipe_launch(L, K);
     VX_CUDA(cudaEventRecord(ev_fork, stream));
     VX_CUDA(cudaStreamWaitEvent(side, ev_fork, 0));
+    launch_mom_screen64(P.M);
     launch_moments_poisson64(P);
     VX_CUDA(cudaEventRecord(ev_join, stream));
     fl.step = s;
@@ -1492,7 +1507,7 @@ void Engine::record_pipe_stage(LaunchSet &L, StageLaunches &K, int s, int &launc
     mx.stream = side;
     launch_maxwell(mx);
     VX_CUDA(cudaEventRecord(ev_mx, side));
-    launches += 1 + 4 + 3;
+    launches += 2 + 4 + 3;
     fl.stream = stream;
     VX_CUDA(cudaStreamWaitEvent(stream, ev_gamma, 0));
     fl.part = 8;
@@ -1720,7 +1735,7 @@ void Engine::run_phases(Run &run, int s, double dt, unsigned phases) {
         K.ml.acell = 1;
         run_moments(L, K.ml);
         launch_assemble(K.al);
-        launches += (L.precision == kF32) ? 3 : 2;
+        launches += 3;  // FP32: the per-cell A^2 copy; FP64: the moments' screen
     }
     if (phases & kPhPoisson) {  // EMFieldSolver::UpdatePotential and E_x
         run_poisson(L, K.pl);
@@ -1875,6 +1890,8 @@ void Engine::moments_only(const std::vector<Run *> &set) {
     ml.nruns = (int)L.runs.size();
     ml.maxnf = L.maxnf;
     ml.fast = L.precision == kF64 ? L.fast64 : 0;
+    ml.screen = L.dmom_screen.as<unsigned>();
+    ml.maxnwin = L.mom_maxnwin;
     ml.stream = stream;
     run_moments(L, ml);
     AsmLaunch al{};

@@ -259,7 +259,7 @@ struct LaunchSet {
     uint64_t key_version = 0;
     std::vector<PatchT<double>> hpatch;
     DevBuf dpatch, dtiles, dfields, dcolpatch, dcolidx, dlvl_ptr, dlvl_off, dlvl_patch, drun_n, drun_ns,
-        drun_nl, dlu, dw, dfcoef, dparams, dcfl_spec, dcfl_out, dns, ddxinv;
+        drun_nl, dlu, dw, dmom_screen, dfcoef, dparams, dcfl_spec, dcfl_out, dns, ddxinv;
     int ntiles = 0, ncols = 0, maxnp = 0, maxn = 0, maxnf = 0;
     std::vector<double> hparams;  // per run: 6 stages x (8 fct + 8 maxwell + 2 laser)
     std::vector<float> hparams32;
@@ -281,6 +281,7 @@ struct LaunchSet {
     // FP64 exact-solve sets of up to kPipeMaxRuns runs: tables of the pipelined moments +
     // solve launch (k64_moments_poisson)
     bool pipe = false;
+    int mom_maxnwin = 0;  // FP64: windows per unit of dmom_screen
     int pipe_nunits = 0, pipe_nitems = 0, pipe_ndone = 0, pipe_summers = 1;
     DevBuf dpipe_col0, dpipe_sig, dpipe_item0, dpipe_nwin, dpipe_c12, dpipe_items, dpipe_need, dpipe_runctr,
         dpipe_rungptr, dpipe_gptr, dpipe_grow, dpipe_scratch, dpipe_state;

@@ -206,7 +206,7 @@ __global__ void k64_gamma(const P64 *patches, const TileRef *tiles, const RunFie
     const RunFields &F = fields[P.run];
     double as = P.qq * a_sq_face(P, F, i);
     double p = P.pmin + P.dp * (double)(j + P.p_pos);
-    P.gam[id] = sqrt(1.0 + ((p * p) + as) * P.g2);
+    P.gam[id] = sqrt_rn(1.0 + ((p * p) + as) * P.g2);
 }
 
 // Face velocities and reconstructed face values (Rectangle.cpp:1278-1312).

@@ -8,6 +8,7 @@
 // and evaluation order.
 #include <cuda_runtime.h>
 #include <algorithm>
+#include "div64.cuh"
 #include "fast64.cuh"
 #include "field_ops.cuh"
 #include "vx_kernels.hpp"
@@ -101,7 +102,7 @@ constexpr int kMomThreads = (kMomCols + 1) * 32;
 // Two window buffers: the column warps fill one while the summing warp adds the other.
 struct MomSmem {
     double cc[2][kMomCols][2][32], cj[2][kMomCols][2][32];
-    unsigned use[2][kMomCols];
+    int redo;
 };
 
 // Barrier of one moment unit's kMomThreads threads: barrier 0 in k64_moments (the whole
@@ -122,13 +123,13 @@ __device__ __forceinline__ void mom_sync(int bar) {
 __device__ __forceinline__ double fast_log_ratio(double Gn, double G) {
     const double s = Gn + G;
     if (G != 0.0 && s != 0.0) {
-        const double z = (Gn - G) * rcp_nr(s);
+        const double z = (Gn - G) * rcp_ulp(s);
         if (fabs(z) <= 0.01) {
             const double z2 = z * z;
             const double poly = __fma_rn(z2, __fma_rn(z2, __fma_rn(z2, 1.0 / 7.0, 0.2), 1.0 / 3.0), 1.0);
             return (2.0 * z) * poly;
         }
-        return log(Gn * rcp_nr(G));
+        return log(Gn * rcp_ulp(G));
     }
     return log(Gn / G);
 }
@@ -161,17 +162,17 @@ __device__ __forceinline__ void mom_window(const P64 &P, const double *f, bool r
             double G = 0.0, V = 0.0;
             if (j <= np + 1) {
                 if (FAST) {
-                    const double g = sqrt(__fma_rn(__fma_rn(p, p, a[q]), P.g2, 1.0));
+                    const double g = sqrt_rn(__fma_rn(__fma_rn(p, p, a[q]), P.g2, 1.0));
                     G = __fma_rn(c1, p, g);
                 } else {
-                    double g = sqrt(1.0 + ((p * p) + a[q]) * P.g2);
+                    double g = sqrt_rn(1.0 + ((p * p) + a[q]) * P.g2);
                     G = g + c1 * p;
                 }
             }
             if (j <= np) V = rtb == 1 ? f3 : (FAST ? rel_pick_fma(P, k0 + q, a1, a2, a3, f3) : rel_pick(P, k0 + q, a1, a2, a3, f3)) + cor;
             const double Gn = __shfl_down_sync(full, G, 1);
             // valid for lanes 0..30 (lane 31's Gn is its own G; beyond n_p + 1, G = 0)
-            const double L = FAST ? c2 * fast_log_ratio(Gn, G) : c2 * log(Gn / G);
+            const double L = FAST ? c2 * fast_log_ratio(Gn, G) : c2 * log(div_rn(Gn, G, rcp_ulp(G)));
             const double Lm = __shfl_up_sync(full, L, 1);
             const double Lp = __shfl_down_sync(full, L, 1);
             const double Vm = __shfl_up_sync(full, V, 1);
@@ -184,16 +185,188 @@ __device__ __forceinline__ void mom_window(const P64 &P, const double *f, bool r
     }
 }
 
-// One unit: the kMomCols columns col0 .. col0 + kMomCols - 1 of the padded column list,
-// formed by warps 0 .. kMomCols - 1 and summed by warp kMomCols (wid: warp within the unit).
+// ---- windows that cannot change a sum
+// Most of a base patch's momentum range holds values many orders below the column's bulk
+// (a thermal f falls by 2^120 within 13 thermal widths; cells under a finer patch count for
+// nothing at all), and forming their contributions was most of the moments' work: about a
+// hundred FP64 instructions per cell and sub-column.  k64_mom_screen bounds |f| per window
+// and column, and a window whose every column lies 2^120 below its own largest value (or
+// is zero, or nested) is not formed.  That alone would be an approximation; what makes it
+// exact is the summing lane, which carries lower and upper bounds through the sum.  Added
+// to a sum more than 2^55 times larger, a skipped window's contributions leave it bit for
+// bit as it is; otherwise they widen the bounds by more than they could ever move the sum
+// (each rounded addition moves it by at most twice its addend), and, rounding being
+// monotone, the exact sum stays between the two when the same contributions are added to
+// both.  Once they meet (within a window of the bulk's first cells, where the sum has
+// outgrown what was skipped below it) they are the reference's sum; a column where they
+// do not (charge that cancels, a bulk of one cell) has its unit formed in full.
+// Contributions are bounded from F >= |f| over the window's cells and stencil: charge
+// |V| <= 8 F with the sub-cell interpolation (its weights sum to less than 7), F without;
+// current |V L + (L+ - L-)(V+ - V-) / 48| <= 1.09 |V| max|L| with |L| <= dp (the logarithm
+// of the node ratio grows by c1 dp / gamma per cell).
+struct MomSum {
+    double lo0 = 0.0, hi0 = 0.0, lo1 = 0.0, hi1 = 0.0;
+    __device__ __forceinline__ bool split() const { return !(lo0 == hi0 && lo1 == hi1); }
+    // a skipped window whose contributions are at most e in size each
+    static __device__ __forceinline__ void widen(double &lo, double &hi, double e) {
+        if (e == 0.0 || (lo == hi && e < fabs(lo) * 0x1p-55)) return;
+        lo = __dadd_rd(lo, -(2 * kMomOut + 4) * e);
+        hi = __dadd_ru(hi, (2 * kMomOut + 4) * e);
+    }
+    // kMomOut contributions in ascending p (both: the bounds have not met)
+    template <class A, class B>
+    __device__ __forceinline__ void add(bool both, bool two, A a, B b) {
+        if (!both) {
+            if (two) {
+#pragma unroll
+                for (int t = 1; t <= kMomOut; t++) {
+                    lo0 += a(t);
+                    lo1 += b(t);
+                }
+            } else {
+#pragma unroll
+                for (int t = 1; t <= kMomOut; t++) lo0 += a(t);
+            }
+            hi0 = lo0;
+            hi1 = lo1;
+        } else {
+            for (int t = 1; t <= kMomOut; t++) {
+                const double v = a(t);
+                lo0 += v;
+                hi0 += v;
+                if (two) {
+                    const double w = b(t);
+                    lo1 += w;
+                    hi1 += w;
+                }
+            }
+        }
+    }
+};
+
+// What a summing lane adds: of a pair of sub-columns, lane = 2 column + sub-column takes
+// the charge and the current; of a single one (rtb = 1), lanes 0 .. kMomCols-1 take the
+// charges and the next kMomCols the currents, so that one FP64 instruction adds both.
+struct MomLane {
+    bool on, two, cur;
+    int w, q;
+    double f0, f1;  // bounds of one contribution over F
+    __device__ __forceinline__ MomLane(const P64 &P, int kg, int lane) {
+        on = lane < 2 * kMomCols;
+        two = kg == 2;
+        cur = !two && lane >= kMomCols;
+        w = two ? lane >> 1 : (cur ? lane - kMomCols : lane);
+        if (!on) w = 0;
+        q = two ? lane & 1 : 0;
+        const double c = P.rtb > 1 ? 8.0 : 1.0, j = (P.rtb > 1 ? 10.0 : 1.25) * P.dp;
+        f0 = on ? (cur ? j : c) : 0.0;
+        f1 = on && two ? j : 0.0;
+    }
+    __device__ __forceinline__ void store(const MomLaunch &M, const P64 &P, int col0, int k0, const MomSum &s) const {
+        if (!on || M.colpatch[col0 + w] < 0) return;
+        const int cl = M.colidx[col0 + w] + k0 + q;  // i_w * rtb + k
+        const double qc = P.q;
+        if (!cur) P.chargeR[cl] = s.lo0 * (P.dp * qc);
+        if (two || cur) P.currentR[cl] = (two ? s.lo1 : s.lo0) * (-qc * qc / P.mass);
+    }
+};
+
+__device__ __forceinline__ int mom_windows(int np) { return (np + kMomOut - 1) / kMomOut; }
+
+// Per unit and window: a bound F >= |f| for each column over the window's cells and the
+// column's stencil, as the high word of a double (0: the column's contributions are all
+// zero), and in word kMomCols whether the window is formed.  One block per unit, a warp per
+// row of f: reads f once (4 rows of halo with the sub-cell interpolation), 22 MB and 10 us
+// on the 4096 x 512 two-level workload.
+__global__ void __launch_bounds__(256) k64_mom_screen(MomLaunch M) {
+    VX_PDL_WAIT();
+    extern __shared__ unsigned s_bound[];  // [row][window], bit 31 on a column's own row: none of its cells count
+    __shared__ unsigned s_max[kMomCols];
+    __shared__ int s_field[kMomCols];
+    const unsigned full = 0xffffffffu;
+    const int col0 = blockIdx.x * kMomCols, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const P64 &P = ((const P64 *)M.patches)[M.colpatch[col0]];
+    const int np = P.np, rtb = P.rtb, nwin = mom_windows(np), halo = rtb > 1 ? 2 : 0;
+    int ncol = 0;  // real columns: consecutive i, the padding at the end
+    while (ncol < kMomCols && M.colpatch[col0 + ncol] >= 0) ncol++;
+    const int i0 = M.colidx[col0] / rtb;
+    for (int r = wid; r < ncol + 2 * halo; r += 8) {
+        const int i = i0 - halo + r;
+        const bool own = r >= halo && r < halo + ncol;
+        for (int w = 0; w < nwin; w++) {
+            const int j = kMomOut * w - 1 + lane;
+            const double v = j <= np ? P.f1[pidx(i, j, P.pitch)] : 0.0;
+            const unsigned h = (unsigned)__double2hiint(v) & 0x7fffffffu;
+            const unsigned e = (h | (unsigned)__double2loint(v)) ? min(h + 1u, 0x7fffffffu) : 0u;
+            unsigned m = __reduce_max_sync(full, e);
+            if (own && P.nested) {
+                const bool counts = lane >= 1 && lane <= kMomOut && j < np && !P.nested[pidx(i, j, P.pitch)];
+                if (!__any_sync(full, counts)) m |= 0x80000000u;
+            }
+            if (lane == 0) s_bound[r * nwin + w] = m;
+        }
+    }
+    __syncthreads();
+    for (int c = threadIdx.x; c < ncol; c += 256) {
+        unsigned m = 0;
+        for (int w = 0; w < nwin; w++) m = max(m, s_bound[(c + halo) * nwin + w] & 0x7fffffffu);
+        s_max[c] = m;
+        bool fin = true;  // a field that is not finite makes every cell's current so
+        for (int k = 0; k < rtb; k++) fin = fin && isfinite(cell_asq(M.fields[P.run], (i0 + c + P.x_pos) * rtb + k));
+        s_field[c] = fin;
+    }
+    __syncthreads();
+    constexpr unsigned kFar = 120u << 20;  // 2^120 in the exponent of a high word
+    unsigned *out = M.screen + (size_t)blockIdx.x * M.maxnwin * kMomScreen;
+    for (int w = threadIdx.x; w < nwin; w += 256) {
+        unsigned form = 0;
+        for (int c = 0; c < kMomCols; c++) {
+            unsigned b = 0;
+            if (c < ncol && !(s_bound[(c + halo) * nwin + w] & 0x80000000u)) {
+                for (int r = c; r <= c + 2 * halo; r++) b = max(b, s_bound[r * nwin + w] & 0x7fffffffu);
+                if (!s_field[c] || (b && !(s_max[c] < 0x7ff00000u && b + kFar <= s_max[c]))) form = 1;
+            }
+            out[w * kMomScreen + c] = b;
+        }
+        out[w * kMomScreen + kMomCols] = form;
+    }
+}
+
+void launch_mom_screen64(const MomLaunch &M) {
+    if (M.ncols == 0) return;
+    const int smem = (kMomCols + 4) * M.maxnwin * (int)sizeof(unsigned);
+    if (smem > 200 * 1024) {  // n_p beyond 78000: every window formed
+        cudaMemsetAsync(M.screen, 1, (size_t)(M.ncols / kMomCols) * M.maxnwin * kMomScreen * sizeof(unsigned), M.stream);
+        return;
+    }
+    if (smem > 48 * 1024) cudaFuncSetAttribute(k64_mom_screen, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(M.ncols / kMomCols);
+    cfg.blockDim = dim3(256);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = M.stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributePriority;  // beside the face kernels of the other stream
+    attr[0].val.priority = M.priority;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = g_launch_pdl ? 2 : 1;
+    cudaLaunchKernelEx(&cfg, k64_mom_screen, M);  // errors surface through cudaGetLastError
+}
+
+// One unit: the kMomCols columns of unit `unit` of the padded column list, formed by warps
+// 0 .. kMomCols - 1 and summed by warp kMomCols (wid: warp within the unit).
 template <bool FAST>
-__device__ __forceinline__ void moments_unit(const MomLaunch &M, int col0, int wid, int lane, MomSmem &S, int bar) {
+__device__ __forceinline__ void moments_unit(const MomLaunch &M, int unit, int wid, int lane, MomSmem &S, int bar) {
+    const int col0 = unit * kMomCols;
     const bool summer = wid == kMomCols;  // the last warp adds; warps 0..kMomCols-1 form columns
     const bool real = !summer && M.colpatch[col0 + wid] >= 0;  // warp-uniform
     const P64 &P = ((const P64 *)M.patches)[M.colpatch[col0]];  // the unit's patch
-    const int np = P.np, rtb = P.rtb;
+    const int rtb = P.rtb, nwin = mom_windows(P.np);
     const int i = summer ? 0 : M.colidx[col0 + wid] / rtb;
     const RunFields &F = M.fields[P.run];
+    const unsigned *screen = M.screen + (size_t)unit * M.maxnwin * kMomScreen;
     const double minv = 1 / P.mass;
     const double c1 = minv * kCInv;
     const double c2 = 1 / c1;
@@ -204,49 +377,53 @@ __device__ __forceinline__ void moments_unit(const MomLaunch &M, int col0, int w
         double a[2] = {0.0, 0.0};
         for (int q = 0; q < kg; q++)
             if (real) a[q] = P.qq * cell_asq(F, (i + P.x_pos) * rtb + k0 + q);
-        // summing warp, lane t < kMomCols * kg: sub-column t % kg of column t / kg
-        double ch = 0.0, cu = 0.0;
-        auto add_window = [&](int bf) {
-            if (lane < kMomCols * kg) {
-                const int w = lane / kg, q = lane - w * kg;
-                const unsigned um = S.use[bf][w];
-                for (int t = 1; t <= kMomOut; t++)
-                    if ((um >> t) & 1u) {
-                        ch += S.cc[bf][w][q][t];
-                        cu += S.cj[bf][w][q][t];
-                    }
-            }
-        };
-        int bf = 0;
-        for (int j0 = 0; j0 < np; j0 += kMomOut, bf ^= 1) {
-            if (!summer) {
-                double cc[2], cj[2];
-                bool use;
-                mom_window<FAST>(P, f, real, i, j0, k0, kg, a, c1, c2, lane, cc, cj, use);
-                for (int q = 0; q < kg; q++) {
-                    S.cc[bf][wid][q][lane] = cc[q];
-                    S.cj[bf][wid][q][lane] = cj[q];
+        const MomLane ml(P, kg, lane);
+        for (int pass = 0; pass < 2; pass++) {  // pass 1: every window, where pass 0 did not settle
+            MomSum s;
+            bool both = false;
+            int next = 0;  // the summing warp's next window
+            // the skipped windows before `w`, then window w from buffer bf
+            auto add_to = [&](int w, int bf) {
+                for (; next < w; next++) {
+                    const double b = __hiloint2double((int)screen[next * kMomScreen + ml.w], 0);
+                    MomSum::widen(s.lo0, s.hi0, b * ml.f0);
+                    MomSum::widen(s.lo1, s.hi1, b * ml.f1);
                 }
-                const unsigned usemask = __ballot_sync(full, use);
-                if (lane == 0) S.use[bf][wid] = usemask;
-            } else if (j0 > 0) {
-                add_window(bf ^ 1);  // the previous window, in ascending j
+                if (w == nwin) return;
+                both = __any_sync(full, s.split());
+                const double *pc = ml.cur ? S.cj[bf][ml.w][0] : S.cc[bf][ml.w][ml.q], *pj = S.cj[bf][ml.w][ml.q];
+                s.add(both, ml.two, [&](int t) { return pc[t]; }, [&](int t) { return pj[t]; });
+                next = w + 1;
+            };
+            int bf = 0, prev = -1;
+            for (int w = 0; w < nwin; w++) {
+                if (!pass && !screen[w * kMomScreen + kMomCols]) continue;  // unit-uniform
+                if (!summer) {
+                    double cc[2], cj[2];
+                    bool use;
+                    mom_window<FAST>(P, f, real, i, w * kMomOut, k0, kg, a, c1, c2, lane, cc, cj, use);
+                    for (int q = 0; q < kg; q++) {
+                        S.cc[bf][wid][q][lane] = cc[q];
+                        S.cj[bf][wid][q][lane] = cj[q];
+                    }
+                } else if (prev >= 0) {
+                    add_to(prev, bf ^ 1);  // the previous window, in ascending j
+                }
+                prev = w;
+                bf ^= 1;
+                mom_sync(bar);
             }
+            if (summer) {
+                if (prev >= 0) add_to(prev, bf ^ 1);
+                add_to(nwin, 0);
+                const bool redo = !pass && __any_sync(full, ml.on && M.colpatch[col0 + ml.w] >= 0 && s.split());
+                if (lane == 0) S.redo = redo;
+                if (!redo) ml.store(M, P, col0, k0, s);
+            }
+            mom_sync(bar);  // the next pair's first window reuses the buffers
+            if (!S.redo) break;
             mom_sync(bar);
         }
-        if (summer) {
-            add_window(bf ^ 1);  // the last window
-            if (lane < kMomCols * kg) {
-                const int w = lane / kg, q = lane - w * kg;
-                if (M.colpatch[col0 + w] >= 0) {
-                    const int cl = M.colidx[col0 + w] + k0 + q;  // i_w * rtb + k
-                    const double qc = P.q;
-                    P.chargeR[cl] = ch * (P.dp * qc);
-                    P.currentR[cl] = cu * (-qc * qc / P.mass);
-                }
-            }
-        }
-        mom_sync(bar);  // the next pair's first window reuses the buffers
     }
 }
 
@@ -254,11 +431,12 @@ template <bool FAST>
 __global__ void __launch_bounds__(kMomThreads, 2) k64_moments(MomLaunch M) {
     VX_PDL_WAIT();
     __shared__ MomSmem S;
-    moments_unit<FAST>(M, blockIdx.x * kMomCols, threadIdx.x >> 5, threadIdx.x & 31, S, 0);
+    moments_unit<FAST>(M, blockIdx.x, threadIdx.x >> 5, threadIdx.x & 31, S, 0);
 }
 
 void launch_moments64(const MomLaunch &M) {
     if (M.ncols == 0) return;
+    launch_mom_screen64(M);
     // M.ncols is a multiple of kMomCols (the list is padded per patch)
     if (M.fast) vx_launch(k64_moments<true>, M.ncols / kMomCols, kMomThreads, 0, M.stream, M);
     else vx_launch(k64_moments<false>, M.ncols / kMomCols, kMomThreads, 0, M.stream, M);
@@ -848,34 +1026,55 @@ __device__ __forceinline__ void mom_item(const PipeLaunch &K, int u, int k0, int
         }
 }
 
-// The column sums of unit u (one warp, lane = sub-column as in k64_moments): every window's
+// The windows of unit u that the screen left out, formed by one warp (rare: see MomSum).
+template <bool FAST>
+__device__ __noinline__ void mom_form_rest(const PipeLaunch &K, int u, int k0, int lane) {
+    const unsigned *screen = K.M.screen + (size_t)(K.unit_col0[u] / kMomCols) * K.M.maxnwin * kMomScreen;
+    const int nw = K.unit_nwin[u];
+    for (int win = 0; win < nw; win++) {
+        if (screen[win * kMomScreen + kMomCols]) continue;
+        double *out = K.scratch + (size_t)(K.unit_item0[u] + (k0 / 2) * nw + win) * kPipeItemDoubles;
+        for (int wid = 0; wid < kMomCols; wid++) mom_item<FAST>(K, u, k0, win * kMomOut, wid, lane, out);
+    }
+    __threadfence();
+    __syncwarp();
+}
+
+// The column sums of unit u (one warp, lanes as MomLane has them): every formed window's
 // contributions in ascending p.  A cell that is not used contributes +0.0, which leaves a
 // sum that starts at +0.0 unchanged bit for bit (such a sum never becomes -0.0), so these
 // are the sums of the used cells alone.  Then the unit counts as done for its chunk.
-__device__ void mom_sum_unit(const PipeLaunch &K, int u, int lane) {
+template <bool FAST>
+__device__ __forceinline__ void mom_sum_unit(const PipeLaunch &K, int u, int lane) {
+    const unsigned full = 0xffffffffu;
     const MomLaunch &M = K.M;
     const int col0 = K.unit_col0[u];
     const P64 &P = ((const P64 *)M.patches)[M.colpatch[col0]];
+    const unsigned *screen = M.screen + (size_t)(col0 / kMomCols) * M.maxnwin * kMomScreen;
     const int rtb = P.rtb, nw = K.unit_nwin[u];
     for (int k0 = 0; k0 < rtb; k0 += 2) {
         const int kg = rtb - k0 < 2 ? rtb - k0 : 2;
-        if (lane < kMomCols * kg) {
-            const int w = lane / kg, q = lane - w * kg;
-            const double *src = K.scratch + (size_t)(K.unit_item0[u] + (k0 / 2) * nw) * kPipeItemDoubles + w * 2 + q;
-            double ch = 0.0, cu = 0.0;
+        const MomLane ml(P, kg, lane);
+        for (int pass = 0; pass < 2; pass++) {
+            const double *src = K.scratch + (size_t)(K.unit_item0[u] + (k0 / 2) * nw) * kPipeItemDoubles +
+                                (ml.cur ? 960 : 0) + ml.w * 2 + ml.q;
+            MomSum s;
             for (int win = 0; win < nw; win++, src += kPipeItemDoubles) {
-#pragma unroll
-                for (int t = 1; t <= kMomOut; t++) {
-                    ch += __ldcg(src + t * 30);
-                    cu += __ldcg(src + 960 + t * 30);
+                if (pass || screen[win * kMomScreen + kMomCols]) {
+                    s.add(__any_sync(full, s.split()), ml.two, [&](int t) { return __ldcg(src + t * 30); },
+                          [&](int t) { return __ldcg(src + 960 + t * 30); });
+                } else {
+                    const double b = __hiloint2double((int)screen[win * kMomScreen + ml.w], 0);
+                    MomSum::widen(s.lo0, s.hi0, b * ml.f0);
+                    MomSum::widen(s.lo1, s.hi1, b * ml.f1);
                 }
             }
-            if (M.colpatch[col0 + w] >= 0) {
-                const int cl = M.colidx[col0 + w] + k0 + q;  // i_w * rtb + k
-                const double qc = P.q;
-                P.chargeR[cl] = ch * (P.dp * qc);
-                P.currentR[cl] = cu * (-qc * qc / P.mass);
+            if (!pass && __any_sync(full, ml.on && M.colpatch[col0 + ml.w] >= 0 && s.split())) {
+                mom_form_rest<FAST>(K, u, k0, lane);
+                continue;
             }
+            ml.store(M, P, col0, k0, s);
+            break;
         }
     }
     __threadfence();  // the column sums, device-wide, before the count
@@ -895,25 +1094,44 @@ __device__ void pipe_columns(const PipeLaunch &K, int *ticket, int g) {
     const int bar = 1 + g, ncol = kMomCols * 32;
     unsigned *items_done = K.state + kPipeDone + K.ndone;      // per unit
     unsigned *queue = items_done + K.nunits;                    // completed units (u + 1), in order
+    // an item of unit u is done: the last one queues the unit
+    auto count = [&](int u) {
+        const unsigned total = (unsigned)(K.unit_item0[u + 1] - K.unit_item0[u]);
+        if (atomicAdd(items_done + u, 1u) + 1 == total) {
+            __threadfence();  // every item's contributions before a summing warp reads them
+            const unsigned slot = atomicAdd(K.state + kPipeQHead, 1u);
+            atomicExch(queue + slot, (unsigned)u + 1);
+        }
+    };
+    auto window = [&](int t, int u, int &kp) {
+        const int loc = t - K.unit_item0[u], nw = K.unit_nwin[u];
+        kp = loc / nw;
+        return loc - kp * nw;
+    };
     for (int it = 0;; it++) {
-        if (tid == 0) ticket[it & 1] = (int)atomicAdd(K.state + kPipeTicket, 1u);
+        if (tid == 0) {  // the next item whose window is formed
+            int t;
+            for (;;) {
+                t = (int)atomicAdd(K.state + kPipeTicket, 1u);
+                if (t >= K.nitems) break;
+                const int u = K.item_unit[t];
+                int kp;
+                const int w = window(t, u, kp);
+                if (K.M.screen[((size_t)(K.unit_col0[u] / kMomCols) * K.M.maxnwin + w) * kMomScreen + kMomCols]) break;
+                count(u);
+            }
+            ticket[it & 1] = t;
+        }
         pipe_bar(bar, ncol);
         const int t = ticket[it & 1];
         if (t >= K.nitems) break;
         const int u = K.item_unit[t];
-        const int loc = t - K.unit_item0[u], nw = K.unit_nwin[u];
-        const int kp = loc / nw;
-        mom_item<FAST>(K, u, 2 * kp, (loc - kp * nw) * kMomOut, wid, lane, K.scratch + (size_t)t * kPipeItemDoubles);
+        int kp;
+        const int w = window(t, u, kp);
+        mom_item<FAST>(K, u, 2 * kp, w * kMomOut, wid, lane, K.scratch + (size_t)t * kPipeItemDoubles);
         __threadfence();  // this warp's contributions, device-wide, before the item counts
         pipe_bar(bar, ncol);
-        if (tid == 0) {
-            const unsigned total = (unsigned)(K.unit_item0[u + 1] - K.unit_item0[u]);
-            if (atomicAdd(items_done + u, 1u) + 1 == total) {
-                __threadfence();  // every item's contributions before a summing warp reads them
-                const unsigned slot = atomicAdd(K.state + kPipeQHead, 1u);
-                atomicExch(queue + slot, (unsigned)u + 1);
-            }
-        }
+        if (tid == 0) count(u);
     }
 }
 
@@ -921,6 +1139,7 @@ __device__ void pipe_columns(const PipeLaunch &K, int *ticket, int g) {
 // the sub-partition's FP64 unit to themselves): takes completed units from the queue in
 // order and forms their column sums.  It waits only for units, which the column warps
 // always complete; a wait that runs out records itself and ends the warp.
+template <bool FAST>
 __device__ void pipe_summer(const PipeLaunch &K, int lane) {
     const unsigned full = 0xffffffffu;
     unsigned *queue = K.state + kPipeDone + K.ndone + K.nunits;
@@ -949,7 +1168,7 @@ __device__ void pipe_summer(const PipeLaunch &K, int lane) {
         v = __shfl_sync(full, v, 0);
         if (!v) break;
         __threadfence();
-        mom_sum_unit(K, (int)v - 1, lane);
+        mom_sum_unit<FAST>(K, (int)v - 1, lane);
     }
 }
 
@@ -969,7 +1188,7 @@ __global__ void __launch_bounds__(1024, 1) k64_moments_poisson(PipeLaunch K) {
             poisson_solve<true, true>(K.P, smem_raw, (double *)(smem_raw + 2 * sizeof(PoisChunk)), &K);
         else poisson_solve<false, true>(K.P, smem_raw, K.P.fields[blockIdx.x].phi, &K);
     } else if ((int)blockIdx.x < K.P.nruns + K.summers) {
-        if (threadIdx.x < 4 * 32) pipe_summer(K, (int)threadIdx.x & 31);  // warps 0..3: one per sub-partition
+        if (threadIdx.x < 4 * 32) pipe_summer<FAST>(K, (int)threadIdx.x & 31);  // warps 0..3: one per sub-partition
     } else {
         int *ticket = reinterpret_cast<int *>(smem_raw);
         const int g = (int)threadIdx.x / kMomThreads;

@@ -107,11 +107,18 @@ struct MomLaunch {
     int acell = 1;        // FP32: refresh the per-cell A^2 copy first (else the Maxwell stage made it)
     int asq32 = 1;        // FP32: the moments kernel also makes the FP32 copy of a^2
     int fast = 0;         // FP64: the fast form's moments (fused multiply-adds, Newton reciprocal)
+    // FP64: per unit (kMomCols columns) and p window kMomScreen words, written by the screen
+    // launch: a bound on |f| for each column and whether the window is formed (fields64.cu)
+    unsigned *screen = nullptr;
+    int maxnwin = 0;      // windows per unit in `screen`
+    int priority = 0;     // FP64: launch priority of the screen (0: the stream's)
     cudaStream_t stream;
 };
+constexpr int kMomScreen = 16;
 constexpr int kMomCols = 15;  // FP64 moment columns per block (padded per patch), plus a summing warp
 constexpr int kMomWindow = 29;  // p cells per window of the FP64 moments (a warp's lanes 1..29)
-void launch_moments64(const MomLaunch &M);
+void launch_moments64(const MomLaunch &M);  // the screen and the moments: two launches
+void launch_mom_screen64(const MomLaunch &M);
 void launch_moments32(const MomLaunch &M);
 
 // Assembly of rho and J on the finest grid (EMSolver::AssembleRhoAndJ).
