@@ -49,6 +49,7 @@ std::pair<int, int> Engine::autotune(const std::vector<Run *> &set, int reps) {
         fl.ptiles = L.dptiles.as<TileRef>();
         fl.nxtiles = L.nxtiles;
         fl.nptiles = L.nptiles;
+        fl.strip_rows = L.strip_rows;
         fl.tile_j = L.tile_j;
         fl.tile_i = L.tile_i;
         run_subs();  // warm-up

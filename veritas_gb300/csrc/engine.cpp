@@ -176,6 +176,7 @@ void Run::upload_rect_desc(Rect &r, int run_index) {
     d.dx = s.GetDx(r.depth);
     d.dx_inv = 1 / d.dx;
     d.dp_inv = 1 / d.dp;
+    d.rtb_inv = 1.0 / d.rtb;
     d.pmin = s.pmin[sp];
     d.q = s.GetCharge(sp);
     d.qq = d.q * d.q;
@@ -619,6 +620,7 @@ std::vector<double> Engine::profile_kernels(Run &run, int reps) {
     fl.ptiles = L.dptiles.as<TileRef>();
     fl.nxtiles = L.nxtiles;
     fl.nptiles = L.nptiles;
+    fl.strip_rows = L.strip_rows;
     fl.fields = L.dfields.as<RunFields>();
     fl.params = L.dparams.as<double>();
     fl.params32 = L.dparams32.as<float>();
@@ -893,15 +895,26 @@ void Engine::build_tiles(LaunchSet &L, TablePack *pk) {
     L.ntiles = (int)tiles.size();
     P.put(L.dtiles, tiles);
     if (L.precision == kF32) {  // strip tiles of the fused face + flux kernels
+        // Rows per strip: a warp walks its strip's rows one after another and shares work
+        // between them, so large sets take 16 (38.6 M cells: p fluxes 254 us, 278 with 8, 432
+        // with 2); a set that cannot give every SM sixteen such warps takes shorter ones,
+        // down to 2 (1062 x 130: 12.4 us with 16 rows, 7.6 with 8, 5.4 with 4, 4.4 with 2).
+        long long row_warps = 0;
+        for (Run *R : L.runs)
+            for (auto &sp : R->rects)
+                for (auto &lvl : sp)
+                    for (auto &rp : lvl) row_warps += (long long)rp->n_x * ((rp->n_p + 31) / 32);
+        L.strip_rows = kMaxStripRows;
+        while (L.strip_rows > 2 && row_warps / L.strip_rows < 16LL * num_sms_) L.strip_rows /= 2;
         std::vector<TileRef> xt, pt;
         pi = 0;
         for (Run *R : L.runs)
             for (auto &sp : R->rects)
                 for (auto &lvl : sp)
                     for (auto &rp : lvl) {
-                        for (int i0 = 0; i0 <= rp->n_x; i0 += kStripRows)
+                        for (int i0 = 0; i0 <= rp->n_x; i0 += L.strip_rows)
                             for (int j0 = -1; j0 <= rp->n_p; j0 += kXCols) xt.push_back({pi, i0, j0});
-                        for (int i0 = -1; i0 <= rp->n_x; i0 += kStripRows)
+                        for (int i0 = -1; i0 <= rp->n_x; i0 += L.strip_rows)
                             for (int j0 = 0; j0 <= rp->n_p; j0 += 32) pt.push_back({pi, i0, j0});
                         pi++;
                     }
@@ -1290,6 +1303,7 @@ StageLaunches Engine::stage_launches(LaunchSet &L) {
     fl.ptiles = L.dptiles.as<TileRef>();
     fl.nxtiles = L.nxtiles;
     fl.nptiles = L.nptiles;
+    fl.strip_rows = L.strip_rows;
     fl.fields = L.dfields.as<RunFields>();
     fl.params = L.dparams.as<double>();
     fl.params32 = L.dparams32.as<float>();

@@ -270,7 +270,7 @@ struct LaunchSet {
     int precision = kF64;
     int tile_j = 32, tile_i = 8;  // FCT tile (p x x) = thread block of the sub-step kernels
     DevBuf dxtiles, dptiles;      // FP32: strip tiles of the fused face + flux kernels
-    int nxtiles = 0, nptiles = 0;
+    int nxtiles = 0, nptiles = 0, strip_rows = kMaxStripRows;
     int poisson = kPoissonLU;
     int fast64 = 0;  // FP64 sets: contracted FCT kernels
     DevBuf dpf;  // per-run PoissonFastDev (scan Poisson sets)

@@ -31,18 +31,18 @@ __global__ void k32_copy10(const P32 *patches, const TileRef *tiles) {
 
 // Fused face + flux sub-steps: one warp per strip tile (whole warps leave together).
 __global__ void k32_xflux(const P32 *patches, const TileRef *tiles, int ntiles, const RunFields *fields, int step,
-                          int use_f0) {
+                          int use_f0, int strip) {
     VX_PDL_WAIT();
     const int wt = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (wt >= ntiles) return;
-    xflux32(patches, tiles[wt], threadIdx.x & 31, fields, step, use_f0);
+    xflux32(patches, tiles[wt], threadIdx.x & 31, fields, step, use_f0, strip);
 }
 __global__ void k32_pflux(const P32 *patches, const TileRef *tiles, int ntiles, const RunFields *fields, int step,
-                          int use_f0) {
+                          int use_f0, int strip) {
     VX_PDL_WAIT();
     const int wt = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (wt >= ntiles) return;
-    pflux32(patches, tiles[wt], threadIdx.x & 31, fields, step, use_f0);
+    pflux32(patches, tiles[wt], threadIdx.x & 31, fields, step, use_f0, strip);
 }
 
 void launch_fct32_substep(const FctLaunch &L, int sub) {
@@ -67,10 +67,10 @@ void launch_fct32_substep(const FctLaunch &L, int sub) {
             vx_launch(k32_copy10, L.ntiles, blk, 0, L.stream, pp, L.tiles);
             break;
         case kSubXFlux:
-            if (L.nxtiles) vx_launch(k32_xflux, (L.nxtiles + 3) / 4, 128, 0, L.stream, pp, L.xtiles, L.nxtiles, L.fields, L.step, L.use_f0);
+            if (L.nxtiles) vx_launch(k32_xflux, (L.nxtiles + 3) / 4, 128, 0, L.stream, pp, L.xtiles, L.nxtiles, L.fields, L.step, L.use_f0, L.strip_rows);
             break;
         case kSubPFlux:
-            if (L.nptiles) vx_launch(k32_pflux, (L.nptiles + 3) / 4, 128, 0, L.stream, pp, L.ptiles, L.nptiles, L.fields, L.step, L.use_f0);
+            if (L.nptiles) vx_launch(k32_pflux, (L.nptiles + 3) / 4, 128, 0, L.stream, pp, L.ptiles, L.nptiles, L.fields, L.step, L.use_f0, L.strip_rows);
             break;
         default:  // the FP32 form has no separate gamma / face / flux sub-steps (fused above)
             break;

@@ -316,11 +316,17 @@ struct FluxView {
     }
 };
 
+// Empty phase space.  f underflows to 0 in FP32 thirteen thermal widths from its centre and
+// is 0 outside the plasma, so on most of a base patch (83 % of the cells of the 0.5 keV
+// wakefield case's, 60 % at 1 keV) every f a warp's row reads is 0, and with it the
+// face values and the fluxes.  One vote per row finds that out, and the row's Lorentz
+// factors, velocities and weights — the bulk of these issue-bound kernels — are not formed.
+
 // x direction: a warp covers kXCols output columns j0 .. j0+29 (its 32 lanes hold the
-// face values of j0-1 .. j0+30) over kStripRows rows; rows are independent in x, and the
+// face values of j0-1 .. j0+30) over `strip` rows; rows are independent in x, and the
 // four rows of f a face reads (i-2 .. i+1) slide down the strip, one new load per row.
 __device__ __forceinline__ void xflux32(const P32 *patches, const TileRef t, int lane, const RunFields *fields,
-                                       int step, int use_f0) {
+                                       int step, int use_f0, int strip) {
     const P32 &P = patches[t.patch];
     const int pit = P.pitch;
     const float *f = use_f0 ? P.f0 : P.f1;
@@ -340,14 +346,28 @@ __device__ __forceinline__ void xflux32(const P32 *patches, const TileRef t, int
     }
     // q^2 A^2 / (m c)^2 of row i0 + k, formed once by lane k and taken by shuffle
     const float a_l = asq32(P, F, t.i0 + lane);
-    for (int r = 0; r < kStripRows; r++) {
+    // whether any lane's f of the four rows is not zero (bit k: row i - 2 + k)
+    unsigned live = (__any_sync(full, fa != 0.0f) ? 1u : 0u) | (__any_sync(full, fb != 0.0f) ? 2u : 0u) |
+                    (__any_sync(full, fc != 0.0f) ? 4u : 0u);
+    for (int r = 0; r < strip; r++, live >>= 1) {
         const int i = t.i0 + r;
         if (i > P.nx) break;  // warp-uniform
         const int id = pidx(i, jj, pit);
         float am = 0.0f, fv = 0.0f, fd = 0.0f;
+        if (col_ok) fd = f[id + pit];  // row i+1 <= nx+1
+        if (__any_sync(full, fd != 0.0f)) live |= 8u;
+        if (!live) {
+            if (lane >= 1 && lane <= kXCols && col_ok && !(P.ifx && P.ifx[id])) {
+                P.FxH[step][id] = 0.0f;
+                if (step == 0) P.FxL[id] = 0.0f;
+            }
+            fa = fb;
+            fb = fc;
+            fc = fd;
+            continue;
+        }
         const float a = __shfl_sync(full, a_l, r);
         if (col_ok) {
-            fd = f[id + pit];  // row i+1 <= nx+1
             const float g0 = sqrt_ge1(1.0f + p0 * p0 + a), g1 = sqrt_ge1(1.0f + p1 * p1 + a);
             am = P.kxf * __fdividef(P.dpnf * (p1 + p0), g1 + g0);
             fv = weno32(fa, fb, fc, fd, am > 0.0f, P.weno_eps);
@@ -364,7 +384,7 @@ __device__ __forceinline__ void xflux32(const P32 *patches, const TileRef t, int
     }
 }
 
-// p direction: a warp covers 32 columns over kStripRows output rows, walking down with
+// p direction: a warp covers 32 columns over `strip` output rows, walking down with
 // the face values of the previous and next rows in registers.  Face row i reads a^2 and
 // gamma at x-faces i and i+1; the i+1 pair is the next row's i pair, so it is carried.
 struct PRow {
@@ -374,20 +394,27 @@ __device__ __forceinline__ void pface32(const FluxView &V, int i, int j, bool co
                                         const PRow &hi, float qe, float &am, float &fv) {
     am = 0.0f;
     fv = 0.0f;
-    if (!col_ok || i < -1 || i > V.nx) return;
-    am = qe - V.kpf * __fdividef(hi.a - lo.a, hi.g + lo.g);
-    const int id = pidx(i, j, V.pit);
-    const float *f = V.f;
-    fv = weno32(f[id - 2], f[id - 1], f[id], f[id + 1], am > 0.0f, V.weno_eps);
+    const bool ok = col_ok && i >= -1 && i <= V.nx;
+    float f1 = 0.0f, f2 = 0.0f, f3 = 0.0f, f4 = 0.0f;
+    if (ok) {
+        const float *f = V.f + pidx(i, j, V.pit);
+        f1 = f[-2];
+        f2 = f[-1];
+        f3 = f[0];
+        f4 = f[1];
+        am = qe - V.kpf * __fdividef(hi.a - lo.a, hi.g + lo.g);
+    }
+    const bool live = __any_sync(0xffffffffu, f1 != 0.0f || f2 != 0.0f || f3 != 0.0f || f4 != 0.0f);
+    if (live && ok) fv = weno32(f1, f2, f3, f4, am > 0.0f, V.weno_eps);
 }
 
 // The row quantities — q^2 A^2 / (m c)^2 at x-faces i0-1 .. i0+rows+1 and q<E_x> of rows
 // i0-1 .. i0+rows — are the same for every lane: lane k forms those of row i0-1+k once
-// (k <= kStripRows + 2 < 32) and each row takes them by shuffle, instead of every lane
+// (k <= strip + 2 < 32) and each row takes them by shuffle, instead of every lane
 // forming every row's (their index clamping and the periodic E_x average were most of the
 // kernel's integer instructions).
 __device__ __forceinline__ void pflux32(const P32 *patches, const TileRef t, int lane, const RunFields *fields,
-                                       int step, int use_f0) {
+                                       int step, int use_f0, int strip) {
     const unsigned full = 0xffffffffu;
     const P32 &P = patches[t.patch];
     const FluxView V(P, fields[P.run], step, use_f0);
@@ -398,7 +425,7 @@ __device__ __forceinline__ void pflux32(const P32 *patches, const TileRef t, int
     const int ir = t.i0 - 1 + lane;
     const float a_l = V.asq_at(ir);
     const float qe_l = (ir >= -1 && ir <= V.nx) ? V.qe_at(ir) : 0.0f;
-    auto prow = [&](int i) {  // i - (i0 - 1) in 0 .. kStripRows + 2
+    auto prow = [&](int i) {  // i - (i0 - 1) in 0 .. strip + 2
         const float a = __shfl_sync(full, a_l, i - (t.i0 - 1));
         return PRow{a, sqrt_ge1(1.0f + p * p + a)};
     };
@@ -407,7 +434,7 @@ __device__ __forceinline__ void pflux32(const P32 *patches, const TileRef t, int
     float amA, fvA, amB, fvB;  // rows i-1 and i
     pface32(V, t.i0 - 1, j, col_ok, r0, r1, qe(t.i0 - 1), amA, fvA);
     pface32(V, t.i0, j, col_ok, r1, r2, qe(t.i0), amB, fvB);
-    const int rows = min(kStripRows, V.nx + 1 - t.i0);
+    const int rows = min(strip, V.nx + 1 - t.i0);
     for (int r = 0; r < rows; r++) {
         const int i = t.i0 + r;
         const PRow r3 = prow(i + 2);

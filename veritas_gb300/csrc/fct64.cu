@@ -178,7 +178,7 @@ __device__ __forceinline__ double patch_efield(const P64 &P, const RunFields &F,
         y = (y < F.n) ? y : (y - F.n);
         t += F.efin[y];
     }
-    return t * (1.0 / P.rtb);
+    return t * P.rtb_inv;
 }
 
 __device__ __forceinline__ double a_sq_face(const P64 &P, const RunFields &F, int i) {
@@ -216,14 +216,14 @@ __global__ void k64_faces(const P64 *patches, const TileRef *tiles, const RunFie
     const double *f = use_f0 ? P.f0 : P.f1;
     const double *g = P.gam;
     if ((part & 1) && i >= 0 && i <= P.nx && j >= -1 && j <= P.np) {
-        double am = P.dp_inv * P.cc * (g[pidx(i, j + 1, pit)] - g[id]);
+        double am = P.kx * (g[pidx(i, j + 1, pit)] - g[id]);
         P.ex[id] = am;
         P.fx[id] = weno_face(f[pidx(i - 2, j, pit)], f[pidx(i - 1, j, pit)], f[id], f[pidx(i + 1, j, pit)], gt0(am));
     }
     if ((part & 2) && i >= -1 && i <= P.nx && j >= 0 && j <= P.np) {
         const RunFields &F = fields[P.run];
         double Em = P.q * patch_efield(P, F, i);
-        double am = Em - P.cc * P.dx_inv * (g[pidx(i + 1, j, pit)] - g[id]);
+        double am = Em - P.kp * (g[pidx(i + 1, j, pit)] - g[id]);
         P.ep[id] = am;
         P.fp[id] = weno_face(f[pidx(i, j - 2, pit)], f[pidx(i, j - 1, pit)], f[id], f[pidx(i, j + 1, pit)], gt0(am));
     }
@@ -240,7 +240,7 @@ __global__ void k64_faces(const P64 *patches, const TileRef *tiles, const RunFie
     if ((part & 8) && i >= -1 && i <= P.nx && j >= 0 && j <= P.np) {
         const RunFields &F = fields[P.run];
         double Em = P.q * patch_efield(P, F, i);
-        double am = Em - P.cc * P.dx_inv * (g[pidx(i + 1, j, pit)] - g[id]);
+        double am = Em - P.kp * (g[pidx(i + 1, j, pit)] - g[id]);
         P.ep[id] = am;
         if (!gt0(am)) P.fp[id] = P.Rp[id];
     }

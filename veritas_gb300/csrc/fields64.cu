@@ -42,7 +42,7 @@ __device__ __forceinline__ void rel_shared(const P64 &P, const double *f, int i,
         double v = P.relc[3 * q] * a1 + P.relc[3 * q + 1] * a2 + P.relc[3 * q + 2] * a3 + f3;
         te += v;
     }
-    cor = f3 - (1.0 / (double)P.rtb) * te;
+    cor = f3 - P.rtb_inv * te;
 }
 __device__ __forceinline__ double rel_pick(const P64 &P, int k, double a1, double a2, double a3, double f3) {
     return P.relc[3 * k] * a1 + P.relc[3 * k + 1] * a2 + P.relc[3 * k + 2] * a3 + f3;
@@ -64,7 +64,7 @@ __device__ __forceinline__ void rel_shared_fma(const P64 &P, const double *f, in
     double te = 0.0;
     for (int q = 0; q < P.rtb; q++)
         te += __fma_rn(P.relc[3 * q + 2], a3, __fma_rn(P.relc[3 * q + 1], a2, __fma_rn(P.relc[3 * q], a1, f3)));
-    cor = __fma_rn(-1.0 / (double)P.rtb, te, f3);
+    cor = __fma_rn(-P.rtb_inv, te, f3);
 }
 __device__ __forceinline__ double rel_pick_fma(const P64 &P, int k, double a1, double a2, double a3, double f3) {
     return __fma_rn(P.relc[3 * k + 2], a3, __fma_rn(P.relc[3 * k + 1], a2, __fma_rn(P.relc[3 * k], a1, f3)));
@@ -187,11 +187,11 @@ __device__ __forceinline__ void mom_window(const P64 &P, const double *f, bool r
 
 // ---- windows that cannot change a sum
 // Most of a base patch's momentum range holds values many orders below the column's bulk
-// (a thermal f falls by 2^120 within 13 thermal widths; cells under a finer patch count for
+// (a thermal f falls by 2^96 within 12 thermal widths; cells under a finer patch count for
 // nothing at all), and forming their contributions was most of the moments' work: about a
 // hundred FP64 instructions per cell and sub-column.  k64_mom_screen bounds |f| per window
-// and column, and a window whose every column lies 2^120 below its own largest value (or
-// is zero, or nested) is not formed.  That alone would be an approximation; what makes it
+// and column, and a window whose every column lies 2^96 below its own largest value that
+// counts (or is zero, or nested) is not formed.  That alone would be an approximation; what makes it
 // exact is the summing lane, which carries lower and upper bounds through the sum.  Added
 // to a sum more than 2^55 times larger, a skipped window's contributions leave it bit for
 // bit as it is; otherwise they widen the bounds by more than they could ever move the sum
@@ -199,7 +199,9 @@ __device__ __forceinline__ void mom_window(const P64 &P, const double *f, bool r
 // monotone, the exact sum stays between the two when the same contributions are added to
 // both.  Once they meet (within a window of the bulk's first cells, where the sum has
 // outgrown what was skipped below it) they are the reference's sum; a column where they
-// do not (charge that cancels, a bulk of one cell) has its unit formed in full.
+// do not (charge that cancels, a bulk of one cell) has its unit formed in full.  What is
+// skipped is below 2^-87 of the sum, an ulp 2^-52 of it: by chance that happens to one sum
+// in 2^34.
 // Contributions are bounded from F >= |f| over the window's cells and stencil: charge
 // |V| <= 8 F with the sub-cell interpolation (its weights sum to less than 7), F without;
 // current |V L + (L+ - L-)(V+ - V-) / 48| <= 1.09 |V| max|L| with |L| <= dp (the logarithm
@@ -281,7 +283,7 @@ __device__ __forceinline__ int mom_windows(int np) { return (np + kMomOut - 1) /
 __global__ void __launch_bounds__(256) k64_mom_screen(MomLaunch M) {
     VX_PDL_WAIT();
     extern __shared__ unsigned s_bound[];  // [row][window], bit 31 on a column's own row: none of its cells count
-    __shared__ unsigned s_max[kMomCols];
+    __shared__ unsigned s_max[kMomCols];   // per column: largest |f| of the cells that count
     __shared__ int s_field[kMomCols];
     const unsigned full = 0xffffffffu;
     const int col0 = blockIdx.x * kMomCols, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -293,6 +295,7 @@ __global__ void __launch_bounds__(256) k64_mom_screen(MomLaunch M) {
     for (int r = wid; r < ncol + 2 * halo; r += 8) {
         const int i = i0 - halo + r;
         const bool own = r >= halo && r < halo + ncol;
+        unsigned top = 0;
         for (int w = 0; w < nwin; w++) {
             const int j = kMomOut * w - 1 + lane;
             const double v = j <= np ? P.f1[pidx(i, j, P.pitch)] : 0.0;
@@ -301,22 +304,23 @@ __global__ void __launch_bounds__(256) k64_mom_screen(MomLaunch M) {
             unsigned m = __reduce_max_sync(full, e);
             if (own && P.nested) {
                 const bool counts = lane >= 1 && lane <= kMomOut && j < np && !P.nested[pidx(i, j, P.pitch)];
+                top = max(top, __reduce_max_sync(full, counts ? e : 0u));
                 if (!__any_sync(full, counts)) m |= 0x80000000u;
+            } else {
+                top = max(top, m);
             }
             if (lane == 0) s_bound[r * nwin + w] = m;
         }
+        if (own && lane == 0) s_max[r - halo] = top;
     }
     __syncthreads();
     for (int c = threadIdx.x; c < ncol; c += 256) {
-        unsigned m = 0;
-        for (int w = 0; w < nwin; w++) m = max(m, s_bound[(c + halo) * nwin + w] & 0x7fffffffu);
-        s_max[c] = m;
         bool fin = true;  // a field that is not finite makes every cell's current so
         for (int k = 0; k < rtb; k++) fin = fin && isfinite(cell_asq(M.fields[P.run], (i0 + c + P.x_pos) * rtb + k));
         s_field[c] = fin;
     }
     __syncthreads();
-    constexpr unsigned kFar = 120u << 20;  // 2^120 in the exponent of a high word
+    constexpr unsigned kFar = 96u << 20;  // 2^96 in the exponent of a high word
     unsigned *out = M.screen + (size_t)blockIdx.x * M.maxnwin * kMomScreen;
     for (int w = threadIdx.x; w < nwin; w += 256) {
         unsigned form = 0;

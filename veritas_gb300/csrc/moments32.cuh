@@ -121,18 +121,31 @@ __device__ __forceinline__ void moments_group(const P32 &P, const RunFields &F, 
             const float pn = fmaf(dpn, (float)(j + 1 + P.p_pos), pmin);
             // interpolation's shared part (Rectangle.cpp:139-155, 183-204)
             float f3 = 0.0f, a1 = 0.0f, a2 = 0.0f, a3 = 0.0f, fmean = 0.0f;
+            float e1 = 0.0f, e2 = 0.0f, e4 = 0.0f, e5 = 0.0f;
             if (j <= P.np) {
                 f3 = f[pidx(i, j, pit)];
                 if (rtb > 1) {
-                    const float g1 = f[pidx(i - 2, j, pit)] - f3, g2 = f[pidx(i - 1, j, pit)] - f3;
-                    const float g4 = f[pidx(i + 1, j, pit)] - f3, g5 = f[pidx(i + 2, j, pit)] - f3;
+                    e1 = f[pidx(i - 2, j, pit)];
+                    e2 = f[pidx(i - 1, j, pit)];
+                    e4 = f[pidx(i + 1, j, pit)];
+                    e5 = f[pidx(i + 2, j, pit)];
+                }
+            }
+            // nothing in this window (f underflows to 0 thirteen thermal widths out, and is 0
+            // outside the plasma), or nothing that counts (cells under a finer patch): its
+            // contributions are zeros, which leave a compensated sum as it is
+            const bool use = lane >= 1 && lane <= kMom32Out && j < P.np && !(P.nested && P.nested[pidx(i, j, pit)]);
+            const bool some = f3 != 0.0f || e1 != 0.0f || e2 != 0.0f || e4 != 0.0f || e5 != 0.0f;
+            if (!__any_sync(full, some) || !__any_sync(full, use)) continue;
+            if (j <= P.np) {
+                if (rtb > 1) {
+                    const float g1 = e1 - f3, g2 = e2 - f3, g4 = e4 - f3, g5 = e5 - f3;
                     a1 = 0.104166666666667f * g1 - 0.708333333333334f * g2 + 0.708333333333334f * g4 - 0.104166666666667f * g5;
                     a2 = 0.117647058823529f * g1 + 0.029411764705882f * g2 + 0.029411764705882f * g4 + 0.117647058823529f * g5;
                     a3 = -0.083333333333333f * g1 + 0.166666666666667f * g2 - 0.166666666666667f * g4 + 0.083333333333334f * g5;
                     fmean = (s0 * a1 + s1 * a2 + s2 * a3) * inv_rtb + f3;
                 }
             }
-            const bool use = lane >= 1 && lane <= kMom32Out && j < P.np && !(P.nested && P.nested[pidx(i, j, pit)]);
 #pragma unroll
             for (int q = 0; q < KG; q++) {
                 const float s = 1.0f + p * p + a[q];

@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(kStageThreads, 5) k32_stage_pre(Stage32Launch 
     const P32 *patches = (const P32 *)F.patches;
     for_warp_units(L.sync, M.ncols + F.nxtiles, [&](int u) {
         if (u < M.ncols) moments32_column(M, u, lane);
-        else xflux32(patches, F.xtiles[u - M.ncols], lane, F.fields, L.step, F.use_f0);
+        else xflux32(patches, F.xtiles[u - M.ncols], lane, F.fields, L.step, F.use_f0, F.strip_rows);
     });
     bar.sync();
     const AsmLaunch &A = L.al;
@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(kStageThreads, 5) k32_stage_fct(Stage32Launch 
     const long long mxn = (long long)X.nruns * X.maxnf;
     // p fluxes (Rectangle.cpp:1326-1394; E_x from the solve) | Maxwell right-hand side
     for_cells(mxn, [&](long long e) { mx_rhs_cell(X, (int)(e / X.maxnf), (int)(e % X.maxnf)); });
-    for_warp_units(L.sync, F.nptiles, [&](int w) { pflux32(patches, F.ptiles[w], lane, F.fields, s, F.use_f0); });
+    for_warp_units(L.sync, F.nptiles, [&](int w) { pflux32(patches, F.ptiles[w], lane, F.fields, s, F.use_f0, F.strip_rows); });
     bar.sync();
     // coarse faces on coarse/fine interfaces, batch by batch
     for (int b = 0; b < L.niface_b; b++) {

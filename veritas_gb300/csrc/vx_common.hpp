@@ -52,11 +52,11 @@ struct PatchT {
     int run, species;
     int has_iface;          // any coarse/fine interface face on this patch
     int r;                  // refinement ratio
-    double dx, dp, dx_inv, dp_inv;
+    double dx, dp, dx_inv, dp_inv, rtb_inv;  // rtb_inv = 1 / rtb
     double pmin, q, qq, mass, cc, g2;  // qq=q*q, cc=cs*cs*m, g2=(m_inv*c_inv)^2
     // FP32 precision form: f is stored as f * fnorm; pnorm = 1/(m c) makes momenta
     // dimensionless (dpn = dp * pnorm); kx = c^2 m / dp and kp = c^2 m / dx scale the
-    // rationalised Lorentz-factor differences into face velocities; weno_eps is the WENO
+    // Lorentz-factor differences (rationalised in FP32) into face velocities; weno_eps is the WENO
     // regulariser in the scaled units.
     double fnorm, pnorm, dpn, kx, kp;
     float weno_eps;

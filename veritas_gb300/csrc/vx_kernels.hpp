@@ -84,10 +84,10 @@ struct FctLaunch {
     int tile_j, tile_i;  // thread block = one tile of tile_j (p) x tile_i (x) cells
     // FP32 fused face + flux kernels: one warp per strip tile
     const TileRef *xtiles, *ptiles;
-    int nxtiles, nptiles;
+    int nxtiles, nptiles, strip_rows;
     cudaStream_t stream;
 };
-constexpr int kStripRows = 16;  // rows per strip tile of the fused FP32 face + flux kernels
+constexpr int kMaxStripRows = 16;  // rows per strip tile of the fused FP32 face + flux kernels, at most
 constexpr int kXCols = 30;      // output columns per x strip (32 lanes hold j0-1 .. j0+30)
 
 void launch_fct64_substep(const FctLaunch &L, int sub);
