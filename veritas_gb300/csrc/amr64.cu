@@ -16,10 +16,10 @@ __global__ void k_ghost(const PatchT<T> *patches, const GhostOp *ops, int n, int
     if (k < n) ghost_op(patches, ops, k, slot);
 }
 template <class T>
-__global__ void k_iface(const PatchT<T> *patches, const IfaceOp *ops, int n, int step) {
+__global__ void k_iface(const PatchT<T> *patches, const IfaceOp *ops, int n, int step, const double *params) {
     VX_PDL_WAIT();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < n) iface_op(patches, ops, k, step);
+    if (k < n) iface_op(patches, ops, k, step, params);
 }
 template <class T>
 __global__ void k_csync(const PatchT<T> *patches, const CSyncOp *ops, int n) {
@@ -161,10 +161,10 @@ void launch_ghost(const void *patches, const GhostOp *ops, int n, int slot, int 
     else vx_launch(k_ghost<double>, (n + 127) / 128, 128, 0, s, (const PatchT<double> *)patches, ops, n, slot);
 }
 
-void launch_iface(const void *patches, const IfaceOp *ops, int n, int step, int prec, cudaStream_t s) {
+void launch_iface(const void *patches, const IfaceOp *ops, int n, int step, const double *params, int prec, cudaStream_t s) {
     if (n <= 0) return;
     if (prec == kF32) launch_iface32(patches, ops, n, step, s);
-    else vx_launch(k_iface<double>, (n + 127) / 128, 128, 0, s, (const PatchT<double> *)patches, ops, n, step);
+    else vx_launch(k_iface<double>, (n + 127) / 128, 128, 0, s, (const PatchT<double> *)patches, ops, n, step, params);
 }
 
 void launch_csync(const void *patches, const CSyncOp *ops, int n, int prec, cudaStream_t s) {

@@ -99,8 +99,21 @@ __device__ __forceinline__ void ghost_op(const PatchT<T> *patches, const GhostOp
 // the r fine faces (CalculateFluxToCoarse*, Rectangle.hpp:132-178).  The high-order mean
 // uses the fine patch's stage fluxes; the stage-0 low-order mean recomputes each fine
 // donor-cell flux the way RGKGetFluxXL/PL do, (dx_inv * f) * a (Rectangle.cpp:1216-1253).
+// FP64: the face's antidiffusive stage flux (what the flux kernels form for all other
+// faces) follows from its stage fluxes so far; the FP32 form has a pass for it.
 template <class T>
-__device__ __forceinline__ void iface_op(const PatchT<T> *patches, const IfaceOp *ops, int k, int step) {
+__device__ __forceinline__ T stage_flux(T *const *H, int id, const double *a, int step, T low) {
+    T h = a[0] * H[0][id];
+    for (int k = 1; k <= step; k++) {
+        if (step == 5 && k == 1) continue;  // b_1 = 0 (Rectangle.cpp:1494)
+        h = h + a[k] * H[k][id];
+    }
+    return h - a[6] * low;
+}
+
+template <class T>
+__device__ __forceinline__ void iface_op(const PatchT<T> *patches, const IfaceOp *ops, int k, int step,
+                                         const double *params) {
     const IfaceOp op = ops[k];
     const PatchT<T> &C = patches[op.coarse];
     const PatchT<T> &F = patches[op.fine];
@@ -128,6 +141,7 @@ __device__ __forceinline__ void iface_op(const PatchT<T> *patches, const IfaceOp
             }
             C.FxL[cid] = tl * scale;
         }
+        if (sizeof(T) == 8) C.FxDS[cid] = stage_flux(C.FxH, cid, params + param_base(C.run, step), step, C.FxL[cid]);
     } else {
         T t = 0;
         for (int q = 0; q < r; q++) t += F.FpH[step][pidx(op.fi + q, op.fj, F.pitch)];
@@ -146,6 +160,7 @@ __device__ __forceinline__ void iface_op(const PatchT<T> *patches, const IfaceOp
             }
             C.FpL[cid] = tl * scale;
         }
+        if (sizeof(T) == 8) C.FpDS[cid] = stage_flux(C.FpH, cid, params + param_base(C.run, step), step, C.FpL[cid]);
     }
 }
 

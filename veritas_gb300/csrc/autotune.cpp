@@ -4,7 +4,7 @@
 // coalesced axis) x tile_i (x) cells.  The best shape depends on the patch sizes of the
 // set (ragged edges, occupancy, register pressure of the precision's kernels), so the
 // engine measures it: for each candidate the tile list is rebuilt and the sub-steps that
-// leave the solution unchanged between steps (gamma, faces, fluxes, ds/f2, limiter R and
+// leave the solution unchanged between steps (gamma, faces, fluxes, f2, limiter R and
 // C — their outputs are recomputed before being read in the next step) are timed with CUDA
 // events on the engine's stream; the fastest shape is kept for the set and becomes the
 // default for new sets of the same precision.  The tile shape changes no arithmetic.
@@ -28,9 +28,9 @@ std::pair<int, int> Engine::autotune(const std::vector<Run *> &set, int reps) {
     fl.stream = stream;
     auto run_subs = [&]() {
         if (L.precision == kF32)
-            for (int sub : {kSubXFlux, kSubPFlux, kSubDsF2, kSubLimR, kSubLimC}) launch_fct32_substep(fl, sub);
+            for (int sub : {kSubXFlux, kSubPFlux, kSubDS, kSubF2, kSubLimR, kSubLimC}) launch_fct32_substep(fl, sub);
         else
-            for (int sub : {kSubGamma, kSubFaces, kSubFlux, kSubDsF2, kSubLimR, kSubLimC}) launch_fct64_substep(fl, sub);
+            for (int sub : {kSubGamma, kSubFaces, kSubFlux, kSubF2, kSubLimR, kSubLimC}) launch_fct64_substep(fl, sub);
     };
     double best_ms = 1e300;
     int best[2] = {L.tile_j, L.tile_i};
@@ -57,7 +57,7 @@ std::pair<int, int> Engine::autotune(const std::vector<Run *> &set, int reps) {
         timer_begin();
         for (int r = 0; r < reps; r++) run_subs();
         const double ms = timer_end() / reps;
-        kernel_launches += (L.precision == kF32 ? 5 : 6) * (reps + 1);
+        kernel_launches += 6 * (reps + 1);
         if (ms < best_ms) {
             best_ms = ms;
             best[0] = sh[0];

@@ -503,6 +503,8 @@ Engine::Engine(int dev) : device(dev) {
     VX_CUDA(cudaSetDevice(dev));
     VX_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
     VX_CUDA(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
+    VX_CUDA(cudaStreamCreateWithFlags(&side2, cudaStreamNonBlocking));
+    VX_CUDA(cudaEventCreateWithFlags(&ev_f2, cudaEventDisableTiming));
     VX_CUDA(cudaEventCreateWithFlags(&ev_pinned_, cudaEventDisableTiming));
     VX_CUDA(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
     VX_CUDA(cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming));
@@ -526,6 +528,8 @@ Engine::~Engine() {
     if (ev_mx) cudaEventDestroy(ev_mx);
     if (ev_pinned_) cudaEventDestroy(ev_pinned_);
     if (side) cudaStreamDestroy(side);
+    if (ev_f2) cudaEventDestroy(ev_f2);
+    if (side2) cudaStreamDestroy(side2);
     if (stream) cudaStreamDestroy(stream);
 }
 
@@ -637,7 +641,7 @@ std::vector<double> Engine::profile_kernels(Run &run, int reps) {
     // stage-0 parameters with dt = 0 keep every kernel well defined
     // FP32 sets run the fused face + flux kernels: "faces" and "flux" time the x and p
     // ones, "gamma" (folded into them) reads 0
-    for (int sub : {kSubGamma, kSubFaces, kSubFlux, kSubDsF2, kSubLimR, kSubLimC, kSubUpdate}) {
+    for (int sub : {kSubGamma, kSubFaces, kSubFlux, kSubF2, kSubLimR, kSubLimC, kSubUpdate}) {
         if (L.precision == kF32 && sub == kSubGamma) {
             out.push_back(0.0);
             continue;
@@ -645,7 +649,10 @@ std::vector<double> Engine::profile_kernels(Run &run, int reps) {
         const int run = L.precision == kF32 && sub == kSubFaces ? kSubXFlux
                         : L.precision == kF32 && sub == kSubFlux ? kSubPFlux
                                                                   : sub;
-        time_it([&] { fct_sub(L, fl, run); });
+        time_it([&] {
+            if (L.precision == kF32 && sub == kSubF2) fct_sub(L, fl, kSubDS);  // "ds_f2": both
+            fct_sub(L, fl, run);
+        });
     }
     MomLaunch ml{};
     ml.patches = L.dpatch.p;
@@ -716,7 +723,8 @@ std::vector<double> Engine::profile_kernels(Run &run, int reps) {
     });
     time_it([&] {
         for (size_t b = 0; b + 1 < L.iface_ptr.size(); b++)
-            launch_iface(L.dpatch.p, L.diface.as<IfaceOp>() + L.iface_ptr[b], L.iface_ptr[b + 1] - L.iface_ptr[b], 0, L.precision, stream);
+            launch_iface(L.dpatch.p, L.diface.as<IfaceOp>() + L.iface_ptr[b], L.iface_ptr[b + 1] - L.iface_ptr[b], 0,
+                         L.dparams.as<double>(), L.precision, stream);
     });
     time_it([&] {
         for (size_t b = 0; b + 1 < L.csync_ptr.size(); b++)
@@ -1370,6 +1378,13 @@ void Engine::record_step(LaunchSet &L) {
             record_pipe_stage(L, K, s, launches);
             continue;
         }
+        fl.step = s;
+        if (s > 0) {  // the low-order solution and its ghost cells, beside the stage's field work
+            VX_CUDA(cudaEventRecord(ev_fork, stream));
+            VX_CUDA(cudaStreamWaitEvent(side2, ev_fork, 0));
+            record_f2(L, fl, side2, launches);
+            VX_CUDA(cudaEventRecord(ev_f2, side2));
+        }
         // FP32 copies of the fields: E_x's comes with each solve (k_efield), the per-cell
         // A^2 the moments read with each Maxwell stage for the next one (the step's first
         // stage makes its own), a^2's with the moments at every stage (the Maxwell stage
@@ -1408,8 +1423,8 @@ void Engine::record_step(LaunchSet &L) {
             fct_sub(L, fl, kSubPFlux);
             launches += 2;
         } else if (L.poisson == kPoissonLU) {
-            // x faces and fluxes, and the E_x-independent half of the p faces, beside the
-            // exact Poisson solve; then the p-face velocities (E_x) and the p fluxes
+            // x faces and fluxes, and the E_x-independent part of the p faces, beside the
+            // exact Poisson solve; then the p fluxes
             fl.part = 1;
             fct_sub(L, fl, kSubFaces);
             fct_sub(L, fl, kSubFlux);
@@ -1417,11 +1432,9 @@ void Engine::record_step(LaunchSet &L) {
             fct_sub(L, fl, kSubFaces);
             VX_CUDA(cudaStreamWaitEvent(stream, ev_join, 0));
             fl.part = 8;
-            fct_sub(L, fl, kSubFaces);
-            fl.part = 2;
             fct_sub(L, fl, kSubFlux);
             fl.part = 0;
-            launches += 5;
+            launches += 4;
         } else {  // the scan solve is short: the p faces in one pass after it
             fl.part = 1;
             fct_sub(L, fl, kSubFaces);
@@ -1433,29 +1446,56 @@ void Engine::record_step(LaunchSet &L) {
             fl.part = 0;
             launches += 4;
         }
-        for (size_t b = 0; b + 1 < L.iface_ptr.size(); b++, launches++)
-            launch_iface(L.dpatch.p, L.diface.as<IfaceOp>() + L.iface_ptr[b], L.iface_ptr[b + 1] - L.iface_ptr[b], s, L.precision, stream);
-        fct_sub(L, fl, kSubDsF2);
-        launches += 1;
-        for (size_t b = 0; b + 1 < L.ghost_ptr.size(); b++, launches++)
-            launch_ghost(L.dpatch.p, L.dghost.as<GhostOp>() + L.ghost_ptr[b], L.ghost_ptr[b + 1] - L.ghost_ptr[b], 2, L.precision, stream);
-        fct_sub(L, fl, kSubLimR);
-        fct_sub(L, fl, kSubLimC);
-        launches += 2;
-        for (size_t b = 0; b + 1 < L.csync_ptr.size(); b++, launches++)
-            launch_csync(L.dpatch.p, L.dcsync.as<CSyncOp>() + L.csync_ptr[b], L.csync_ptr[b + 1] - L.csync_ptr[b], L.precision, stream);
-        fct_sub(L, fl, kSubUpdate);
-        launches += 1;
-        for (size_t b = 0; b + 1 < L.ghost_ptr.size(); b++, launches++)
-            launch_ghost(L.dpatch.p, L.dghost.as<GhostOp>() + L.ghost_ptr[b], L.ghost_ptr[b + 1] - L.ghost_ptr[b], 1, L.precision, stream);
-        if (s == 5) {
-            fct_sub(L, fl, kSubCopy10);
-            launches += 1;
-        }
+        record_fct_tail(L, fl, s, side2, launches);
         VX_CUDA(cudaStreamWaitEvent(stream, ev_mx, 0));
     }
     L.launches_per_step = launches;
     if (pipe) pipe_pending_ = true;
+}
+
+// The low-order solution of stage fl.step and the ghost cells of f2 (Mesh::PushData(2)), on
+// `st`.  Both need only f0 and the step's stage-0 fluxes; the previous stage must be over
+// (its update reads f2).
+void Engine::record_f2(LaunchSet &L, const FctLaunch &fl, cudaStream_t st, int &launches) {
+    FctLaunch f = fl;
+    f.stream = st;
+    fct_sub(L, f, kSubF2);
+    launches += 1;
+    for (size_t b = 0; b + 1 < L.ghost_ptr.size(); b++, launches++)
+        launch_ghost(L.dpatch.p, L.dghost.as<GhostOp>() + L.ghost_ptr[b], L.ghost_ptr[b + 1] - L.ghost_ptr[b], 2, L.precision, st);
+}
+
+void Engine::record_iface(LaunchSet &L, int s, int &launches) {
+    for (size_t b = 0; b + 1 < L.iface_ptr.size(); b++, launches++)
+        launch_iface(L.dpatch.p, L.diface.as<IfaceOp>() + L.iface_ptr[b], L.iface_ptr[b + 1] - L.iface_ptr[b], s,
+                     L.dparams.as<double>(), L.precision, stream);
+}
+
+// The rest of stage s after its fluxes, on the main stream: interface faces, (stage 0: the
+// low-order solution, which later stages have beside their field work — joined here through
+// ev_f2 when it ran on side2; the pipelined form joins its side stream before the p fluxes),
+// limiter, update, ghost cells of f1.
+void Engine::record_fct_tail(LaunchSet &L, const FctLaunch &fl, int s, cudaStream_t f2_stream, int &launches) {
+    record_iface(L, s, launches);
+    if (L.precision == kF32) {
+        fct_sub(L, fl, kSubDS);
+        launches += 1;
+    }
+    if (s == 0) record_f2(L, fl, stream, launches);
+    else if (f2_stream == side2) VX_CUDA(cudaStreamWaitEvent(stream, ev_f2, 0));
+    fct_sub(L, fl, kSubLimR);
+    fct_sub(L, fl, kSubLimC);
+    launches += 2;
+    for (size_t b = 0; b + 1 < L.csync_ptr.size(); b++, launches++)
+        launch_csync(L.dpatch.p, L.dcsync.as<CSyncOp>() + L.csync_ptr[b], L.csync_ptr[b + 1] - L.csync_ptr[b], L.precision, stream);
+    fct_sub(L, fl, kSubUpdate);
+    launches += 1;
+    for (size_t b = 0; b + 1 < L.ghost_ptr.size(); b++, launches++)
+        launch_ghost(L.dpatch.p, L.dghost.as<GhostOp>() + L.ghost_ptr[b], L.ghost_ptr[b + 1] - L.ghost_ptr[b], 1, L.precision, stream);
+    if (s == 5) {
+        fct_sub(L, fl, kSubCopy10);
+        launches += 1;
+    }
 }
 
 // One RK stage of an FP64 exact-solve set in the pipelined form.  Main stream: the
@@ -1515,6 +1555,7 @@ void Engine::record_pipe_stage(LaunchSet &L, StageLaunches &K, int s, int &launc
     fct_sub(L, fl, kSubFlux);
     fl.part = 4;
     fct_sub(L, fl, kSubFaces);
+    if (s > 0) record_f2(L, fl, side, launches);
     VX_CUDA(cudaEventRecord(ev_gamma, side));
     VX_CUDA(cudaStreamWaitEvent(side, ev_join, 0));
     mx.step = s;
@@ -1525,30 +1566,10 @@ void Engine::record_pipe_stage(LaunchSet &L, StageLaunches &K, int s, int &launc
     fl.stream = stream;
     VX_CUDA(cudaStreamWaitEvent(stream, ev_gamma, 0));
     fl.part = 8;
-    fct_sub(L, fl, kSubFaces);
-    fl.part = 2;
     fct_sub(L, fl, kSubFlux);
     fl.part = 0;
-    launches += 2;
-    for (size_t b = 0; b + 1 < L.iface_ptr.size(); b++, launches++)
-        launch_iface(L.dpatch.p, L.diface.as<IfaceOp>() + L.iface_ptr[b], L.iface_ptr[b + 1] - L.iface_ptr[b], s, L.precision, stream);
-    fct_sub(L, fl, kSubDsF2);
     launches += 1;
-    for (size_t b = 0; b + 1 < L.ghost_ptr.size(); b++, launches++)
-        launch_ghost(L.dpatch.p, L.dghost.as<GhostOp>() + L.ghost_ptr[b], L.ghost_ptr[b + 1] - L.ghost_ptr[b], 2, L.precision, stream);
-    fct_sub(L, fl, kSubLimR);
-    fct_sub(L, fl, kSubLimC);
-    launches += 2;
-    for (size_t b = 0; b + 1 < L.csync_ptr.size(); b++, launches++)
-        launch_csync(L.dpatch.p, L.dcsync.as<CSyncOp>() + L.csync_ptr[b], L.csync_ptr[b + 1] - L.csync_ptr[b], L.precision, stream);
-    fct_sub(L, fl, kSubUpdate);
-    launches += 1;
-    for (size_t b = 0; b + 1 < L.ghost_ptr.size(); b++, launches++)
-        launch_ghost(L.dpatch.p, L.dghost.as<GhostOp>() + L.ghost_ptr[b], L.ghost_ptr[b + 1] - L.ghost_ptr[b], 1, L.precision, stream);
-    if (s == 5) {
-        fct_sub(L, fl, kSubCopy10);
-        launches += 1;
-    }
+    record_fct_tail(L, fl, s, side, launches);
     VX_CUDA(cudaStreamWaitEvent(stream, ev_mx, 0));
 }
 
@@ -1767,10 +1788,12 @@ void Engine::run_phases(Run &run, int s, double dt, unsigned phases) {
             fct_sub(L, fl, kSubFlux);
             launches += 3;
         }
-        for (size_t b = 0; b + 1 < L.iface_ptr.size(); b++, launches++)
-            launch_iface(L.dpatch.p, L.diface.as<IfaceOp>() + L.iface_ptr[b], L.iface_ptr[b + 1] - L.iface_ptr[b], s,
-                         L.precision, stream);
-        fct_sub(L, fl, kSubDsF2);
+        record_iface(L, s, launches);
+        if (L.precision == kF32) {
+            fct_sub(L, fl, kSubDS);
+            launches += 1;
+        }
+        fct_sub(L, fl, kSubF2);
         launches += 1;
     }
     if (phases & kPhSub1) {  // PushData(2), FCTTimeStep(.., 1), PushBoundaryC

@@ -322,7 +322,9 @@ public:
     int device;
     cudaStream_t stream = nullptr;
     cudaStream_t side = nullptr;       // Poisson solve beside the E-independent x-direction work
+    cudaStream_t side2 = nullptr;      // the low-order solution beside both
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+    cudaEvent_t ev_f2 = nullptr;
     cudaEvent_t ev_gamma = nullptr, ev_mx = nullptr;  // Maxwell stage beside the FCT chain
     std::vector<Run *> runs;
     bool use_graphs = true;
@@ -416,6 +418,9 @@ private:
     int prio_hi_ = 0;             // greatest stream priority of the device
     int num_sms_ = 1;
     PipeLaunch pipe_launch(LaunchSet &L, const StageLaunches &K);
+    void record_f2(LaunchSet &L, const FctLaunch &fl, cudaStream_t st, int &launches);
+    void record_iface(LaunchSet &L, int s, int &launches);
+    void record_fct_tail(LaunchSet &L, const FctLaunch &fl, int s, cudaStream_t f2_stream, int &launches);
     void record_pipe_stage(LaunchSet &L, StageLaunches &K, int s, int &launches);
     cudaEvent_t ev0_ = nullptr, ev1_ = nullptr;
     DevBuf flush_;

@@ -8,9 +8,13 @@
 namespace vx {
 
 // Streaming sub-steps: one block of (32, tile_i) threads per tile.
-__global__ void k32_ds_f2(const P32 *patches, const TileRef *tiles, const float *params, int s) {
+__global__ void k32_ds(const P32 *patches, const TileRef *tiles, const float *params, int s) {
     VX_PDL_WAIT();
-    ds_f2_32(patches, tiles[blockIdx.x], (int)threadIdx.x, (int)threadIdx.y, params, s);
+    ds_32(patches, tiles[blockIdx.x], (int)threadIdx.x, (int)threadIdx.y, params, s);
+}
+__global__ void k32_f2(const P32 *patches, const TileRef *tiles, const float *params, int s) {
+    VX_PDL_WAIT();
+    f2_32(patches, tiles[blockIdx.x], (int)threadIdx.x, (int)threadIdx.y, params, s);
 }
 __global__ void k32_limR(const P32 *patches, const TileRef *tiles) {
     VX_PDL_WAIT();
@@ -51,8 +55,11 @@ void launch_fct32_substep(const FctLaunch &L, int sub) {
     const P32 *pp = (const P32 *)L.patches;
     if (L.ntiles == 0) return;
     switch (sub) {
-        case kSubDsF2:
-            vx_launch(k32_ds_f2, L.ntiles, blk, 0, L.stream, pp, L.tiles, L.params32, L.step);
+        case kSubF2:
+            vx_launch(k32_f2, L.ntiles, blk, 0, L.stream, pp, L.tiles, L.params32, L.step);
+            break;
+        case kSubDS:
+            vx_launch(k32_ds, L.ntiles, blk, 0, L.stream, pp, L.tiles, L.params32, L.step);
             break;
         case kSubLimR:
             vx_launch(k32_limR, L.ntiles, blk, 0, L.stream, pp, L.tiles);

@@ -104,10 +104,8 @@ __device__ __forceinline__ void st4(float *p, const V4 &x, int j, int lo, int hi
         if (j + e >= lo && j + e < hi) p[e] = x.v[e];
 }
 
-// RK flux combination and low-order solution (Rectangle.cpp:1396-1534): DS over the
-// padded block, f2 over the interior.
-__device__ __forceinline__ void ds_f2_32(const P32 *patches, const TileRef t, int tx, int row, const float *params,
-                                         int s) {
+// RK flux combination (Rectangle.cpp:1396-1517): DS over the padded block.
+__device__ __forceinline__ void ds_32(const P32 *patches, const TileRef t, int tx, int row, const float *params, int s) {
     VX_VTILE32
     const float *a = params + param_base(P.run, s);
     const float asum = a[6];
@@ -128,28 +126,41 @@ __device__ __forceinline__ void ds_f2_32(const P32 *patches, const TileRef t, in
         }
     }
     const V4 lx = ld4(P.FxL + id), lp = ld4(P.FpL + id);
-    V4 dx, dp, lsx, lsp;
+    V4 dx, dp;
 #pragma unroll
     for (int e = 0; e < 4; e++) {
-        lsx.v[e] = asum * lx.v[e];
-        lsp.v[e] = asum * lp.v[e];
-        dx.v[e] = hx.v[e] - lsx.v[e];
-        dp.v[e] = hp.v[e] - lsp.v[e];
+        dx.v[e] = hx.v[e] - __fmul_rn(asum, lx.v[e]);
+        dp.v[e] = hp.v[e] - __fmul_rn(asum, lp.v[e]);
     }
     st4(P.FxDS + id, dx, j, -2, P.np + 2);
     st4(P.FpDS + id, dp, j, -2, P.np + 2);
+}
+
+// Low-order solution (Rectangle.cpp:1518-1534) on the interior.  It needs only the step's
+// stage-0 fluxes: after stage 0 it and the ghost cells it feeds are formed beside the
+// stage's field work, off the chain from the solve to the update.
+__device__ __forceinline__ void f2_32(const P32 *patches, const TileRef t, int tx, int row, const float *params, int s) {
+    VX_VTILE32
     if (i < 0 || i >= P.nx || j + 3 < 0 || j >= P.np) return;
+    const float asum = params[param_base(P.run, s) + 6];
+    const V4 lx = ld4(P.FxL + id), lp = ld4(P.FpL + id);
     const V4 f0 = ld4(P.f0 + id), lxn = ld4(P.FxL + id + pit);
     const float lp4 = (j + 3 < P.np) ? P.FpL[id + 4] : 0.0f;  // j + 4 <= np
-    V4 f2;
+    // the cell's own low-order fluxes are shared with its neighbours in the row: rounded once
+    V4 lsx, lsp, f2;
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+        lsx.v[e] = __fmul_rn(asum, lx.v[e]);
+        lsp.v[e] = __fmul_rn(asum, lp.v[e]);
+    }
 #pragma unroll
     for (int e = 0; e < 4; e++) {
         const int je = j + e;
         float v = f0.v[e];
         if (active32(P, i, je)) v += lsx.v[e];
         if (active32(P, i, je)) v += lsp.v[e];
-        if (active32(P, i, je + 1)) v -= asum * (e < 3 ? lp.v[e + 1] : lp4);
-        if (active32(P, i + 1, je)) v -= asum * lxn.v[e];
+        if (active32(P, i, je + 1)) v = e < 3 ? v - lsp.v[e + 1] : __fmaf_rn(-asum, lp4, v);
+        if (active32(P, i + 1, je)) v = __fmaf_rn(-asum, lxn.v[e], v);
         f2.v[e] = v;
     }
     st4(P.f2 + id, f2, j, 0, P.np);

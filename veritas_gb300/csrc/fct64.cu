@@ -227,80 +227,139 @@ __global__ void k64_faces(const P64 *patches, const TileRef *tiles, const RunFie
         P.ep[id] = am;
         P.fp[id] = weno_face(f[pidx(i, j - 2, pit)], f[pidx(i, j - 1, pit)], f[id], f[pidx(i, j + 1, pit)], gt0(am));
     }
-    // The p faces in two halves, so that the E_x-independent one runs beside the Poisson
-    // solve: part 4 forms both upwind candidates (fp and, as scratch, Rp, which the
-    // limiter rewrites later in the stage); part 8, once E_x is known, the velocity and the
-    // choice.
+    // The part of the p faces that does not need E_x, formed beside the Poisson solve: both
+    // upwind candidates (fp and, as scratch, Rp) and the velocity's second term (Rm; the
+    // limiter rewrites both later in the stage).  k64_pflux_pick goes on from these.
     if ((part & 4) && i >= -1 && i <= P.nx && j >= 0 && j <= P.np) {
         double vr, vl;
         weno_values<true>(f[pidx(i, j - 2, pit)], f[pidx(i, j - 1, pit)], f[id], f[pidx(i, j + 1, pit)], true, vr, vl);
         P.fp[id] = vr;
         P.Rp[id] = vl;
-    }
-    if ((part & 8) && i >= -1 && i <= P.nx && j >= 0 && j <= P.np) {
-        const RunFields &F = fields[P.run];
-        double Em = P.q * patch_efield(P, F, i);
-        double am = Em - P.kp * (g[pidx(i + 1, j, pit)] - g[id]);
-        P.ep[id] = am;
-        if (!gt0(am)) P.fp[id] = P.Rp[id];
+        P.Rm[id] = P.kp * (g[pidx(i + 1, j, pit)] - g[id]);
     }
 }
 
-// High-order fluxes for stage `step` and, on stage 0, the donor-cell low-order fluxes
-// (Rectangle.cpp:1313-1394).  Coarse faces on a coarse/fine interface are skipped here
-// and written by the interface kernel.
-__global__ void k64_flux(const P64 *patches, const TileRef *tiles, int step, int use_f0, int part) {
+// The stage's antidiffusive flux of a face from its high-order flux `v` of stage s, those of
+// the earlier stages and its low-order flux (Rectangle.cpp:1396-1517).  RK coefficients
+// arrive pre-multiplied by dt.  Formed where the flux is: v need not be read again.
+__device__ __forceinline__ double stage_flux64(double *const *H, int id, const double *a, int s, double v,
+                                               double low) {
+    double h = a[0] * (s == 0 ? v : H[0][id]);
+    for (int k = 1; k <= s; k++) {
+        if (s == 5 && k == 1) continue;  // b_1 = 0 (Rectangle.cpp:1494)
+        h = h + a[k] * (k == s ? v : H[k][id]);
+    }
+    return h - a[6] * low;
+}
+
+// High-order fluxes for stage `step`, on stage 0 the donor-cell low-order fluxes
+// (Rectangle.cpp:1313-1394), and the antidiffusive stage fluxes.  Coarse faces on a
+// coarse/fine interface are skipped here and written by the interface kernel.
+__global__ void k64_flux(const P64 *patches, const TileRef *tiles, const double *params, int step, int use_f0,
+                         int part) {
     VX_PDL_WAIT();
     VX_TILE_PROLOGUE
     const double *f = use_f0 ? P.f0 : P.f1;
+    const double *a = params + param_base(P.run, step);
     const double w3 = 1 / 48.0;
     if ((part & 1) && i >= 0 && i <= P.nx && j >= -1 && j <= P.np && !(P.ifx && P.ifx[id])) {
         double am = P.ex[id], ap1 = P.ex[id + 1], am1 = P.ex[id - 1];
         double fm = P.fx[id], fp1 = P.fx[id + 1], fm1 = P.fx[id - 1];
-        P.FxH[step][id] = P.dx_inv * (fm * am + w3 * (fp1 - fm1) * (ap1 - am1));
-        if (step == 0) P.FxL[id] = P.dx_inv * ((gt0(am) ? f[id - pit] : f[id]) * am);
+        const double v = P.dx_inv * (fm * am + w3 * (fp1 - fm1) * (ap1 - am1));
+        P.FxH[step][id] = v;
+        double low;
+        if (step == 0) {
+            low = P.dx_inv * ((gt0(am) ? f[id - pit] : f[id]) * am);
+            P.FxL[id] = low;
+        } else {
+            low = P.FxL[id];
+        }
+        P.FxDS[id] = stage_flux64(P.FxH, id, a, step, v, low);
     }
     if ((part & 2) && i >= -1 && i <= P.nx && j >= 0 && j <= P.np && !(P.ifp && P.ifp[id])) {
         double am = P.ep[id], ap1 = P.ep[id + pit], am1 = P.ep[id - pit];
         double fm = P.fp[id], fp1 = P.fp[id + pit], fm1 = P.fp[id - pit];
-        P.FpH[step][id] = P.dp_inv * (fm * am + w3 * (fp1 - fm1) * (ap1 - am1));
-        if (step == 0) P.FpL[id] = P.dp_inv * ((gt0(am) ? f[id - 1] : f[id]) * am);
+        const double v = P.dp_inv * (fm * am + w3 * (fp1 - fm1) * (ap1 - am1));
+        P.FpH[step][id] = v;
+        double low;
+        if (step == 0) {
+            low = P.dp_inv * ((gt0(am) ? f[id - 1] : f[id]) * am);
+            P.FpL[id] = low;
+        } else {
+            low = P.FpL[id];
+        }
+        P.FpDS[id] = stage_flux64(P.FpH, id, a, step, v, low);
     }
+}
+
+// The p fluxes once E_x is known, from what k64_faces (part 4) left: velocity E - Rm, face
+// value fp or Rp by its sign, for the face's row and the rows on either side.  q E_x is a
+// row's value: formed once per block and row.  One pass in place of a face pass and a flux
+// pass, and nothing of it waits for the solve but the velocity's difference: it is on the
+// step's critical path (the solve is not).  The velocity itself is kept on stage 0, where
+// the interface kernel reads it.
+__global__ void k64_pflux_pick(const P64 *patches, const TileRef *tiles, const RunFields *fields, const double *params,
+                               int step, int use_f0) {
+    VX_PDL_WAIT();
+    __shared__ double s_e[66];  // q E_x of the tile's rows i0 - 1 .. i0 + rows
+    const TileRef t = tiles[blockIdx.x];
+    const P64 &P = patches[t.patch];
+    {
+        const int r = (int)(threadIdx.y * blockDim.x + threadIdx.x), i = t.i0 - 1 + r;
+        if (r < (int)blockDim.y + 2)
+            s_e[r] = (i >= -1 && i <= P.nx) ? P.q * patch_efield(P, fields[P.run], i) : 0.0;
+    }
+    __syncthreads();
+    const int i = t.i0 + (int)threadIdx.y, j = t.j0 + (int)threadIdx.x;
+    if (i < -1 || i > P.nx || j < 0 || j > P.np) return;
+    const int pit = P.pitch, id = pidx(i, j, pit);
+    const double *f = use_f0 ? P.f0 : P.f1;
+    const double *a = params + param_base(P.run, step);
+    const double w3 = 1 / 48.0;
+    double am[3], fv[3];  // rows i-1, i, i+1; zero past the face range, as the planes are there
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+        const int k = i - 1 + d, kd = id + (d - 1) * pit;
+        am[d] = fv[d] = 0.0;
+        if (k >= -1 && k <= P.nx) {
+            am[d] = s_e[(int)threadIdx.y + d] - P.Rm[kd];
+            fv[d] = gt0(am[d]) ? P.fp[kd] : P.Rp[kd];
+        }
+    }
+    if (step == 0) P.ep[id] = am[1];
+    if (P.ifp && P.ifp[id]) return;
+    const double v = P.dp_inv * (fv[1] * am[1] + w3 * (fv[2] - fv[0]) * (am[2] - am[0]));
+    P.FpH[step][id] = v;
+    double low;
+    if (step == 0) {
+        low = P.dp_inv * ((gt0(am[1]) ? f[id - 1] : f[id]) * am[1]);
+        P.FpL[id] = low;
+    } else {
+        low = P.FpL[id];
+    }
+    P.FpDS[id] = stage_flux64(P.FpH, id, a, step, v, low);
 }
 
 __device__ __forceinline__ bool active_face(const P64 &P, int i, int j) {
     return i >= P.xm && i < P.xp && j >= P.pm && j < P.pp;
 }
 
-// Stage flux combination (Rectangle.cpp:1396-1517) over the whole padded block, and the
-// low-order solution f2 = f0 + div(LS) on the interior in the reference's accumulation
-// order (Rectangle.cpp:1518-1534).  RK coefficients arrive pre-multiplied by dt.
-__global__ void k64_ds_f2(const P64 *patches, const TileRef *tiles, const double *params, int s) {
+// The low-order solution f2 = f0 + div(LS) on the interior in the reference's accumulation
+// order (Rectangle.cpp:1518-1534).  It needs only the step's stage-0 fluxes, so after
+// stage 0 it is formed beside the stage's field work.
+__global__ void k64_f2(const P64 *patches, const TileRef *tiles, const double *params, int s) {
     VX_PDL_WAIT();
     VX_TILE_PROLOGUE
-    if (i < -2 || j < -2) return;
-    const double *a = params + param_base(P.run, s);
-    const double asum = a[6];
-    double hx, hp;
-    hx = a[0] * P.FxH[0][id];
-    hp = a[0] * P.FpH[0][id];
-    for (int k = 1; k <= s; k++) {
-        if (s == 5 && k == 1) continue;  // b_1 = 0 (Rectangle.cpp:1494)
-        hx = hx + a[k] * P.FxH[k][id];
-        hp = hp + a[k] * P.FpH[k][id];
-    }
+    if (i < 0 || i >= P.nx || j < 0 || j >= P.np) return;
+    const double asum = params[param_base(P.run, s) + 6];
     double lsx = asum * P.FxL[id];
     double lsp = asum * P.FpL[id];
-    P.FxDS[id] = hx - lsx;
-    P.FpDS[id] = hp - lsp;
-    if (i >= 0 && i < P.nx && j >= 0 && j < P.np) {
-        double v = P.f0[id];
-        if (active_face(P, i, j)) v += lsx;
-        if (active_face(P, i, j)) v += lsp;
-        if (active_face(P, i, j + 1)) v -= asum * P.FpL[id + 1];
-        if (active_face(P, i + 1, j)) v -= asum * P.FxL[id + pit];
-        P.f2[id] = v;
-    }
+    double v = P.f0[id];
+    if (active_face(P, i, j)) v += lsx;
+    if (active_face(P, i, j)) v += lsp;
+    if (active_face(P, i, j + 1)) v -= asum * P.FpL[id + 1];
+    if (active_face(P, i + 1, j)) v -= asum * P.FxL[id + pit];
+    P.f2[id] = v;
 }
 
 // Zalesak R+/R- on i in [-1,nx], j in [-1,np] (Rectangle.cpp:1536-1579).
@@ -418,10 +477,14 @@ void VX_FCT64_LAUNCH(const FctLaunch &L, int sub) {
             vx_launch(k64_faces, L.ntiles, blk, 0, L.stream, pp, L.tiles, L.fields, L.use_f0, L.part ? L.part : 3);
             break;
         case kSubFlux:
-            vx_launch(k64_flux, L.ntiles, blk, 0, L.stream, pp, L.tiles, L.step, L.use_f0, L.part ? L.part : 3);
+            if (L.part == 8)
+                vx_launch(k64_pflux_pick, L.ntiles, blk, 0, L.stream, pp, L.tiles, L.fields, L.params, L.step, L.use_f0);
+            else
+                vx_launch(k64_flux, L.ntiles, blk, 0, L.stream, pp, L.tiles, L.params, L.step, L.use_f0,
+                          L.part ? L.part : 3);
             break;
-        case kSubDsF2:
-            vx_launch(k64_ds_f2, L.ntiles, blk, 0, L.stream, pp, L.tiles, L.params, L.step);
+        case kSubF2:
+            vx_launch(k64_f2, L.ntiles, blk, 0, L.stream, pp, L.tiles, L.params, L.step);
             break;
         case kSubLimR:
             vx_launch(k64_limR, L.ntiles, blk, 0, L.stream, pp, L.tiles);

@@ -202,11 +202,14 @@ __global__ void __launch_bounds__(kStageThreads, 5) k32_stage_fct(Stage32Launch 
     bar.sync();
     // coarse faces on coarse/fine interfaces, batch by batch
     for (int b = 0; b < L.niface_b; b++) {
-        for_ops(L.iface_ptr, b, [&](int k) { iface_op(patches, L.iface, k, s); });
+        for_ops(L.iface_ptr, b, [&](int k) { iface_op(patches, L.iface, k, s, nullptr); });
         bar.sync();
     }
     // RK flux combination and low-order solution | Maxwell stage combination
-    for_tiles(F, [&](const TileRef &t, int tx, int row) { ds_f2_32(patches, t, tx, row, F.params32, s); });
+    for_tiles(F, [&](const TileRef &t, int tx, int row) {
+        ds_32(patches, t, tx, row, F.params32, s);
+        f2_32(patches, t, tx, row, F.params32, s);
+    });
     for_cells(mxn, [&](long long e) { mx_update_cell(X, (int)(e / X.maxnf), (int)(e % X.maxnf)); });
     bar.sync();
     // ghost cells of f2 (Mesh::PushData(2))
@@ -293,7 +296,7 @@ __global__ void k_ghost32(const PatchT<float> *patches, const GhostOp *ops, int 
 __global__ void k_iface32(const PatchT<float> *patches, const IfaceOp *ops, int n, int step) {
     VX_PDL_WAIT();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < n) iface_op(patches, ops, k, step);
+    if (k < n) iface_op(patches, ops, k, step, nullptr);
 }
 __global__ void k_csync32(const PatchT<float> *patches, const CSyncOp *ops, int n) {
     VX_PDL_WAIT();

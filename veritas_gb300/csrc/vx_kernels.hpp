@@ -61,14 +61,16 @@ enum FctSub : int {
     kSubGamma = 0,
     kSubFaces,
     kSubFlux,
-    kSubDsF2,
+    kSubF2,
     kSubLimR,
     kSubLimC,
     kSubUpdate,
     kSubCopy10,
     // FP32 form only: gamma + x faces + x fluxes, and p faces + p fluxes, each fused
+    // and the stage flux combination (the FP64 flux kernels form it)
     kSubXFlux,
     kSubPFlux,
+    kSubDS,
 };
 
 struct FctLaunch {
@@ -80,7 +82,9 @@ struct FctLaunch {
     const float *params32;    // the same blocks in FP32 (FP32 form)
     int step;
     int use_f0;
-    int part;  // faces / flux: 1 x faces only, 2 p faces only, 0 both
+    // faces, flux: 1 x faces only, 2 p faces only, 0 both; faces 4: both upwind candidates of the
+    // p faces and the E_x-free part of their velocity; flux 8: p fluxes from those
+    int part;
     int tile_j, tile_i;  // thread block = one tile of tile_j (p) x tile_i (x) cells
     // FP32 fused face + flux kernels: one warp per strip tile
     const TileRef *xtiles, *ptiles;
@@ -293,7 +297,7 @@ struct IfaceOp;
 struct CSyncOp;
 // `prec` selects the patch storage type (kF64 or kF32) of the descriptor array.
 void launch_ghost(const void *patches, const GhostOp *ops, int n, int slot, int prec, cudaStream_t s);
-void launch_iface(const void *patches, const IfaceOp *ops, int n, int step, int prec, cudaStream_t s);
+void launch_iface(const void *patches, const IfaceOp *ops, int n, int step, const double *params, int prec, cudaStream_t s);
 // Launch-set op tables gathered on the device: segment s copies count ops from src to
 // dst + dst_off and adds base to their patch ids (the run's first patch in the set).
 struct OpSegment {
