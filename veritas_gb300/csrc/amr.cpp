@@ -130,8 +130,7 @@ constexpr int kMaxBatches = 255;  // op batches per list (the fills and exchange
 // Assigns each op of an ordered list the smallest batch that keeps the list's read /
 // write orders (RAW, WAR, WAW) on the cells it touches, with the last write / read batch
 // of each cell kept in dense per-patch byte planes (batch + 1, 0 for none; allocated when
-// a patch is first touched): the restriction ops of large nested regions number in the
-// millions.
+// a patch is first touched): the cells of large nested regions number in the millions.
 struct PlaneScheduler {
     explicit PlaneScheduler(const std::vector<Rect *> &patches) : flat(patches), last_w(patches.size()), last_r(patches.size()) {}
     const std::vector<Rect *> &flat;
@@ -176,8 +175,8 @@ struct PlaneScheduler {
     // largest batch any of them needs, which keeps each cell's read / write orders (a
     // later batch than a cell's own minimum never runs before an op it must follow, and
     // the ops emitted after see the batch in the planes).  Bounds are checked once for
-    // the row; one batch entry per cell op.
-    void add_restrict_row(int dst, int di, int dj, int src, int si, int sj, int r, int len) {
+    // the row; returns its batch (rows are a list of their own).
+    int add_restrict_row(int dst, int di, int dj, int src, int si, int sj, int r, int len) {
         slot(src, si, sj);
         slot(src, si + r - 1, sj + r * len - 1);  // bounds of the row's blocks
         slot(dst, di, dj);
@@ -200,8 +199,8 @@ struct PlaneScheduler {
         }
         uint8_t *dwm = last_w[dst].data() + cw;
         for (int k = 0; k < len; k++) dwm[k] = (uint8_t)(b + 1);
-        batch.insert(batch.end(), (size_t)len, b);
         nbatches = std::max(nbatches, b + 1);
+        return b;
     }
 };
 
@@ -234,12 +233,14 @@ void Run::validate_ops() const {
     for (const GhostOp &op : ghost_ops) {
         need(in(op.dst, op.di, op.dj), "ghost target");
         if (op.kind == kGhostCopy) need(in(op.src, op.si, op.sj), "ghost source");
-        if (op.kind == kGhostRestrict)
-            need(in(op.src, op.si, op.sj) && in(op.src, op.si + r - 1, op.sj + r - 1), "restriction source");
         if (op.kind == kGhostInterp) {
             need(in(op.src, op.si - 2, op.sj - 2) && in(op.src, op.si + 2, op.sj + 2), "interpolation stencil");
             need(op.sub >= 0 && op.sub < r * r, "interpolation entry");
         }
+    }
+    for (const GhostOp &op : ghost_rows) {
+        need(op.sub >= 1 && in(op.dst, op.di, op.dj) && in(op.dst, op.di, op.dj + op.sub - 1), "restriction target");
+        need(in(op.src, op.si, op.sj) && in(op.src, op.si + r - 1, op.sj + r * op.sub - 1), "restriction source");
     }
     for (const IfaceOp &op : iface_ops) {
         need(in(op.coarse, op.ci, op.cj), "interface face");
@@ -310,15 +311,14 @@ void Run::build_amr() {
     lap("links");
     // ------------------------------------------------------------ ghost fills
     ghost_ops.clear();
+    ghost_rows.clear();
+    std::vector<int> row_batch;
     PlaneScheduler gs(flat);
     auto emit = [&](const GhostOp &op) {
         int reads[64][3], writes[1][3] = {{op.dst, op.di, op.dj}};  // r <= 8: at most 64 reads
         int nr = 0;
         if (op.kind == kGhostCopy) {
             reads[nr][0] = op.src, reads[nr][1] = op.si, reads[nr][2] = op.sj, nr++;
-        } else if (op.kind == kGhostRestrict) {
-            for (int a = 0; a < r; a++)
-                for (int b = 0; b < r; b++) reads[nr][0] = op.src, reads[nr][1] = op.si + a, reads[nr][2] = op.sj + b, nr++;
         } else if (op.kind == kGhostInterp) {
             for (int a = -2; a <= 2; a++)
                 for (int b = -2; b <= 2; b++) reads[nr][0] = op.src, reads[nr][1] = op.si + a, reads[nr][2] = op.sj + b, nr++;
@@ -409,9 +409,9 @@ void Run::build_amr() {
                     while (j1 < R.n_p && R.nested[R.ns(i, j1)] && R.finer[R.ns(i, j1)] == fid) j1++;
                     const Rect &F = *flat[fid];
                     const int si = (R.x_pos + i) * r - F.x_pos;
-                    gs.add_restrict_row(R.id, i, j, F.id, si, (R.p_pos + j) * r - F.p_pos, r, j1 - j);
-                    for (int k = j; k < j1; k++)
-                        ghost_ops.push_back({kGhostRestrict, R.id, i, k, F.id, si, (R.p_pos + k) * r - F.p_pos, 0});
+                    const int sj = (R.p_pos + j) * r - F.p_pos;
+                    row_batch.push_back(gs.add_restrict_row(R.id, i, j, F.id, si, sj, r, j1 - j));
+                    ghost_rows.push_back({kGhostRestrict, R.id, i, j, F.id, si, sj, j1 - j});
                     j = j1;
                 }
         }
@@ -502,6 +502,7 @@ void Run::build_amr() {
         for (int i = L - 1; i > 0; i--) type2(sp[i - 1]);
     }
     sort_by_batch(ghost_ops, gs.batch, gs.nbatches, ghost_b);
+    sort_by_batch(ghost_rows, row_batch, gs.nbatches, ghost_rb);
     lap("ghost ops");
 
     // ------------------------------------------------------------ interface fluxes
@@ -610,6 +611,7 @@ void Run::build_amr() {
     validate_ops();
     lap("validate");
     dghost_ops = upload(ghost_ops, eng->stream);
+    dghost_rows = upload(ghost_rows, eng->stream);
     diface_ops = upload(iface_ops, eng->stream);
     dcsync_ops = upload(csync_ops, eng->stream);
     lap("op upload");

@@ -30,6 +30,9 @@ struct GhostOp {
     int src, si, sj;
     int sub;
 };
+// Restrictions come as rows in a list of their own (`sub` consecutive cells (di, dj + k) from
+// the blocks at (si, sj + r k)): a nested region holds millions of them, and one record per
+// cell was most of the fill's traffic.
 
 enum CSyncKind : int { kCSame = 0, kCDiff = 1, kCUpdate = 2 };
 

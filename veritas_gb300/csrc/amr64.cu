@@ -10,10 +10,9 @@
 namespace vx {
 
 template <class T>
-__global__ void k_ghost(const PatchT<T> *patches, const GhostOp *ops, int n, int slot) {
+__global__ void k_ghost(const PatchT<T> *patches, const GhostOp *ops, int n, const GhostOp *rows, int nrows, int slot) {
     VX_PDL_WAIT();
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < n) ghost_op(patches, ops, k, slot);
+    ghost_work(patches, ops, n, rows, nrows, blockIdx.x * (long long)blockDim.x + threadIdx.x, slot);
 }
 template <class T>
 __global__ void k_iface(const PatchT<T> *patches, const IfaceOp *ops, int n, int step, const double *params) {
@@ -155,10 +154,15 @@ void copy_from_host(const void *src_dev, void *dst, size_t bytes, cudaStream_t s
     vx_launch_plain(k_copy_from_host, blocks, 256, 0, s, (const uint4 *)src_dev, (uint4 *)dst, n16);
 }
 
-void launch_ghost(const void *patches, const GhostOp *ops, int n, int slot, int prec, cudaStream_t s) {
-    if (n <= 0) return;
-    if (prec == kF32) launch_ghost32(patches, ops, n, slot, s);
-    else vx_launch(k_ghost<double>, (n + 127) / 128, 128, 0, s, (const PatchT<double> *)patches, ops, n, slot);
+void launch_ghost(const void *patches, const GhostOp *ops, int n, const GhostOp *rows, int nrows, int slot, int prec,
+                  cudaStream_t s) {
+    if (n <= 0 && nrows <= 0) return;
+    if (prec == kF32) {
+        launch_ghost32(patches, ops, n, rows, nrows, slot, s);
+        return;
+    }
+    const int blocks = ((n + 31) / 32 + nrows + 3) / 4;
+    vx_launch(k_ghost<double>, blocks, 128, 0, s, (const PatchT<double> *)patches, ops, n, rows, nrows, slot);
 }
 
 void launch_iface(const void *patches, const IfaceOp *ops, int n, int step, const double *params, int prec, cudaStream_t s) {

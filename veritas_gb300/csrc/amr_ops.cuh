@@ -76,23 +76,46 @@ __device__ __forceinline__ void ghost_op(const PatchT<T> *patches, const GhostOp
     if (op.kind == kGhostCopy) {
         const PatchT<T> &S = patches[op.src];
         v = slot_plane(S, slot)[pidx(op.si, op.sj, S.pitch)];
-    } else if (op.kind == kGhostRestrict) {  // Rectangle::GetValueFromFinerLevel (Rectangle.cpp:314-327)
-        const PatchT<T> &S = patches[op.src];
-        const T *f = slot_plane(S, slot);
-        const int r = D.r;
-        T t = 0;
-        for (int a = 0; a < r; a++)
-            for (int b = 0; b < r; b++) t += f[pidx(op.si + a, op.sj + b, S.pitch)];
-        // std::pow(r, 2.0) of the reference, an exact integer; for a power of two the
-        // product with its exact reciprocal is the same correctly rounded value
-        if ((r & (r - 1)) == 0) t *= (T)(1.0 / (double)(r * r));
-        else t /= (T)(r * r);
-        v = t;
     } else if (op.kind == kGhostInterp) {
         const PatchT<T> &S = patches[op.src];
         v = coarse_interp(S, slot_plane(S, slot), op.si, op.sj, op.sub);
     }
     slot_plane(D, slot)[pidx(op.di, op.dj, D.pitch)] = v;
+}
+
+// A row of restrictions (Rectangle::GetValueFromFinerLevel, Rectangle.cpp:314-327), by one
+// warp: neighbouring lanes take neighbouring cells.
+template <class T>
+__device__ __forceinline__ void restrict_row(const PatchT<T> *patches, const GhostOp *rows, int k, int lane, int slot) {
+    const GhostOp op = rows[k];
+    const PatchT<T> &D = patches[op.dst];
+    const PatchT<T> &S = patches[op.src];
+    const int r = D.r, pit = S.pitch;
+    const T *f = slot_plane(S, slot) + pidx(op.si, op.sj, pit);
+    T *d = slot_plane(D, slot) + pidx(op.di, op.dj, D.pitch);
+    // std::pow(r, 2.0) of the reference, an exact integer; for a power of two the
+    // product with its exact reciprocal is the same correctly rounded value
+    const bool pow2 = (r & (r - 1)) == 0;
+    const T inv = (T)(1.0f / (float)(r * r));
+    for (int c = lane; c < op.sub; c += 32) {
+        T t = 0;
+        for (int a = 0; a < r; a++)
+            for (int b = 0; b < r; b++) t += f[a * pit + c * r + b];
+        if (pow2) t *= inv;
+        else t /= (T)(r * r);
+        d[c] = t;
+    }
+}
+// Op batch as one launch: ops one per thread, then rows one per warp (thread index e).
+template <class T>
+__device__ __forceinline__ void ghost_work(const PatchT<T> *patches, const GhostOp *ops, int n, const GhostOp *rows,
+                                           int nrows, long long e, int slot) {
+    const long long pad = ((long long)n + 31) / 32 * 32;
+    if (e < pad) {
+        if (e < n) ghost_op(patches, ops, (int)e, slot);
+    } else if ((e - pad) / 32 < nrows) {
+        restrict_row(patches, rows, (int)((e - pad) / 32), (int)(e & 31), slot);
+    }
 }
 
 // Coarse faces on a coarse/fine interface: the mean of the finer patch's fluxes through

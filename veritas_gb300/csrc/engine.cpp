@@ -718,8 +718,8 @@ std::vector<double> Engine::profile_kernels(Run &run, int reps) {
     time_it([&] { launch_maxwell(mx); });
     // the AMR op batches of one stage (each entry: all batches of that kind)
     time_it([&] {
-        for (size_t b = 0; b + 1 < L.ghost_ptr.size(); b++)
-            launch_ghost(L.dpatch.p, L.dghost.as<GhostOp>() + L.ghost_ptr[b], L.ghost_ptr[b + 1] - L.ghost_ptr[b], 1, L.precision, stream);
+        int ghost_launches = 0;
+        record_ghosts(L, 1, stream, ghost_launches);
     });
     time_it([&] {
         for (size_t b = 0; b + 1 < L.iface_ptr.size(); b++)
@@ -1084,6 +1084,9 @@ void Engine::build_set(LaunchSet &L) {
         gather(GhostOp{}, [](Run &R) -> DevBuf & { return R.dghost_ops; },
                [](Run &R) -> const std::vector<int> & { return R.ghost_b.ptr; }, merge_ghost_ops, L.dghost,
                L.ghost_ptr);
+        gather(GhostOp{}, [](Run &R) -> DevBuf & { return R.dghost_rows; },
+               [](Run &R) -> const std::vector<int> & { return R.ghost_rb.ptr; }, merge_ghost_ops, L.dghost_rows,
+               L.ghost_rptr);
         gather(IfaceOp{}, [](Run &R) -> DevBuf & { return R.diface_ops; },
                [](Run &R) -> const std::vector<int> & { return R.iface_b.ptr; }, merge_iface_ops, L.diface,
                L.iface_ptr);
@@ -1094,6 +1097,7 @@ void Engine::build_set(LaunchSet &L) {
         for (const std::vector<int> *p : {&L.ghost_ptr, &L.iface_ptr, &L.csync_ptr})
             for (size_t b = 0; b + 1 < p->size(); b++) L.max_batch = std::max(L.max_batch, (*p)[b + 1] - (*p)[b]);
         pk.put(L.dghost_ptr, L.ghost_ptr);
+        pk.put(L.dghost_rptr, L.ghost_rptr);
         pk.put(L.diface_ptr, L.iface_ptr);
         pk.put(L.dcsync_ptr, L.csync_ptr);
     }
@@ -1453,6 +1457,14 @@ void Engine::record_step(LaunchSet &L) {
     if (pipe) pipe_pending_ = true;
 }
 
+// Mesh::PushData(slot) (Mesh.cpp:91-106) for every run of the set, batch by batch.
+void Engine::record_ghosts(LaunchSet &L, int slot, cudaStream_t st, int &launches) {
+    for (size_t b = 0; b + 1 < L.ghost_ptr.size(); b++, launches++)
+        launch_ghost(L.dpatch.p, L.dghost.as<GhostOp>() + L.ghost_ptr[b], L.ghost_ptr[b + 1] - L.ghost_ptr[b],
+                     L.dghost_rows.as<GhostOp>() + L.ghost_rptr[b], L.ghost_rptr[b + 1] - L.ghost_rptr[b], slot,
+                     L.precision, st);
+}
+
 // The low-order solution of stage fl.step and the ghost cells of f2 (Mesh::PushData(2)), on
 // `st`.  Both need only f0 and the step's stage-0 fluxes; the previous stage must be over
 // (its update reads f2).
@@ -1461,8 +1473,7 @@ void Engine::record_f2(LaunchSet &L, const FctLaunch &fl, cudaStream_t st, int &
     f.stream = st;
     fct_sub(L, f, kSubF2);
     launches += 1;
-    for (size_t b = 0; b + 1 < L.ghost_ptr.size(); b++, launches++)
-        launch_ghost(L.dpatch.p, L.dghost.as<GhostOp>() + L.ghost_ptr[b], L.ghost_ptr[b + 1] - L.ghost_ptr[b], 2, L.precision, st);
+    record_ghosts(L, 2, st, launches);
 }
 
 void Engine::record_iface(LaunchSet &L, int s, int &launches) {
@@ -1490,8 +1501,7 @@ void Engine::record_fct_tail(LaunchSet &L, const FctLaunch &fl, int s, cudaStrea
         launch_csync(L.dpatch.p, L.dcsync.as<CSyncOp>() + L.csync_ptr[b], L.csync_ptr[b + 1] - L.csync_ptr[b], L.precision, stream);
     fct_sub(L, fl, kSubUpdate);
     launches += 1;
-    for (size_t b = 0; b + 1 < L.ghost_ptr.size(); b++, launches++)
-        launch_ghost(L.dpatch.p, L.dghost.as<GhostOp>() + L.ghost_ptr[b], L.ghost_ptr[b + 1] - L.ghost_ptr[b], 1, L.precision, stream);
+    record_ghosts(L, 1, stream, launches);
     if (s == 5) {
         fct_sub(L, fl, kSubCopy10);
         launches += 1;
@@ -1599,6 +1609,8 @@ void Engine::record_step_persistent32(LaunchSet &L) {
     S.mx.asq32_out = 1;  // the next stage's x fluxes run beside its moments (see launch_stage32_pre)
     S.ghost = L.dghost.as<GhostOp>();
     S.ghost_ptr = L.dghost_ptr.as<int>();
+    S.ghost_rows = L.dghost_rows.as<GhostOp>();
+    S.ghost_rptr = L.dghost_rptr.as<int>();
     S.nghost_b = L.ghost_ptr.empty() ? 0 : (int)L.ghost_ptr.size() - 1;
     S.iface = L.diface.as<IfaceOp>();
     S.iface_ptr = L.diface_ptr.as<int>();
@@ -1797,9 +1809,7 @@ void Engine::run_phases(Run &run, int s, double dt, unsigned phases) {
         launches += 1;
     }
     if (phases & kPhSub1) {  // PushData(2), FCTTimeStep(.., 1), PushBoundaryC
-        for (size_t b = 0; b + 1 < L.ghost_ptr.size(); b++, launches++)
-            launch_ghost(L.dpatch.p, L.dghost.as<GhostOp>() + L.ghost_ptr[b], L.ghost_ptr[b + 1] - L.ghost_ptr[b], 2,
-                         L.precision, stream);
+        record_ghosts(L, 2, stream, launches);
         fct_sub(L, fl, kSubLimR);
         fct_sub(L, fl, kSubLimC);
         launches += 2;
@@ -1810,9 +1820,7 @@ void Engine::run_phases(Run &run, int s, double dt, unsigned phases) {
     if (phases & kPhSub2) {  // FCTTimeStep(.., 2), PushData(1)
         fct_sub(L, fl, kSubUpdate);
         launches += 1;
-        for (size_t b = 0; b + 1 < L.ghost_ptr.size(); b++, launches++)
-            launch_ghost(L.dpatch.p, L.dghost.as<GhostOp>() + L.ghost_ptr[b], L.ghost_ptr[b + 1] - L.ghost_ptr[b], 1,
-                         L.precision, stream);
+        record_ghosts(L, 1, stream, launches);
     }
     if ((phases & kPhSub3) && s == 5) {  // FCTTimeStep(.., 3): Mesh::Advance runs it at the last stage only
         fct_sub(L, fl, kSubCopy10);

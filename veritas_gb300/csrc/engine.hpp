@@ -209,13 +209,13 @@ public:
     void enforce_neutralization();
     // AMR: flat patch list (species -> depth -> patch), connectivity and op lists.
     std::vector<Rect *> flat;
-    std::vector<GhostOp> ghost_ops;
-    Batched ghost_b;
+    std::vector<GhostOp> ghost_ops, ghost_rows;  // ghost_rows: restriction rows
+    Batched ghost_b, ghost_rb;                   // (as many batches each)
     std::vector<CSyncOp> csync_ops;
     Batched csync_b;
     std::vector<IfaceOp> iface_ops;
     Batched iface_b;
-    DevBuf dghost_ops, dcsync_ops, diface_ops;  // the op lists on the device (set tables gather them)
+    DevBuf dghost_ops, dghost_rows, dcsync_ops, diface_ops;  // the op lists on the device (set tables gather them)
     DevBuf drelc;                   // sub-cell interpolation weights per depth
     DevBuf drefc;                   // coarse-to-fine interpolation weights (refinement ratio)
     std::vector<int> relc_off;      // offset of depth d's weights in drelc
@@ -266,7 +266,7 @@ struct LaunchSet {
     DevBuf dparams32;
     std::vector<double> w, fcoef;
     // AMR op tables of all runs, batch by batch (global patch ids)
-    DevBuf dghost, diface, dcsync;
+    DevBuf dghost, dghost_rows, diface, dcsync;
     int precision = kF64;
     int tile_j = 32, tile_i = 8;  // FCT tile (p x x) = thread block of the sub-step kernels
     DevBuf dxtiles, dptiles;      // FP32: strip tiles of the fused face + flux kernels
@@ -274,8 +274,8 @@ struct LaunchSet {
     int poisson = kPoissonLU;
     int fast64 = 0;  // FP64 sets: contracted FCT kernels
     DevBuf dpf;  // per-run PoissonFastDev (scan Poisson sets)
-    std::vector<int> ghost_ptr, iface_ptr, csync_ptr;
-    DevBuf dghost_ptr, diface_ptr, dcsync_ptr;  // the batch offsets on the device (persistent form)
+    std::vector<int> ghost_ptr, ghost_rptr, iface_ptr, csync_ptr;
+    DevBuf dghost_ptr, dghost_rptr, diface_ptr, dcsync_ptr;  // the batch offsets on the device (persistent form)
     int max_batch = 0;                          // largest op batch
     int launches_per_step = 0;                  // kernels of one recorded step
     // FP64 exact-solve sets of up to kPipeMaxRuns runs: tables of the pipelined moments +
@@ -290,7 +290,7 @@ struct LaunchSet {
     // gathers, their segment lists
     std::unique_ptr<TablePack> pending_pack;
     std::vector<std::function<void()>> pending_gathers;
-    DevBuf dsegs[3];
+    DevBuf dsegs[4];
     cudaGraphExec_t graph = nullptr;
     ~LaunchSet();
 };
@@ -418,6 +418,7 @@ private:
     int prio_hi_ = 0;             // greatest stream priority of the device
     int num_sms_ = 1;
     PipeLaunch pipe_launch(LaunchSet &L, const StageLaunches &K);
+    void record_ghosts(LaunchSet &L, int slot, cudaStream_t st, int &launches);
     void record_f2(LaunchSet &L, const FctLaunch &fl, cudaStream_t st, int &launches);
     void record_iface(LaunchSet &L, int s, int &launches);
     void record_fct_tail(LaunchSet &L, const FctLaunch &fl, int s, cudaStream_t f2_stream, int &launches);

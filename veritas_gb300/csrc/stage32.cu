@@ -184,6 +184,14 @@ __device__ __forceinline__ void for_ops(const int *ptr, int b, Body body) {
     for_cells(hi - lo, [&](long long e) { body(lo + (int)e); });
 }
 
+// Batch b of the ghost fills of `slot`: ops one per thread, restriction rows one per warp.
+__device__ __forceinline__ void for_ghosts(const Stage32Launch &L, int b, const P32 *patches, int slot) {
+    const int o = L.ghost_ptr[b], n = L.ghost_ptr[b + 1] - o;
+    const int w = L.ghost_rptr[b], nr = L.ghost_rptr[b + 1] - w;
+    for_cells(((long long)n + 31) / 32 * 32 + 32LL * nr,
+              [&](long long e) { ghost_work(patches, L.ghost + o, n, L.ghost_rows + w, nr, e, slot); });
+}
+
 // The FCT stage of every patch (fluxes .. ghost fills of f1) with the Maxwell stage beside it.
 // Five blocks per SM (48 registers, a few spilled on the limiter and interpolation paths):
 // the p-flux strips and streaming phases gain more from the extra warps than the spills
@@ -214,7 +222,7 @@ __global__ void __launch_bounds__(kStageThreads, 5) k32_stage_fct(Stage32Launch 
     bar.sync();
     // ghost cells of f2 (Mesh::PushData(2))
     for (int b = 0; b < L.nghost_b; b++) {
-        for_ops(L.ghost_ptr, b, [&](int k) { ghost_op(patches, L.ghost, k, 2); });
+        for_ghosts(L, b, patches, 2);
         bar.sync();
     }
     // limiter R | a^2 on the faces
@@ -232,7 +240,7 @@ __global__ void __launch_bounds__(kStageThreads, 5) k32_stage_fct(Stage32Launch 
     for_tiles(F, [&](const TileRef &t, int tx, int row) { update32(patches, t, tx, row); });
     bar.sync();
     for (int b = 0; b < L.nghost_b; b++) {
-        for_ops(L.ghost_ptr, b, [&](int k) { ghost_op(patches, L.ghost, k, 1); });
+        for_ghosts(L, b, patches, 1);
         if (b + 1 < L.nghost_b || s == 5) bar.sync();
     }
     if (s == 5)  // FCTTimeStep(.., 3) at the last stage: f0 = f1
@@ -288,10 +296,10 @@ void launch_stage32_fct(const Stage32Launch &L) {
 }
 
 // ---------------------------------------------------------------- per-sub-step kernels
-__global__ void k_ghost32(const PatchT<float> *patches, const GhostOp *ops, int n, int slot) {
+__global__ void k_ghost32(const PatchT<float> *patches, const GhostOp *ops, int n, const GhostOp *rows, int nrows,
+                          int slot) {
     VX_PDL_WAIT();
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < n) ghost_op(patches, ops, k, slot);
+    ghost_work(patches, ops, n, rows, nrows, blockIdx.x * (long long)blockDim.x + threadIdx.x, slot);
 }
 __global__ void k_iface32(const PatchT<float> *patches, const IfaceOp *ops, int n, int step) {
     VX_PDL_WAIT();
@@ -328,8 +336,10 @@ __global__ void k_mx_asq32(MaxwellLaunch L) {
     mx_asq_cell(L, run, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
-void launch_ghost32(const void *patches, const GhostOp *ops, int n, int slot, cudaStream_t s) {
-    if (n > 0) vx_launch(k_ghost32, (n + 127) / 128, 128, 0, s, (const PatchT<float> *)patches, ops, n, slot);
+void launch_ghost32(const void *patches, const GhostOp *ops, int n, const GhostOp *rows, int nrows, int slot,
+                    cudaStream_t s) {
+    const int blocks = ((n + 31) / 32 + nrows + 3) / 4;
+    vx_launch(k_ghost32, blocks, 128, 0, s, (const PatchT<float> *)patches, ops, n, rows, nrows, slot);
 }
 void launch_iface32(const void *patches, const IfaceOp *ops, int n, int step, cudaStream_t s) {
     if (n > 0) vx_launch(k_iface32, (n + 127) / 128, 128, 0, s, (const PatchT<float> *)patches, ops, n, step);

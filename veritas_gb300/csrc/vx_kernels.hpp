@@ -296,7 +296,9 @@ struct GhostOp;
 struct IfaceOp;
 struct CSyncOp;
 // `prec` selects the patch storage type (kF64 or kF32) of the descriptor array.
-void launch_ghost(const void *patches, const GhostOp *ops, int n, int slot, int prec, cudaStream_t s);
+// One batch of a ghost fill: n ops and nrows restriction rows.
+void launch_ghost(const void *patches, const GhostOp *ops, int n, const GhostOp *rows, int nrows, int slot, int prec,
+                  cudaStream_t s);
 void launch_iface(const void *patches, const IfaceOp *ops, int n, int step, const double *params, int prec, cudaStream_t s);
 // Launch-set op tables gathered on the device: segment s copies count ops from src to
 // dst + dst_off and adds base to their patch ids (the run's first patch in the set).
@@ -324,7 +326,8 @@ void launch_negate(double *dst, const double *src, int n, cudaStream_t s);
 // The op batches, assembly and Maxwell stage of FP32 launch sets, as kernels over the same
 // bodies as the persistent stage kernels below (one compilation, so the per-sub-step and
 // the persistent forms give the same bits).
-void launch_ghost32(const void *patches, const GhostOp *ops, int n, int slot, cudaStream_t s);
+void launch_ghost32(const void *patches, const GhostOp *ops, int n, const GhostOp *rows, int nrows, int slot,
+                    cudaStream_t s);
 void launch_iface32(const void *patches, const IfaceOp *ops, int n, int step, cudaStream_t s);
 void launch_csync32(const void *patches, const CSyncOp *ops, int n, cudaStream_t s);
 void launch_assemble32(const AsmLaunch &A);
@@ -354,6 +357,8 @@ struct Stage32Launch {
     MaxwellLaunch mx;  // Maxwell stage
     const GhostOp *ghost;  // op tables and their batch offsets (device arrays)
     const int *ghost_ptr;
+    const GhostOp *ghost_rows;  // restriction rows, same batches
+    const int *ghost_rptr;
     int nghost_b;
     const IfaceOp *iface;
     const int *iface_ptr;
