@@ -42,30 +42,47 @@ constexpr int kMaxR = 8;
 
 // Rectangle::GetWenoValueFromCoarseLevel (Rectangle.cpp:343-415): the corrected r x r
 // interpolants of coarse cell (ic, jc), out[kx * r + kp] for x sub-cell kx, p sub-cell kp.
-template <class T>
-__device__ void interp_block(const PatchT<T> &C, const T *f, int ic, int jc, T *out) {
-    const int r = C.r;
+// R: the refinement ratio when known at compile time (its arrays are then registers; with
+// the general bound they are 104 words of local memory per thread), 0 otherwise.
+template <int R, class T>
+__device__ __forceinline__ void interp_block_r(const PatchT<T> &C, const T *f, int ic, int jc, T *out) {
+    const int r = R ? R : C.r;
     const int pit = C.pitch;
-    T temps[5][kMaxR];
+    T temps[5][R ? R : kMaxR];
+#pragma unroll
     for (int k = -2; k < 3; k++)
         interp_ref(C.refc, r, f[pidx(ic - 2, jc + k, pit)], f[pidx(ic - 1, jc + k, pit)], f[pidx(ic, jc + k, pit)],
                    f[pidx(ic + 1, jc + k, pit)], f[pidx(ic + 2, jc + k, pit)], temps[k + 2]);
     T sum = 0;
+#pragma unroll
     for (int k = 0; k < r; k++) {
         interp_ref(C.refc, r, temps[0][k], temps[1][k], temps[2][k], temps[3][k], temps[4][k], out + k * r);
         for (int l = 0; l < r; l++) sum += out[k * r + l];
     }
     // 1 / r^2: r^2 is an exact small integer (the reference's std::pow(r, 2) gives it)
     T correction = f[pidx(ic, jc, pit)] - (T)1 / (T)(r * r) * sum;
+#pragma unroll
     for (int q = 0; q < r * r; q++) out[q] += correction;
+}
+template <class T>
+__device__ void interp_block(const PatchT<T> &C, const T *f, int ic, int jc, T *out) {
+    if (C.r == 2) interp_block_r<2>(C, f, ic, jc, out);
+    else interp_block_r<0>(C, f, ic, jc, out);
 }
 
 // Entry `sub` of interp_block.
 template <class T>
-__device__ T coarse_interp(const PatchT<T> &C, const T *f, int ic, int jc, int sub) {
+__device__ __noinline__ T coarse_interp_any(const PatchT<T> &C, const T *f, int ic, int jc, int sub) {
     T out[kMaxR * kMaxR];
-    interp_block(C, f, ic, jc, out);
+    interp_block_r<0>(C, f, ic, jc, out);
     return out[sub];
+}
+template <class T>
+__device__ __forceinline__ T coarse_interp(const PatchT<T> &C, const T *f, int ic, int jc, int sub) {
+    if (C.r != 2) return coarse_interp_any(C, f, ic, jc, sub);
+    T out[4];
+    interp_block_r<2>(C, f, ic, jc, out);
+    return sub == 0 ? out[0] : sub == 1 ? out[1] : sub == 2 ? out[2] : out[3];
 }
 
 template <class T>
