@@ -293,6 +293,7 @@ void Run::build_amr() {
                 R.nested.assign(cells, 0);
                 R.ifx.assign(cells, 0);
                 R.ifp.assign(cells, 0);
+                R.cmask.assign(cells, 0);
             }
     multi_patch = nrect > (int)rects.size();
     lap("cell arrays");
@@ -607,19 +608,52 @@ void Run::build_amr() {
             for (auto &rp : sp[l]) same_calls(*rp, kCUpdate);
     }
     sort_by_batch(csync_ops, cs.batch, cs.nbatches, csync_b);
-    lap("csync ops");
     validate_ops();
     lap("validate");
+    // The limiter's C and the update are one pass where no exchange intervenes.  A face of the
+    // exchange makes the two cells beside it wait: they are updated after it, from C values
+    // kept for all their faces.
+    late_ops.clear();
+    auto late = [&](int patch, int i, int j) {
+        Rect &R = *flat[patch];
+        if (i < 0 || i >= R.n_x || j < 0 || j >= R.n_p || (R.cmask[R.ns(i, j)] & kCLater)) return;
+        R.cmask[R.ns(i, j)] |= kCLater | kCStore;
+        R.cmask[R.ns(i + 1, j)] |= kCStore;
+        R.cmask[R.ns(i, j + 1)] |= kCStore;
+        late_ops.push_back({patch, i, j});
+    };
+    auto touched = [&](int patch, int i, int j, bool xf) {
+        Rect &R = *flat[patch];
+        R.cmask[R.ns(i, j)] |= kCStore;
+        late(patch, i, j);
+        late(patch, xf ? i - 1 : i, xf ? j : j - 1);
+    };
+    for (const CSyncOp &op : csync_ops) {
+        const bool xf = op.t < 2;
+        touched(op.nb, op.ni, op.nj, xf);
+        for (int k = 0; k < (op.kind == kCDiff ? r : 1); k++)
+            touched(op.caller, xf ? op.ci : op.ci + k, xf ? op.cj + k : op.cj, xf);
+    }
+    late_b.ptr = {0, (int)late_ops.size()};
+    lap("csync ops");
     dghost_ops = upload(ghost_ops, eng->stream);
     dghost_rows = upload(ghost_rows, eng->stream);
     diface_ops = upload(iface_ops, eng->stream);
     dcsync_ops = upload(csync_ops, eng->stream);
+    dlate_ops = upload(late_ops, eng->stream);
     lap("op upload");
 
     // ------------------------------------------------------------ device masks, weights
     for (Rect *R : flat) {
         const size_t pe = R->plane_elems();
-        std::vector<uint8_t> m(3 * pe, 0);
+        auto any = [](const std::vector<uint8_t> &v) {
+            return std::any_of(v.begin(), v.end(), [](uint8_t b) { return b != 0; });
+        };
+        R->any_nested = any(R->nested);
+        R->any_ifx = any(R->ifx);
+        R->any_ifp = any(R->ifp);
+        R->any_cmask = any(R->cmask);
+        std::vector<uint8_t> m(4 * pe, 0);
         // rows of (n_p + 4) cells in the reference's index order become pitched rows
         const size_t w = (size_t)R->n_p + 4;
         for (int i = -2; i < R->n_x + 2; i++) {
@@ -627,6 +661,7 @@ void Run::build_amr() {
             std::memcpy(&m[d], &R->nested[q], w);
             std::memcpy(&m[pe + d], &R->ifx[q], w);
             std::memcpy(&m[2 * pe + d], &R->ifp[q], w);
+            std::memcpy(&m[3 * pe + d], &R->cmask[q], w);
         }
         R->masks = DevBuf(m.size(), DevBuf::Uninit{});  // the blocking copy below fills it
         VX_CUDA(cudaMemcpy(R->masks.p, m.data(), m.size(), cudaMemcpyHostToDevice));

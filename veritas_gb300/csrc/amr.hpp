@@ -54,6 +54,12 @@ struct IfaceOp {
     int fine, fi, fj;
 };
 
+// A cell whose antidiffusive update waits for the limiter exchange: one of its faces takes
+// part in it.
+struct CellOp {
+    int patch, i, j;
+};
+
 // Error flags of one patch (Rectangle::getError): local cells [i0,i1) x [j0,j1) are
 // tested against crit with the patch's five error weights; out_off locates the patch's
 // n_x * n_p flag bytes.

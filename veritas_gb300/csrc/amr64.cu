@@ -108,6 +108,7 @@ __device__ __forceinline__ void rebase(GhostOp &op, int b) {
     op.dst += b;
     if (op.src >= 0) op.src += b;
 }
+__device__ __forceinline__ void rebase(CellOp &op, int b) { op.patch += b; }
 __device__ __forceinline__ void rebase(IfaceOp &op, int b) {
     op.coarse += b;
     op.fine += b;
@@ -132,6 +133,9 @@ __global__ void k_merge_ops(const OpSegment *segs, Op *dst) {
 constexpr int kMergeParts = 8;
 void merge_ghost_ops(const OpSegment *segs, int nseg, GhostOp *dst, cudaStream_t s) {
     if (nseg > 0) vx_launch_plain(k_merge_ops<GhostOp>, dim3(nseg, kMergeParts), 256, 0, s, segs, dst);
+}
+void merge_late_ops(const OpSegment *segs, int nseg, CellOp *dst, cudaStream_t s) {
+    if (nseg > 0) vx_launch_plain(k_merge_ops<CellOp>, dim3(nseg, kMergeParts), 256, 0, s, segs, dst);
 }
 void merge_iface_ops(const OpSegment *segs, int nseg, IfaceOp *dst, cudaStream_t s) {
     if (nseg > 0) vx_launch_plain(k_merge_ops<IfaceOp>, dim3(nseg, kMergeParts), 256, 0, s, segs, dst);

@@ -212,12 +212,13 @@ void Run::upload_rect_desc(Rect &r, int run_index) {
     if (r.masks.p) {
         const size_t pe = r.plane_elems();
         uint8_t *m = r.masks.as<uint8_t>();
-        d.nested = m;
-        d.ifx = m + pe;
-        d.ifp = m + 2 * pe;
-        d.has_iface = 1;
+        d.nested = r.any_nested ? m : nullptr;
+        d.ifx = r.any_ifx ? m + pe : nullptr;
+        d.ifp = r.any_ifp ? m + 2 * pe : nullptr;
+        d.cmask = r.any_cmask ? m + 3 * pe : nullptr;
+        d.has_iface = r.any_ifx || r.any_ifp;
     } else {
-        d.nested = d.ifx = d.ifp = nullptr;
+        d.nested = d.ifx = d.ifp = d.cmask = nullptr;
         d.has_iface = 0;
     }
 }
@@ -1093,6 +1094,8 @@ void Engine::build_set(LaunchSet &L) {
         gather(CSyncOp{}, [](Run &R) -> DevBuf & { return R.dcsync_ops; },
                [](Run &R) -> const std::vector<int> & { return R.csync_b.ptr; }, merge_csync_ops, L.dcsync,
                L.csync_ptr);
+        gather(CellOp{}, [](Run &R) -> DevBuf & { return R.dlate_ops; },
+               [](Run &R) -> const std::vector<int> & { return R.late_b.ptr; }, merge_late_ops, L.dlate, L.late_ptr);
         L.max_batch = 0;
         for (const std::vector<int> *p : {&L.ghost_ptr, &L.iface_ptr, &L.csync_ptr})
             for (size_t b = 0; b + 1 < p->size(); b++) L.max_batch = std::max(L.max_batch, (*p)[b + 1] - (*p)[b]);
@@ -1315,6 +1318,8 @@ StageLaunches Engine::stage_launches(LaunchSet &L) {
     fl.ptiles = L.dptiles.as<TileRef>();
     fl.nxtiles = L.nxtiles;
     fl.nptiles = L.nptiles;
+    fl.late = L.dlate.as<CellOp>();
+    fl.nlate = L.late_ptr.empty() ? 0 : L.late_ptr.back();
     fl.strip_rows = L.strip_rows;
     fl.fields = L.dfields.as<RunFields>();
     fl.params = L.dparams.as<double>();
@@ -1495,12 +1500,14 @@ void Engine::record_fct_tail(LaunchSet &L, const FctLaunch &fl, int s, cudaStrea
     if (s == 0) record_f2(L, fl, stream, launches);
     else if (f2_stream == side2) VX_CUDA(cudaStreamWaitEvent(stream, ev_f2, 0));
     fct_sub(L, fl, kSubLimR);
-    fct_sub(L, fl, kSubLimC);
+    fct_sub(L, fl, kSubCUpdate);
     launches += 2;
-    for (size_t b = 0; b + 1 < L.csync_ptr.size(); b++, launches++)
-        launch_csync(L.dpatch.p, L.dcsync.as<CSyncOp>() + L.csync_ptr[b], L.csync_ptr[b + 1] - L.csync_ptr[b], L.precision, stream);
-    fct_sub(L, fl, kSubUpdate);
-    launches += 1;
+    if (fl.nlate) {
+        for (size_t b = 0; b + 1 < L.csync_ptr.size(); b++, launches++)
+            launch_csync(L.dpatch.p, L.dcsync.as<CSyncOp>() + L.csync_ptr[b], L.csync_ptr[b + 1] - L.csync_ptr[b], L.precision, stream);
+        fct_sub(L, fl, kSubLate);
+        launches += 1;
+    }
     record_ghosts(L, 1, stream, launches);
     if (s == 5) {
         fct_sub(L, fl, kSubCopy10);

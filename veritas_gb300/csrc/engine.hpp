@@ -123,7 +123,7 @@ struct Rect {
     int pitch = 0;
     DevBuf slab;   // all per-patch planes
     DevBuf cols;   // chargeR, currentR
-    DevBuf masks;  // nested, ifx, ifp (AMR only)
+    DevBuf masks;  // nested, ifx, ifp, cmask
     // Device descriptor.  For FP32 runs the plane pointers address float planes: the
     // layout of PatchT<float> is identical (see the static_assert in engine.cpp), and the
     // host never dereferences them.
@@ -138,7 +138,8 @@ struct Rect {
     std::vector<int> xm, xp, pm, pp;
     std::vector<char> sxm, sxp, spm, spp;
     std::vector<int> finer, finer_x, finer_p;
-    std::vector<uint8_t> nested, ifx, ifp;
+    std::vector<uint8_t> nested, ifx, ifp, cmask;
+    bool any_nested = false, any_ifx = false, any_ifp = false, any_cmask = false;
     int ns(int i, int j) const { return (i + 2) * (n_p + 4) + (j + 2); }
 };
 
@@ -215,7 +216,9 @@ public:
     Batched csync_b;
     std::vector<IfaceOp> iface_ops;
     Batched iface_b;
-    DevBuf dghost_ops, dghost_rows, dcsync_ops, diface_ops;  // the op lists on the device (set tables gather them)
+    std::vector<CellOp> late_ops;  // cells updated after the limiter exchange (one batch)
+    Batched late_b;
+    DevBuf dghost_ops, dghost_rows, dcsync_ops, diface_ops, dlate_ops;  // the op lists on the device (set tables gather them)
     DevBuf drelc;                   // sub-cell interpolation weights per depth
     DevBuf drefc;                   // coarse-to-fine interpolation weights (refinement ratio)
     std::vector<int> relc_off;      // offset of depth d's weights in drelc
@@ -266,7 +269,7 @@ struct LaunchSet {
     DevBuf dparams32;
     std::vector<double> w, fcoef;
     // AMR op tables of all runs, batch by batch (global patch ids)
-    DevBuf dghost, dghost_rows, diface, dcsync;
+    DevBuf dghost, dghost_rows, diface, dcsync, dlate;
     int precision = kF64;
     int tile_j = 32, tile_i = 8;  // FCT tile (p x x) = thread block of the sub-step kernels
     DevBuf dxtiles, dptiles;      // FP32: strip tiles of the fused face + flux kernels
@@ -274,7 +277,7 @@ struct LaunchSet {
     int poisson = kPoissonLU;
     int fast64 = 0;  // FP64 sets: contracted FCT kernels
     DevBuf dpf;  // per-run PoissonFastDev (scan Poisson sets)
-    std::vector<int> ghost_ptr, ghost_rptr, iface_ptr, csync_ptr;
+    std::vector<int> ghost_ptr, ghost_rptr, iface_ptr, csync_ptr, late_ptr;
     DevBuf dghost_ptr, dghost_rptr, diface_ptr, dcsync_ptr;  // the batch offsets on the device (persistent form)
     int max_batch = 0;                          // largest op batch
     int launches_per_step = 0;                  // kernels of one recorded step
@@ -290,7 +293,7 @@ struct LaunchSet {
     // gathers, their segment lists
     std::unique_ptr<TablePack> pending_pack;
     std::vector<std::function<void()>> pending_gathers;
-    DevBuf dsegs[4];
+    DevBuf dsegs[5];
     cudaGraphExec_t graph = nullptr;
     ~LaunchSet();
 };
@@ -386,7 +389,9 @@ public:
     // queued by flush_prepared() (or their first use).
     void prepare(const std::vector<Run *> &set);
     void flush_prepared();
-    int tile_pref[2][2] = {{32, 8}, {128, 8}};  // [precision 64, 32] -> (tile_j, tile_i)
+    // [precision 64, 32] -> (tile_j, tile_i); FP32: four rows (38.6 M cells 10.7 ms per step, eight
+    // rows 11.1, two 10.7; 2.8 M cells 1.17, 1.19, 1.17)
+    int tile_pref[2][2] = {{32, 8}, {128, 4}};
 
 private:
     std::map<std::vector<Run *>, std::unique_ptr<LaunchSet>> sets_;

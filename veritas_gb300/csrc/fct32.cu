@@ -16,9 +16,16 @@ __global__ void k32_f2(const P32 *patches, const TileRef *tiles, const float *pa
     VX_PDL_WAIT();
     f2_32(patches, tiles[blockIdx.x], (int)threadIdx.x, (int)threadIdx.y, params, s);
 }
-__global__ void k32_limR(const P32 *patches, const TileRef *tiles) {
+// Limiter R, and C with the update: 64 registers (two blocks of the largest tile shape per
+// SM), a few less than the compiler takes by itself, for the warps in flight: limiter R 204
+// -> 185 us on 38.6 M cells; a third block's 42 registers spill (235 us).
+__global__ void __launch_bounds__(512, 2) k32_limR(const P32 *patches, const TileRef *tiles) {
     VX_PDL_WAIT();
     limR32(patches, tiles[blockIdx.x], (int)threadIdx.x, (int)threadIdx.y);
+}
+__global__ void __launch_bounds__(512, 2) k32_cupdate(const P32 *patches, const TileRef *tiles) {
+    VX_PDL_WAIT();
+    cupdate32(patches, tiles[blockIdx.x], (int)threadIdx.x, (int)threadIdx.y);
 }
 __global__ void k32_limC(const P32 *patches, const TileRef *tiles) {
     VX_PDL_WAIT();
@@ -27,6 +34,11 @@ __global__ void k32_limC(const P32 *patches, const TileRef *tiles) {
 __global__ void k32_update(const P32 *patches, const TileRef *tiles) {
     VX_PDL_WAIT();
     update32(patches, tiles[blockIdx.x], (int)threadIdx.x, (int)threadIdx.y);
+}
+__global__ void k32_late(const P32 *patches, const CellOp *ops, int n) {
+    VX_PDL_WAIT();
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < n) late_update32(patches, ops, k);
 }
 __global__ void k32_copy10(const P32 *patches, const TileRef *tiles) {
     VX_PDL_WAIT();
@@ -69,6 +81,12 @@ void launch_fct32_substep(const FctLaunch &L, int sub) {
             break;
         case kSubUpdate:
             vx_launch(k32_update, L.ntiles, blk, 0, L.stream, pp, L.tiles);
+            break;
+        case kSubCUpdate:
+            vx_launch(k32_cupdate, L.ntiles, blk, 0, L.stream, pp, L.tiles);
+            break;
+        case kSubLate:
+            if (L.nlate) vx_launch(k32_late, (L.nlate + 127) / 128, 128, 0, L.stream, pp, L.late, L.nlate);
             break;
         case kSubCopy10:
             vx_launch(k32_copy10, L.ntiles, blk, 0, L.stream, pp, L.tiles);

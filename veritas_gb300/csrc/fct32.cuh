@@ -20,6 +20,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include "amr.hpp"
 #include "vx_kernels.hpp"
 
 namespace vx {
@@ -136,36 +137,6 @@ __device__ __forceinline__ void ds_32(const P32 *patches, const TileRef t, int t
     st4(P.FpDS + id, dp, j, -2, P.np + 2);
 }
 
-// Low-order solution (Rectangle.cpp:1518-1534) on the interior.  It needs only the step's
-// stage-0 fluxes: after stage 0 it and the ghost cells it feeds are formed beside the
-// stage's field work, off the chain from the solve to the update.
-__device__ __forceinline__ void f2_32(const P32 *patches, const TileRef t, int tx, int row, const float *params, int s) {
-    VX_VTILE32
-    if (i < 0 || i >= P.nx || j + 3 < 0 || j >= P.np) return;
-    const float asum = params[param_base(P.run, s) + 6];
-    const V4 lx = ld4(P.FxL + id), lp = ld4(P.FpL + id);
-    const V4 f0 = ld4(P.f0 + id), lxn = ld4(P.FxL + id + pit);
-    const float lp4 = (j + 3 < P.np) ? P.FpL[id + 4] : 0.0f;  // j + 4 <= np
-    // the cell's own low-order fluxes are shared with its neighbours in the row: rounded once
-    V4 lsx, lsp, f2;
-#pragma unroll
-    for (int e = 0; e < 4; e++) {
-        lsx.v[e] = __fmul_rn(asum, lx.v[e]);
-        lsp.v[e] = __fmul_rn(asum, lp.v[e]);
-    }
-#pragma unroll
-    for (int e = 0; e < 4; e++) {
-        const int je = j + e;
-        float v = f0.v[e];
-        if (active32(P, i, je)) v += lsx.v[e];
-        if (active32(P, i, je)) v += lsp.v[e];
-        if (active32(P, i, je + 1)) v = e < 3 ? v - lsp.v[e + 1] : __fmaf_rn(-asum, lp4, v);
-        if (active32(P, i + 1, je)) v = __fmaf_rn(-asum, lxn.v[e], v);
-        f2.v[e] = v;
-    }
-    st4(P.f2 + id, f2, j, 0, P.np);
-}
-
 // min(1, Q / P) for P > 0, else 0 (Q >= 0: a stencil extremum minus the centre value).
 // Q >= P gives 1 without a quotient; otherwise the hardware reciprocal (within 2 ulp),
 // except for a subnormal P, where it is not defined and IEEE division is used.
@@ -175,37 +146,123 @@ __device__ __forceinline__ float limiter_ratio(float Q, float P) {
     return fminf(1.0f, P >= 1.17549435e-38f ? __fdividef(Q, P) : Q / P);
 }
 
+// ---- sub-steps that read neighbours in x and p
+// One warp per row of a tile, four p cells per lane.  The p neighbours past a lane's four
+// cells come from the next lanes; only the tile's two edge lanes load theirs (every lane
+// loading its own cost as much in L1 as five more planes, and L1 bounded these kernels: 38.6
+// M cells, C and update in one pass 335 us per stage against 137 us for its six planes).
+// Walking several rows with one warp, each row of a plane loaded once, needs 72 to 86
+// registers and was slower (limiter R 199 against 186 us, 27 against 16 us on 2.8 M cells).
+#define VX_ROW32                                                  \
+    const P32 &P = patches[t.patch];                              \
+    const int i = t.i0 + row; /* warp-uniform */                  \
+    const int j = t.j0 + 4 * lane, pit = P.pitch;                 \
+    const bool col = j <= P.np + 1; /* four cells inside a row */ \
+    const unsigned full = 0xffffffffu;
+
+__device__ __forceinline__ V4 ld4_if(bool ok, const float *p) { return ok ? ld4(p) : V4{{0.0f, 0.0f, 0.0f, 0.0f}}; }
+__device__ __forceinline__ V4 max4(const V4 &a, const V4 &b) {
+    V4 r;
+#pragma unroll
+    for (int e = 0; e < 4; e++) r.v[e] = fmaxf(a.v[e], b.v[e]);
+    return r;
+}
+__device__ __forceinline__ V4 min4(const V4 &a, const V4 &b) {
+    V4 r;
+#pragma unroll
+    for (int e = 0; e < 4; e++) r.v[e] = fminf(a.v[e], b.v[e]);
+    return r;
+}
+
+// Low-order solution (Rectangle.cpp:1518-1534) on the interior.  It needs only the step's
+// stage-0 fluxes: after stage 0 it and the ghost cells it feeds are formed beside the
+// stage's field work, off the chain from the solve to the update.
+__device__ __forceinline__ void f2_32(const P32 *patches, const TileRef t, int lane, int row, const float *params, int s) {
+    VX_ROW32
+    if (i < 0 || i >= P.nx) return;
+    const int id = pidx(i, j, pit);
+    const float asum = params[param_base(P.run, s) + 6];
+    const V4 lx = ld4_if(col, P.FxL + id), lp = ld4_if(col, P.FpL + id);
+    const V4 f0 = ld4_if(col, P.f0 + id), lxn = ld4_if(col, P.FxL + id + pit);
+    float lp4 = __shfl_down_sync(full, lp.v[0], 1);
+    if (lane == 31) lp4 = (j + 3 < P.np) ? P.FpL[id + 4] : 0.0f;  // j + 4 <= np
+    // the cell's own low-order fluxes are shared with its neighbours in the row: rounded once
+    V4 lsx, lsp, f2;
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+        lsx.v[e] = __fmul_rn(asum, lx.v[e]);
+        lsp.v[e] = __fmul_rn(asum, lp.v[e]);
+    }
+    const bool ai = i >= P.xm && i < P.xp, an = i + 1 >= P.xm && i + 1 < P.xp;
+    const int lo = P.pm - j, hi = P.pp - j;
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+        const bool aj = e >= lo && e < hi, ajn = e + 1 >= lo && e + 1 < hi;
+        float v = f0.v[e];
+        if (ai && aj) v += lsx.v[e];
+        if (ai && aj) v += lsp.v[e];
+        if (ai && ajn) v = e < 3 ? v - lsp.v[e + 1] : __fmaf_rn(-asum, lp4, v);
+        if (an && aj) v = __fmaf_rn(-asum, lxn.v[e], v);
+        f2.v[e] = v;
+    }
+    if (col) st4(P.f2 + id, f2, j, 0, P.np);
+}
+
 // Zalesak R+ and R- (Rectangle.cpp:1536-1582), cells i in [-1, nx], j in [-1, np].
-__device__ __forceinline__ void limR32(const P32 *patches, const TileRef t, int tx, int row) {
-    VX_VTILE32
-    if (i < -1 || i > P.nx || j + 3 < -1 || j > P.np) return;
+__device__ __forceinline__ void limR32(const P32 *patches, const TileRef t, int lane, int row) {
+    VX_ROW32
+    if (i < -1 || i > P.nx) return;
+    const int id = pidx(i, j, pit);
     const float *DX = P.FxDS, *DP = P.FpDS, *f0 = P.f0, *f2 = P.f2;
-    const V4 dxi = ld4(DX + id), dxn = ld4(DX + id + pit), dpi = ld4(DP + id);
-    const V4 a0 = ld4(f0 + id), a2 = ld4(f2 + id);
-    const V4 u0 = ld4(f0 + id + pit), u2 = ld4(f2 + id + pit);
-    const V4 d0 = ld4(f0 + id - pit), d2 = ld4(f2 + id - pit);
-    const bool lo_ok = j >= -1, hi_ok = j + 3 <= P.np;  // element 0 / element 3 valid
-    const float l0 = lo_ok ? f0[id - 1] : 0.0f, l2 = lo_ok ? f2[id - 1] : 0.0f;
-    const float r0 = hi_ok ? f0[id + 4] : 0.0f, r2 = hi_ok ? f2[id + 4] : 0.0f;
-    const float dp4 = hi_ok ? DP[id + 4] : 0.0f;
-    V4 rp, rm;
+    const V4 dxi = ld4_if(col, DX + id), dxn = ld4_if(col, DX + id + pit), dpi = ld4_if(col, DP + id);
+    // the cell beyond the tile's edge that lane 0 (j - 1) and lane 31 (j + 4) need
+    const bool edge = (lane == 0 && j >= -1) || (lane == 31 && j + 3 <= P.np);
+    const float edp = (edge && lane == 31) ? DP[id + 4] : 0.0f;
+    float dp4 = __shfl_down_sync(full, dpi.v[0], 1);
+    if (lane == 31) dp4 = edp;
+    V4 Pp, Pm, rp, rm;
+    bool some = false;
 #pragma unroll
     for (int e = 0; e < 4; e++) {
         const float dpn = e < 3 ? dpi.v[e + 1] : dp4;
-        const float Pp = fmaxf(0.0f, dxi.v[e]) - fminf(0.0f, dxn.v[e]) + fmaxf(0.0f, dpi.v[e]) - fminf(0.0f, dpn);
-        const float Pm = fmaxf(0.0f, dxn.v[e]) - fminf(0.0f, dxi.v[e]) + fmaxf(0.0f, dpn) - fminf(0.0f, dpi.v[e]);
-        const float c0 = a0.v[e], c2 = a2.v[e];
-        const float lf0 = e > 0 ? a0.v[e - 1] : l0, lf2 = e > 0 ? a2.v[e - 1] : l2;
-        const float rf0 = e < 3 ? a0.v[e + 1] : r0, rf2 = e < 3 ? a2.v[e + 1] : r2;
-        const float wMax = fmaxf(fmaxf(c0, c2), fmaxf(fmaxf(u0.v[e], u2.v[e]),
-                           fmaxf(fmaxf(d0.v[e], d2.v[e]), fmaxf(fmaxf(rf0, rf2), fmaxf(lf0, lf2)))));
-        const float wMin = fminf(fminf(c0, c2), fminf(fminf(u0.v[e], u2.v[e]),
-                           fminf(fminf(d0.v[e], d2.v[e]), fminf(fminf(rf0, rf2), fminf(lf0, lf2)))));
-        const float Qm = -wMin + c2;
-        const float Qp = wMax - c2;
-        rp.v[e] = limiter_ratio(Qp, Pp);
-        rm.v[e] = limiter_ratio(Qm, Pm);
+        Pp.v[e] = fmaxf(0.0f, dxi.v[e]) - fminf(0.0f, dxn.v[e]) + fmaxf(0.0f, dpi.v[e]) - fminf(0.0f, dpn);
+        Pm.v[e] = fmaxf(0.0f, dxn.v[e]) - fminf(0.0f, dxi.v[e]) + fmaxf(0.0f, dpn) - fminf(0.0f, dpi.v[e]);
+        some = some || Pp.v[e] > 0.0f || Pm.v[e] > 0.0f;
+        rp.v[e] = rm.v[e] = 0.0f;
     }
+    // nothing flows in or out of any of the warp's cells (empty phase space): R is 0
+    if (__any_sync(full, some)) {
+        const V4 a0 = ld4_if(col, f0 + id), c2 = ld4_if(col, f2 + id);
+        const V4 u0 = ld4_if(col, f0 + id + pit), u2 = ld4_if(col, f2 + id + pit);
+        const V4 d0 = ld4_if(col, f0 + id - pit), d2 = ld4_if(col, f2 + id - pit);
+        float e0 = 0.0f, e2 = 0.0f;
+        if (edge) {
+            const int eoff = lane == 0 ? -1 : 4;
+            e0 = f0[id + eoff];
+            e2 = f2[id + eoff];
+        }
+        const V4 mxc = max4(a0, c2), mnc = min4(a0, c2);
+        float lmx = __shfl_up_sync(full, mxc.v[3], 1), lmn = __shfl_up_sync(full, mnc.v[3], 1);
+        float rmx = __shfl_down_sync(full, mxc.v[0], 1), rmn = __shfl_down_sync(full, mnc.v[0], 1);
+        if (lane == 0) {
+            lmx = fmaxf(e0, e2);
+            lmn = fminf(e0, e2);
+        }
+        if (lane == 31) {
+            rmx = fmaxf(e0, e2);
+            rmn = fminf(e0, e2);
+        }
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            const float wMax = fmaxf(fmaxf(mxc.v[e], fmaxf(fmaxf(u0.v[e], u2.v[e]), fmaxf(d0.v[e], d2.v[e]))),
+                                     fmaxf(e < 3 ? mxc.v[e + 1] : rmx, e > 0 ? mxc.v[e - 1] : lmx));
+            const float wMin = fminf(fminf(mnc.v[e], fminf(fminf(u0.v[e], u2.v[e]), fminf(d0.v[e], d2.v[e]))),
+                                     fminf(e < 3 ? mnc.v[e + 1] : rmn, e > 0 ? mnc.v[e - 1] : lmn));
+            rp.v[e] = limiter_ratio(wMax - c2.v[e], Pp.v[e]);
+            rm.v[e] = limiter_ratio(-wMin + c2.v[e], Pm.v[e]);
+        }
+    }
+    if (!col) return;
     st4(P.Rp + id, rp, j, -1, P.np + 1);
     st4(P.Rm + id, rm, j, -1, P.np + 1);
 }
@@ -254,6 +311,121 @@ __device__ __forceinline__ void update32(const P32 *patches, const TileRef t, in
         out.v[e] = v;
     }
     st4(P.f1 + id, out, j, 0, P.np);
+}
+
+// The two above in one pass, for the cells beside which no limiter exchange takes place: C
+// of a cell's four faces is formed from R where it is used, so neither C plane is written
+// or read (six planes moved instead of twelve).  Cells of the exchange (cmask) keep their C
+// values for it and are updated after it (late_update32).  Where no flux is left to limit
+// (empty phase space, smooth regions at rest) R is not read.
+__device__ __forceinline__ void cupdate32(const P32 *patches, const TileRef t, int lane, int row) {
+    VX_ROW32
+    if (i > P.nx + 1) return;
+    const int id = pidx(i, j, pit), np = P.np;
+    unsigned mask = 0;
+    if (P.cmask && col) mask = *reinterpret_cast<const unsigned *>(P.cmask + id);  // four cells' bytes
+    const V4 one{{1.0f, 1.0f, 1.0f, 1.0f}};
+    V4 cx = one, cp = one;  // C is 1 outside the interior
+    if (i >= 0 && i < P.nx) {
+        const float *Rp = P.Rp, *Rm = P.Rm, *DX = P.FxDS, *DP = P.FpDS;
+        const bool in = i >= 1, inn = i + 1 < P.nx;  // rows i and i + 1 have faces between cells
+        V4 dx = ld4_if(col, DX + id), dxn = ld4_if(col, DX + id + pit), dp = ld4_if(col, DP + id);
+        const V4 f2 = ld4_if(col, P.f2 + id);
+        float edp = 0.0f;
+        if (lane == 31 && j + 3 < np) edp = DP[id + 4];
+        // fluxes outside the face window count as zero
+        const bool ai = i >= P.xm && i < P.xp, an = i + 1 >= P.xm && i + 1 < P.xp;
+        const int lo = P.pm - j, hi = P.pp - j;
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            const bool aj = e >= lo && e < hi;
+            if (!(ai && aj)) dx.v[e] = 0.0f;
+            if (!(an && aj)) dxn.v[e] = 0.0f;
+            if (!(ai && aj)) dp.v[e] = 0.0f;
+        }
+        float dp4 = __shfl_down_sync(full, dp.v[0], 1);
+        if (lane == 31) dp4 = (ai && 4 >= lo && 4 < hi) ? edp : 0.0f;
+        bool some = mask != 0 || dp4 != 0.0f;
+#pragma unroll
+        for (int e = 0; e < 4; e++) some = some || dx.v[e] != 0.0f || dxn.v[e] != 0.0f || dp.v[e] != 0.0f;
+        if (!__any_sync(full, some)) {
+            if (col) st4(P.f1 + id, f2, j, 0, np);
+            return;
+        }
+        const V4 rpc = ld4_if(col, Rp + id), rmc = ld4_if(col, Rm + id);
+        const V4 rpd = ld4_if(col && in, Rp + id - pit), rmd = ld4_if(col && in, Rm + id - pit);
+        const V4 rpn = ld4_if(col && inn, Rp + id + pit), rmn = ld4_if(col && inn, Rm + id + pit);
+        // R beyond the tile's edge: lane 0 the cell j - 1, lane 31 the cell j + 4
+        float ep = 0.0f, em = 0.0f;
+        if ((lane == 0 && j >= 0) || (lane == 31 && j + 4 < np)) {
+            const int eoff = lane == 0 ? -1 : 4;
+            ep = Rp[id + eoff];
+            em = Rm[id + eoff];
+        }
+        // C of a face between two cells, from R of the upper (p, m) and the lower (l, lm) and its flux
+        auto face = [](float flux, float p, float m, float l, float lm) {
+            const bool up = flux > 0.0f;
+            return fminf(up ? p : l, up ? lm : m);
+        };
+        float lp = __shfl_up_sync(full, rpc.v[3], 1), lm = __shfl_up_sync(full, rmc.v[3], 1);
+        if (lane == 0) {
+            lp = ep;
+            lm = em;
+        }
+        V4 cxn = one;
+        if (in) {
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                cx.v[e] = face(dx.v[e], rpc.v[e], rmc.v[e], rpd.v[e], rmd.v[e]);
+                const float c = face(dp.v[e], rpc.v[e], rmc.v[e], e > 0 ? rpc.v[e - 1] : lp, e > 0 ? rmc.v[e - 1] : lm);
+                cp.v[e] = j + e < np ? c : 1.0f;
+            }
+        }
+        if (inn) {
+#pragma unroll
+            for (int e = 0; e < 4; e++) cxn.v[e] = face(dxn.v[e], rpn.v[e], rmn.v[e], rpc.v[e], rmc.v[e]);
+        }
+        float cp4 = __shfl_down_sync(full, cp.v[0], 1);
+        if (lane == 31) cp4 = (in && j + 4 < np) ? face(edp, ep, em, rpc.v[3], rmc.v[3]) : 1.0f;
+        // a p face between two cells of the four: its product is rounded once and used twice
+        V4 w, out;
+#pragma unroll
+        for (int e = 0; e < 4; e++) w.v[e] = __fmul_rn(cp.v[e], dp.v[e]);
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            float v = __fmaf_rn(cx.v[e], dx.v[e], f2.v[e]);
+            v = e > 0 ? v + w.v[e] : __fmaf_rn(cp.v[0], dp.v[0], v);
+            v = e < 3 ? v - w.v[e + 1] : __fmaf_rn(-cp4, dp4, v);
+            out.v[e] = __fmaf_rn(-cxn.v[e], dxn.v[e], v);
+        }
+        if (col) st4(P.f1 + id, out, j, 0, np);
+    }
+    if (mask) {
+#pragma unroll
+        for (int e = 0; e < 4; e++)
+            if (((mask >> (8 * e)) & kCStore) && j + e < np + 2) {
+                const bool out = j + e < 0 || j + e >= np;
+                P.Cx[id + e] = out ? 1.0f : cx.v[e];
+                P.Cp[id + e] = out ? 1.0f : cp.v[e];
+            }
+    }
+}
+#undef VX_ROW32
+
+// The update of a cell beside an exchanged face, from the C planes; rounded as the passes
+// above round the cell of its place in the four (e = (j + 2) mod 4).
+__device__ __forceinline__ void late_update32(const P32 *patches, const CellOp *ops, int k) {
+    const CellOp op = ops[k];
+    const P32 &P = patches[op.patch];
+    const int i = op.i, j = op.j, pit = P.pitch, id = pidx(i, j, pit), e = (j + 2) & 3;
+    float v = P.f2[id];
+    if (active32(P, i, j)) v = __fmaf_rn(P.Cx[id], P.FxDS[id], v);
+    if (active32(P, i, j))
+        v = e > 0 ? v + __fmul_rn(P.Cp[id], P.FpDS[id]) : __fmaf_rn(P.Cp[id], P.FpDS[id], v);
+    if (active32(P, i, j + 1))
+        v = e < 3 ? v - __fmul_rn(P.Cp[id + 1], P.FpDS[id + 1]) : __fmaf_rn(-P.Cp[id + 1], P.FpDS[id + 1], v);
+    if (active32(P, i + 1, j)) v = __fmaf_rn(-P.Cx[id + pit], P.FxDS[id + pit], v);
+    P.f1[id] = v;
 }
 
 // f0 = f1 over the padded block (Rectangle.cpp:1614-1621).

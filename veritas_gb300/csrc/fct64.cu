@@ -17,6 +17,7 @@
 // Newton-refined hardware reciprocal instead of five IEEE divisions).  Its kernels
 // live in namespace vx::fast64 and its launcher is launch_fct64_substep_fast.
 #include <cuda_runtime.h>
+#include "amr.hpp"
 #include "div64.cuh"
 #include "fast64.cuh"
 #include "vx_kernels.hpp"
@@ -453,6 +454,68 @@ __global__ void k64_update(const P64 *patches, const TileRef *tiles) {
     P.f1[id] = v;
 }
 
+// The two above in one pass, for the cells beside which no limiter exchange takes place: C
+// of a cell's four faces is formed from R where it is used, so neither C plane is written
+// or read.  Cells of the exchange (cmask) keep their C values for it and are updated
+// after it (late_update).
+__global__ void k64_cupdate(const P64 *patches, const TileRef *tiles) {
+    VX_PDL_WAIT();
+    VX_TILE_PROLOGUE
+    if (i < -2 || j < -2) return;
+    const uint8_t mask = P.cmask ? P.cmask[id] : 0;
+    const bool cell = i >= 0 && i < P.nx && j >= 0 && j < P.np;
+    if (!cell && !(mask & kCStore)) return;
+    const double *Rp = P.Rp, *Rm = P.Rm, *DX = P.FxDS, *DP = P.FpDS;
+    auto face_x = [&](int a, int k, double d) {  // C of x face (a, j), k its index
+        if (!(a >= 1 && a < P.nx)) return 1.0;
+        const bool up = gt0(d);
+        return vmin_r(Rp[up ? k : k - pit], Rm[up ? k - pit : k]);
+    };
+    auto face_p = [&](int b, int k, double d) {  // C of p face (i, b)
+        if (!(i >= 1 && i < P.nx && b < P.np)) return 1.0;
+        const bool up = gt0(d);
+        return vmin_r(Rp[up ? k : k - 1], Rm[up ? k - 1 : k]);
+    };
+    double cx = 1.0, cp = 1.0;
+    if (cell) {
+        const double dx = DX[id], dp = DP[id];
+        cx = face_x(i, id, dx);
+        cp = face_p(j, id, dp);
+        double v = P.f2[id];
+        if (active_face(P, i, j)) v += cx * dx;
+        if (active_face(P, i, j)) v += cp * dp;
+        if (active_face(P, i, j + 1)) {
+            const double d = DP[id + 1];
+            v -= face_p(j + 1, id + 1, d) * d;
+        }
+        if (active_face(P, i + 1, j)) {
+            const double d = DX[id + pit];
+            v -= face_x(i + 1, id + pit, d) * d;
+        }
+        P.f1[id] = v;
+    }
+    if (mask & kCStore) {
+        P.Cx[id] = cx;
+        P.Cp[id] = cp;
+    }
+}
+
+// The update of the cells beside an exchanged face, from the C planes.
+__global__ void k64_late(const P64 *patches, const CellOp *ops, int n) {
+    VX_PDL_WAIT();
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= n) return;
+    const CellOp op = ops[k];
+    const P64 &P = patches[op.patch];
+    const int i = op.i, j = op.j, pit = P.pitch, id = pidx(i, j, pit);
+    double v = P.f2[id];
+    if (active_face(P, i, j)) v += P.Cx[id] * P.FxDS[id];
+    if (active_face(P, i, j)) v += P.Cp[id] * P.FpDS[id];
+    if (active_face(P, i, j + 1)) v -= P.Cp[id + 1] * P.FpDS[id + 1];
+    if (active_face(P, i + 1, j)) v -= P.Cx[id + pit] * P.FxDS[id + pit];
+    P.f1[id] = v;
+}
+
 // Last stage: f0 = f1 over the padded block (Rectangle.cpp:1614-1621).
 __global__ void k64_copy10(const P64 *patches, const TileRef *tiles) {
     VX_PDL_WAIT();
@@ -494,6 +557,12 @@ void VX_FCT64_LAUNCH(const FctLaunch &L, int sub) {
             break;
         case kSubUpdate:
             vx_launch(k64_update, L.ntiles, blk, 0, L.stream, pp, L.tiles);
+            break;
+        case kSubCUpdate:
+            vx_launch(k64_cupdate, L.ntiles, blk, 0, L.stream, pp, L.tiles);
+            break;
+        case kSubLate:
+            if (L.nlate) vx_launch(k64_late, (L.nlate + 127) / 128, 128, 0, L.stream, pp, L.late, L.nlate);
             break;
         case kSubCopy10:
             vx_launch(k64_copy10, L.ntiles, blk, 0, L.stream, pp, L.tiles);

@@ -32,7 +32,7 @@ size_t Run::device_bytes() const {
     for (const DevBuf *d : {&dBy, &dBz, &dEy, &dEz, &dAy, &dAz, &dasq, &dphi, &dcharge, &dJ, &dneut, &defin, &dex0,
                             &dasq32, &defin32, &dacell32, &drelc32, &dlu_perm, &dlb_band, &dlb_fptr, &dlb_fcol, &dlb_fval, &dlb_slot,
                             &dlb_sload, &dlb_take, &dub_band, &dub_diag, &dub_sweep, &dub_fptr, &dub_fcol,
-                            &dub_fval, &dpf_Y, &drelc, &drefc, &dghost_ops, &dghost_rows, &diface_ops, &dcsync_ops})
+                            &dub_fval, &dpf_Y, &drelc, &drefc, &dghost_ops, &dghost_rows, &diface_ops, &dcsync_ops, &dlate_ops})
         b += d->bytes;
     return b;
 }

@@ -229,16 +229,19 @@ __global__ void __launch_bounds__(kStageThreads, 5) k32_stage_fct(Stage32Launch 
     for_tiles(F, [&](const TileRef &t, int tx, int row) { limR32(patches, t, tx, row); });
     for_cells(mxn, [&](long long e) { mx_asq_cell(X, (int)(e / X.maxnf), (int)(e % X.maxnf)); });
     bar.sync();
-    // limiter C, then its exchange across patch edges (Mesh::PushBoundaryC), batch by batch
-    for_tiles(F, [&](const TileRef &t, int tx, int row) { limC32(patches, t, tx, row); });
+    // limiter C and the update; then the exchange of C across patch edges (Mesh::PushBoundaryC),
+    // batch by batch, and the update of the cells beside it
+    for_tiles(F, [&](const TileRef &t, int tx, int row) { cupdate32(patches, t, tx, row); });
     bar.sync();
-    for (int b = 0; b < L.ncsync_b; b++) {
-        for_ops(L.csync_ptr, b, [&](int k) { csync_op(patches, L.csync, k); });
+    if (F.nlate) {
+        for (int b = 0; b < L.ncsync_b; b++) {
+            for_ops(L.csync_ptr, b, [&](int k) { csync_op(patches, L.csync, k); });
+            bar.sync();
+        }
+        for_cells(F.nlate, [&](long long e) { late_update32(patches, F.late, (int)e); });
         bar.sync();
     }
-    // antidiffusive update, then the ghost cells of f1 (Mesh::PushData(1))
-    for_tiles(F, [&](const TileRef &t, int tx, int row) { update32(patches, t, tx, row); });
-    bar.sync();
+    // the ghost cells of f1 (Mesh::PushData(1))
     for (int b = 0; b < L.nghost_b; b++) {
         for_ghosts(L, b, patches, 1);
         if (b + 1 < L.nghost_b || s == 5) bar.sync();

@@ -72,8 +72,10 @@ struct PatchT {
     T *FxL, *FpL;           // stage-0 low-order fluxes
     T *FxDS, *FpDS;         // antidiffusive stage fluxes
     T *Rp, *Rm, *Cx, *Cp;   // Zalesak limiter
+    // byte planes; null where the patch has nothing set
     uint8_t *nested;        // is_nested (cells covered by a finer patch)
     uint8_t *ifx, *ifp;     // is_interrior_level_boundary_x / _p
+    uint8_t *cmask;         // kCStore: keep this cell's C values, kCLater: cell updated after the exchange
     double *chargeR, *currentR;  // per finest column of this patch (n_x * rtb)
     const double *relc;     // interpolation weights onto the rtb finest sub-cells, 3*rtb
     const double *refc;     // interpolation weights onto the r sub-cells of a coarse cell, 3*r
@@ -96,6 +98,8 @@ struct RunFields {
     float *asq32;       // FP32 copies of asq (n+1) and efin (n) for the FP32 form
     float *efin32;
 };
+
+constexpr uint8_t kCStore = 1, kCLater = 2;
 
 VX_HD inline int pidx(int i, int j, int pitch) { return (i + 2) * pitch + (j + 2); }
 

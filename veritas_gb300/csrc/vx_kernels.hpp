@@ -66,6 +66,8 @@ enum FctSub : int {
     kSubLimC,
     kSubUpdate,
     kSubCopy10,
+    kSubCUpdate,  // limiter C and update in one pass (but for the cells of the limiter exchange)
+    kSubLate,     // the update of those, after the exchange
     // FP32 form only: gamma + x faces + x fluxes, and p faces + p fluxes, each fused
     // and the stage flux combination (the FP64 flux kernels form it)
     kSubXFlux,
@@ -73,6 +75,7 @@ enum FctSub : int {
     kSubDS,
 };
 
+struct CellOp;
 struct FctLaunch {
     const void *patches;  // device array of PatchT<T>
     const TileRef *tiles;
@@ -89,6 +92,8 @@ struct FctLaunch {
     // FP32 fused face + flux kernels: one warp per strip tile
     const TileRef *xtiles, *ptiles;
     int nxtiles, nptiles, strip_rows;
+    const CellOp *late;  // cells updated after the limiter exchange
+    int nlate;
     cudaStream_t stream;
 };
 constexpr int kMaxStripRows = 16;  // rows per strip tile of the fused FP32 face + flux kernels, at most
@@ -293,6 +298,7 @@ void launch_fp64_latency(long long *cyc, double *val, int iters, cudaStream_t s)
 
 // AMR op batches (amr.hpp, amr64.cu)
 struct GhostOp;
+struct CellOp;
 struct IfaceOp;
 struct CSyncOp;
 // `prec` selects the patch storage type (kF64 or kF32) of the descriptor array.
@@ -307,6 +313,7 @@ struct OpSegment {
     long long dst_off;
     int count, base;
 };
+void merge_late_ops(const OpSegment *segs, int nseg, CellOp *dst, cudaStream_t s);
 void merge_ghost_ops(const OpSegment *segs, int nseg, GhostOp *dst, cudaStream_t s);
 // bytes (a multiple of 16) from page-locked host memory, given by its device address, to
 // device memory, copied by a kernel
