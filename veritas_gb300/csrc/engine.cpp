@@ -1539,7 +1539,9 @@ PipeLaunch Engine::pipe_launch(LaunchSet &L, const StageLaunches &K) {
     P.nitems = L.pipe_nitems;
     P.scratch = L.dpipe_scratch.as<double>();
     P.summers = L.pipe_summers;
-    P.workers = std::max(1, std::min(num_sms_ - (int)L.runs.size() - P.summers, (L.pipe_nitems + 1) / 2));
+    const int parts = L.pipe_nitems * kPipeParts, blocks = std::max(1, num_sms_ - (int)L.runs.size() - P.summers);
+    P.groups = std::min(kPipeGroups, std::max(1, (parts + blocks - 1) / blocks));
+    P.workers = std::min(blocks, (parts + P.groups - 1) / P.groups);
     P.need = L.dpipe_need.as<int>();
     P.ndone = L.pipe_ndone;
     P.run_ctr = L.dpipe_runctr.as<int>();

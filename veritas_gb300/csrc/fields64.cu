@@ -1089,18 +1089,18 @@ __device__ __forceinline__ void mom_sum_unit(const PipeLaunch &K, int u, int lan
     }
 }
 
-// A group of a worker block: column warps 0 .. kMomCols-1 take items until none are left;
-// the warp that completes a unit (the unit's item count reaches its total) appends the
-// unit to the queue of completed units.  They never wait for anything but each other.
+// A group of a worker block: kPipeCols column warps take parts of items until none are
+// left; the warp that completes a unit (its part count reaches its total) appends the unit
+// to the queue of completed units.  They never wait for anything but each other.
 template <bool FAST>
-__device__ void pipe_columns(const PipeLaunch &K, int *ticket, int g) {
-    const int tid = (int)threadIdx.x - g * kMomThreads, wid = tid >> 5, lane = tid & 31;
-    const int bar = 1 + g, ncol = kMomCols * 32;
+__device__ void pipe_columns(const PipeLaunch &K, int *ticket, int g, int tid) {
+    const int wid = tid >> 5, lane = tid & 31;
+    const int bar = 1 + g, ncol = kPipeCols * 32, nparts = K.nitems * kPipeParts;
     unsigned *items_done = K.state + kPipeDone + K.ndone;      // per unit
     unsigned *queue = items_done + K.nunits;                    // completed units (u + 1), in order
-    // an item of unit u is done: the last one queues the unit
+    // a part of unit u is done: the last one queues the unit
     auto count = [&](int u) {
-        const unsigned total = (unsigned)(K.unit_item0[u + 1] - K.unit_item0[u]);
+        const unsigned total = (unsigned)(K.unit_item0[u + 1] - K.unit_item0[u]) * kPipeParts;
         if (atomicAdd(items_done + u, 1u) + 1 == total) {
             __threadfence();  // every item's contributions before a summing warp reads them
             const unsigned slot = atomicAdd(K.state + kPipeQHead, 1u);
@@ -1117,22 +1117,23 @@ __device__ void pipe_columns(const PipeLaunch &K, int *ticket, int g) {
             int t;
             for (;;) {
                 t = (int)atomicAdd(K.state + kPipeTicket, 1u);
-                if (t >= K.nitems) break;
-                const int u = K.item_unit[t];
+                if (t >= nparts) break;
+                const int u = K.item_unit[t / kPipeParts];
                 int kp;
-                const int w = window(t, u, kp);
+                const int w = window(t / kPipeParts, u, kp);
                 if (K.M.screen[((size_t)(K.unit_col0[u] / kMomCols) * K.M.maxnwin + w) * kMomScreen + kMomCols]) break;
                 count(u);
             }
             ticket[it & 1] = t;
         }
         pipe_bar(bar, ncol);
-        const int t = ticket[it & 1];
-        if (t >= K.nitems) break;
+        const int tk = ticket[it & 1];
+        if (tk >= nparts) break;
+        const int t = tk / kPipeParts, c = (tk - t * kPipeParts) * kPipeCols + wid;
         const int u = K.item_unit[t];
         int kp;
         const int w = window(t, u, kp);
-        mom_item<FAST>(K, u, 2 * kp, w * kMomOut, wid, lane, K.scratch + (size_t)t * kPipeItemDoubles);
+        if (c < kMomCols) mom_item<FAST>(K, u, 2 * kp, w * kMomOut, c, lane, K.scratch + (size_t)t * kPipeItemDoubles);
         __threadfence();  // this warp's contributions, device-wide, before the item counts
         pipe_bar(bar, ncol);
         if (tid == 0) count(u);
@@ -1179,7 +1180,7 @@ __device__ void pipe_summer(const PipeLaunch &K, int lane) {
 // Moments, assembly and the exact solve in one launch.  Block r < nruns solves run r (its
 // forward sweep starts as soon as the moments of its first rows are summed, instead of
 // after the whole moments kernel); the next K.summers blocks carry four summing warps each
-// (pipe_summer); every other block carries two groups of column warps (pipe_columns).
+// (pipe_summer); every other block carries up to kPipeGroups groups of column warps (pipe_columns).
 // Column warps wait for nothing outside their group, summing warps only for column
 // warps, the solve only for summing warps: every wait ends whatever order the blocks are
 // scheduled in.  Same arithmetic as k64_moments + k_assemble + k_poisson.
@@ -1195,8 +1196,8 @@ __global__ void __launch_bounds__(1024, 1) k64_moments_poisson(PipeLaunch K) {
         if (threadIdx.x < 4 * 32) pipe_summer<FAST>(K, (int)threadIdx.x & 31);  // warps 0..3: one per sub-partition
     } else {
         int *ticket = reinterpret_cast<int *>(smem_raw);
-        const int g = (int)threadIdx.x / kMomThreads;
-        if (((int)threadIdx.x & (kMomThreads - 1)) < kMomCols * 32) pipe_columns<FAST>(K, ticket + 2 * g, g);
+        const int g = (int)threadIdx.x / (kPipeCols * 32);
+        if (g < K.groups) pipe_columns<FAST>(K, ticket + 2 * g, g, (int)threadIdx.x - g * kPipeCols * 32);
     }
     // the last block out zeroes the tickets, the queue, done and item counters for the next launch
     __syncthreads();
@@ -1237,7 +1238,7 @@ void launch_moments_poisson64(const PipeLaunch &K0) {
     const int base = 2 * (int)sizeof(PoisChunk);
     K.P.x_in_smem = (K.P.maxn <= kPoisSmemMaxN && base + 8 * K.P.maxn <= max_smem) ? 1 : 0;
     const int smem_solve = base + (K.P.x_in_smem ? 8 * K.P.maxn : 0);
-    const int smem = std::max(smem_solve, 16);
+    const int smem = std::max(smem_solve, 2 * (int)sizeof(int) * kPipeGroups);
     auto kern = K.M.fast ? k64_moments_poisson<true> : k64_moments_poisson<false>;
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     cudaLaunchConfig_t cfg = {};

@@ -185,17 +185,28 @@ constexpr int kPoisRowsHost = 256;  // rows per chunk of k_poisson (fields64.cu 
 
 // Moments, assembly and exact Poisson solve of an FP64 set in one launch
 // (k64_moments_poisson): blocks 0 .. nruns-1 solve, each following its run's moments as
-// they are completed; the other blocks are persistent workers.  Column warps (two groups
-// of 15 per worker block) take items — one p window of one moment unit's 15 columns (one
-// pair of sub-columns) — by ticket in the order the forward sweeps first need the units'
-// columns, and write each cell's charge and current contributions to `scratch`; the warp
-// that completes a unit's last item queues the unit.  Summing warps (four per summing
+// they are completed; the other blocks are persistent workers.  Groups of kPipeCols column
+// warps take parts of items — an item is one p window of one moment unit's 15 columns (one
+// pair of sub-columns), a part kPipeCols of the columns — by ticket in the order the
+// forward sweeps first need the units' columns, and write each cell's charge and current
+// contributions to `scratch`; the warp that completes a unit's last part queues the unit.  Summing warps (four per summing
 // block, one per sub-partition) take queued units in order, add their contributions in
 // ascending p (the reference's order) and add one to the done counter of the chunk that
 // needs the unit first.  The solve waits (bounded) for a chunk's counter before it
 // assembles rho and J at the x positions whose right-hand sides the chunk reads first.
 constexpr int kPipeErr = 0, kPipeTicket = 32, kPipeLeave = 64, kPipeQHead = 96, kPipeQTail = 128,
               kPipeDone = 160;  // words of the state (each on its own 128-byte line)
+// Columns of an item that a group of column warps forms at a time: one warp for each
+// sub-partition's FP64 unit, which one warp's dependent chain keeps busy (latency and
+// occupancy of an FP64 instruction are both about 64 cycles).  All 15 at a time held the
+// item for four times as long, which small sets and every forward sweep's first chunk wait
+// for: step of 50 x 38 in two levels 0.99 -> 0.78 ms, of 2048 x 256 3.94 -> 3.87 ms, 512 x
+// 128 with ions 68.3 -> 64.0 ms per 23 steps, 4096 x 512 in two levels the same.
+constexpr int kPipeCols = 4, kPipeParts = (kMomCols + kPipeCols - 1) / kPipeCols;
+// Groups per worker block: the second covers the first's loads and barriers (one, two,
+// four, eight: 4096 x 512 15.5, 14.95, 14.94, 14.94 ms, 512 x 128 68.4, 64.0, 64.8, 69.2);
+// one where every group then has a block of its own (50 x 38: 0.78, 0.82, 0.89, 0.96).
+constexpr int kPipeGroups = 2;
 constexpr int kPipeMaxRuns = 4;  // sets of more runs keep separate launches (each solve holds an SM)
 constexpr int kPipeItemDoubles = 2 * 32 * 30;  // per item: [cc, cj][lane t][column w][sub-column q]
 constexpr size_t kPipeMaxScratch = (size_t)2 << 30;  // larger sets keep separate launches
@@ -224,6 +235,7 @@ struct PipeLaunch {
     int phantom;             // units each wait expects beyond the real ones (> 0: every wait runs out)
     int priority;            // launch priority (the moments go ahead of the face kernels beside them)
     int summers;             // summing blocks
+    int groups;              // groups per column-warp block, at most kPipeGroups
     int workers;             // column-warp blocks
     // Optional globaltimer trace (ns) of run 0: [0] the solve's start, [1 + c] chunk c's rows
     // ready, [1 + trace_nch + k] the last unit of done counter k summed; the solve's own
