@@ -596,7 +596,8 @@ static void run_moments(const LaunchSet &L, const MomLaunch &ml) {
     if (L.precision == kF32) launch_moments32(ml);
     else launch_moments64(ml);
 }
-static void run_poisson(const LaunchSet &L, const PoissonLaunch &pl) {
+// A: the scan solve forms rho and J first (AsmLaunch's work)
+static void run_poisson(const LaunchSet &L, const PoissonLaunch &pl, const AsmLaunch *A = nullptr) {
     if (L.poisson == kPoissonScan) {
         PoissonFastLaunch f{};
         f.pf = L.dpf.as<PoissonFastDev>();
@@ -607,6 +608,10 @@ static void run_poisson(const LaunchSet &L, const PoissonLaunch &pl) {
         f.maxn = pl.maxn;
         f.f32 = L.precision == kF32;
         f.stream = pl.stream;
+        if (A) {
+            f.A = *A;
+            f.assemble = 1;
+        }
         launch_poisson_fast(f);
     } else {
         launch_poisson(pl);
@@ -1400,14 +1405,15 @@ void Engine::record_step(LaunchSet &L) {
         // runs beside the face kernels that read it, so it cannot write the copy).
         ml.acell = s == 0;
         run_moments(L, ml);
-        launch_assemble(al);
-        launches += (L.precision == kF32 && s != 0) ? 2 : 3;  // FP64: with the moments' screen
+        const bool fuse = L.poisson == kPoissonScan && L.maxn <= kPsAssembleMaxN;  // the solve assembles
+        if (!fuse) launch_assemble(al);
+        launches += (fuse ? -1 : 0) + ((L.precision == kF32 && s != 0) ? 2 : 3);  // FP64: with the moments' screen
         // the Poisson solve (and E_x) runs beside the x-direction face work, which does
         // not read E_x; the p-direction faces wait for both
         VX_CUDA(cudaEventRecord(ev_fork, stream));
         VX_CUDA(cudaStreamWaitEvent(side, ev_fork, 0));
         pl.stream = side;
-        run_poisson(L, pl);
+        run_poisson(L, pl, fuse ? &al : nullptr);
         launches += 1;  // the scan solve forms E_x itself
         fl.step = s;
         // The Maxwell stage (EMFieldSolver::RGKStep) writes A and a^2, which the Vlasov

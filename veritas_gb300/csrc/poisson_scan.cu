@@ -16,12 +16,12 @@
 // One thread-block cluster per run: the kPsCluster blocks of a cluster hold consecutive
 // chunks of the vector in shared memory (T segments of L elements each, stored
 // segment-minor so that a warp's threads walk their segments on different banks).  A
-// pass runs every segment serially, then fixes the segments up with their carry: the
-// prefix sum of the preceding segment sums (a block scan plus the preceding blocks' totals
-// read through distributed shared memory), or for the decaying recurrences the sum over
-// preceding segment ends weighted by rho^{L (q-1)}, which drops below 1e-20 after a few
-// segments (three for L >= 8, which the block size is chosen for).  The cluster barriers
-// are hardware barriers of co-scheduled blocks.
+// pass runs every segment serially; its carry — the prefix sum of the preceding segment
+// sums (a block scan plus the preceding blocks' totals read through distributed shared
+// memory), or for the decaying recurrences the sum over preceding segment ends weighted by
+// rho^{L (q-1)}, which drops below 1e-20 after a few segments (three for L >= 8, which the
+// block size is chosen for) — is added as the next pass runs.  The cluster barriers are
+// hardware barriers of co-scheduled blocks.
 //
 // FP64 throughout, with fused multiply-adds (E_x itself comes from k_efield, which keeps
 // the reference's rounding).  The result is not the LU's rounding order; both have the
@@ -30,6 +30,10 @@
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <utility>
+
+#include "field_ops.cuh"
 #include "vx_kernels.hpp"
 
 namespace vx {
@@ -39,121 +43,124 @@ namespace {
 namespace cg = cooperative_groups;
 
 constexpr int kPsMaxTerms = 24;  // carry-gather terms of a decaying pass (rho^24 < 1e-27)
+constexpr int kPsGather = 4;     // of them, loaded together
+// Threads beyond the T of the scans: they share the element-wise work (an FP64 instruction
+// of a warp takes about 64 cycles of its sub-partition, so a block of one warp would use a
+// quarter of the SM's units), and the last warp forms the values at the vector's ends.
+constexpr int kPsMinThreads = 128;
 
-// E_x at cell i (EMSolver::GetEfield order); phi read past L1, since other blocks of the
-// cluster wrote it in this launch.
-__device__ __forceinline__ double efield_at(const double *phi, int n, double fcoef, double ex0, int i) {
-    int ip1 = i + 1, im1 = i - 1, ip2 = i + 2, im2 = i - 2;
-    ip1 = (ip1 > -1) ? ip1 : (ip1 + n);
-    im1 = (im1 > -1) ? im1 : (im1 + n);
-    ip2 = (ip2 > -1) ? ip2 : (ip2 + n);
-    im2 = (im2 > -1) ? im2 : (im2 + n);
-    ip1 = (ip1 < n) ? ip1 : (ip1 - n);
-    im1 = (im1 < n) ? im1 : (im1 - n);
-    ip2 = (ip2 < n) ? ip2 : (ip2 - n);
-    im2 = (im2 < n) ? im2 : (im2 - n);
-    return -fcoef * (8 * (__ldcg(phi + ip1) - __ldcg(phi + im1)) - __ldcg(phi + ip2) + __ldcg(phi + im2)) + ex0;
-}
-
-// Exclusive scan of one value per thread, in thread order; the block's total goes to *tot.
-__device__ double block_exclusive_sum(double v, double *sb, double *tot) {
-    const unsigned full = 0xffffffffu;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int nw = blockDim.x >> 5;
-    double x = v;
-    for (int o = 1; o < 32; o <<= 1) {
-        const double p = __shfl_up_sync(full, x, o);
-        if (lane >= o) x = x + p;
-    }
-    if (lane == 31) sb[wid] = x;
-    __syncthreads();
-    if (wid == 0) {
-        double w = (lane < nw) ? sb[lane] : 0.0;
-        for (int o = 1; o < 32; o <<= 1) {
-            const double p = __shfl_up_sync(full, w, o);
-            if (lane >= o) w = w + p;
-        }
-        sb[lane] = w;
-        if (lane == nw - 1) *tot = w;
-    }
-    __syncthreads();
-    double ex = __shfl_up_sync(full, x, 1);
-    if (lane == 0) ex = 0.0;
-    if (wid > 0) ex = sb[wid - 1] + ex;
-    return ex;
-}
-
-// Per-block scratch of a pass.
+// Per-block scratch of the passes.  Each pass has its own cells for what other blocks read
+// (sa, s_tot), so that no cluster barrier is needed before the next pass writes.
 struct ScanScratch {
-    double *sa;     // [T] segment ends without carry (read across the cluster)
-    double *sb;     // [32] warp totals
-    double *pw;     // [L] mult^(s+1) of the decaying passes
-    double *wt;     // [kPsMaxTerms] rho^(L q) carry weights
-    double *s_tot;  // block total of a prefix-sum pass (read across the cluster)
-    double *s_pre;  // preceding blocks' totals
-    int nterms;     // carry terms of a decaying pass
+    double sa[2][kPsMaxThreads];  // decaying passes: segment ends without carry (read across the cluster)
+    double s_tot[2];              // prefix sums: block totals (read across the cluster)
+    double sb[32];                // warp totals
+    double pw[kPsMaxSeg];         // rho^(s+1)
+    double wt[kPsMaxTerms];       // rho^(L q) carry weights
+    double s_pre;                 // preceding blocks' totals
+    int nterms;                   // carry terms of a decaying pass
 };
 
-// y_k = v_k + mult y_{k-1} over the run's m unknowns, in place, ascending (or descending
-// when REV); mult = 1 when UNIT.  Thread t owns segment t (REV: segment T-1-t, so thread
-// order is scan order either way); blocks are in scan order by rank (REV: reversed).
-// Segments past the end of the vector are short or empty; in scan order they come last
-// (REV: first), so no full-length weight ever crosses one.
-template <bool REV, bool UNIT>
-__device__ void scan_pass(cg::cluster_group &cl, double *xs, int L, int m, int g0, double mult, const ScanScratch &W) {
+// Carry into thread tid's segment of a prefix-sum pass: the preceding blocks' totals in scan
+// order, plus the block's exclusive scan (thread order) of the segment sums y.
+template <bool REV>
+__device__ double sum_carry(cg::cluster_group &cl, ScanScratch &W, int T, double y) {
+    const unsigned full = 0xffffffffu;
     constexpr int C = kPsCluster;
-    const int T = blockDim.x, stride = T + 1;
-    const int rank = (int)cl.block_rank();
-    const int tid = threadIdx.x;
-    const int seg = REV ? T - 1 - tid : tid;
-    const int len = max(0, min(L, m - (g0 + seg * L)));
-    double y = 0.0;
-    for (int s = 0; s < len; s++) {
-        double *p = &xs[(REV ? len - 1 - s : s) * stride + seg];
-        y = UNIT ? (*p + y) : (*p + mult * y);
-        *p = y;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nw = T >> 5;
+    const int rank = (int)cl.block_rank(), cpos = REV ? C - 1 - rank : rank;
+    double x = y;
+    if (wid < nw) {
+        for (int o = 1; o < 32; o <<= 1) {
+            const double p = __shfl_up_sync(full, x, o);
+            if (lane >= o) x = x + p;
+        }
+        if (lane == 31) W.sb[wid] = x;
     }
-    const int cpos = REV ? C - 1 - rank : rank;  // this block's place in scan order
-    double carry;
-    if (UNIT) {
-        const double ex = block_exclusive_sum(y, W.sb, W.s_tot);
-        cl.sync();
-        if (tid == 0) {
-            double pre = 0.0;
-            for (int q = 0; q < cpos; q++) pre = pre + *cl.map_shared_rank(W.s_tot, REV ? C - 1 - q : q);
-            *W.s_pre = pre;
+    if (nw > 1) {
+        __syncthreads();
+        if (wid == 0) {
+            double w = (lane < nw) ? W.sb[lane] : 0.0;
+            for (int o = 1; o < nw; o <<= 1) {
+                const double p = __shfl_up_sync(full, w, o);
+                if (lane >= o) w = w + p;
+            }
+            W.sb[lane] = w;
+            if (lane == nw - 1) W.s_tot[REV] = w;
         }
         __syncthreads();
-        carry = *W.s_pre + ex;
-    } else {
-        W.sa[tid] = y;
-        cl.sync();
-        // carry = sum_q rho^{L (q-1)} y_end(sp - q): terms below 1e-20 relative are dropped
-        const int sp = cpos * T + tid;
-        const int nq = min(W.nterms, sp);
-        carry = 0.0;
-        for (int q = 1; q <= nq; q++) {
-            const int src = sp - q;
-            const int r = REV ? C - 1 - src / T : src / T;
-            carry = carry + W.wt[q - 1] * cl.map_shared_rank(W.sa, r)[src % T];
-        }
+    } else if (tid == 31) {
+        W.s_tot[REV] = x;
     }
-    cl.sync();  // every remote read of sa / s_tot is done before the next pass rewrites them
-    for (int s = 0; s < len; s++) {
-        double *p = &xs[(REV ? len - 1 - s : s) * stride + seg];
-        *p = *p + (UNIT ? carry : W.pw[s] * carry);
+    auto arrival = cl.barrier_arrive();
+    double ex = 0.0;
+    if (wid < nw) {
+        ex = __shfl_up_sync(full, x, 1);
+        if (lane == 0) ex = 0.0;
+        if (wid > 0) ex = W.sb[wid - 1] + ex;
+    }
+    cl.barrier_wait(std::move(arrival));
+    if (tid == 0) {
+        double v[C - 1];
+#pragma unroll
+        for (int q = 0; q < C - 1; q++) v[q] = q < cpos ? cl.map_shared_rank(W.s_tot, REV ? C - 1 - q : q)[REV] : 0.0;
+        double pre = 0.0;
+#pragma unroll
+        for (int q = 0; q < C - 1; q++)
+            if (q < cpos) pre = pre + v[q];
+        W.s_pre = pre;
     }
     __syncthreads();
+    return W.s_pre + ex;
 }
 
-__global__ void __cluster_dims__(kPsCluster, 1, 1) __launch_bounds__(kPsMaxThreads)
+// Carry into thread tid's segment of a decaying pass, from the segment ends y:
+// sum_q rho^{L (q-1)} y_end(sp - q), terms below 1e-20 relative dropped.
+template <bool REV>
+__device__ double decay_carry(cg::cluster_group &cl, ScanScratch &W, int T, double y) {
+    constexpr int C = kPsCluster;
+    const int tid = threadIdx.x, rank = (int)cl.block_rank();
+    if (tid < T) W.sa[REV][tid] = y;
+    cl.sync();
+    double carry = 0.0;
+    if (tid < T) {
+        const int sp = (REV ? C - 1 - rank : rank) * T + tid, nq = min(W.nterms, sp);
+        for (int q0 = 1; q0 <= nq; q0 += kPsGather) {  // the remote reads of a group in flight together
+            double v[kPsGather];
+#pragma unroll
+            for (int k = 0; k < kPsGather; k++) {
+                const int src = sp - q0 - k;
+                v[k] = q0 + k <= nq ? cl.map_shared_rank(W.sa[REV], REV ? C - 1 - src / T : src / T)[src % T] : 0.0;
+            }
+#pragma unroll
+            for (int k = 0; k < kPsGather; k++)
+                if (q0 + k <= nq) carry = carry + W.wt[q0 + k - 1] * v[k];
+        }
+    }
+    return carry;
+}
+
+// phi of unknown g from its element of (c z) and the Woodbury coefficients t.
+__device__ __forceinline__ double phi_value(const PoissonFastDev &D, int g, double v, const double t[3]) {
+    const double z = v * D.c_inv;
+    return z - (D.Y[3 * g] * t[0] + D.Y[3 * g + 1] * t[1] + D.Y[3 * g + 2] * t[2]);
+}
+
+// With P.assemble the launch forms rho and J from the moments too (one cell per thread),
+// instead of a launch of its own before it.  Six cluster barriers: one per pass for its
+// carries, one before the Woodbury entries are read, one before phi replaces the vector.
+// The solve is latency from end to end (the FP64 units are idle most of the time): 13.4 us
+// at n = 1062 and 22.7 us at n = 8192, against 21.4 and 26.9 us with eleven barriers, the
+// remote reads one at a time and E_x read back from global memory.
+__global__ void __cluster_dims__(kPsCluster, 1, 1) __launch_bounds__(kPsMaxThreads + 32)
     k_poisson_scan(PoissonFastLaunch P) {
     VX_PDL_WAIT();
     extern __shared__ double xs[];  // [L][T + 1]: element (segment s, offset o) at o (T + 1) + s
-    __shared__ double sa[kPsMaxThreads], sb[32], pw[kPsMaxSeg], wt[kPsMaxTerms], s_tot, s_pre, s_u[3];
-    __shared__ int s_nterms;
+    __shared__ ScanScratch W;
+    __shared__ double s_halo[4], s_phi0, s_ex0;
     cg::cluster_group cl = cg::this_cluster();
-    const int T = blockDim.x, stride = T + 1;
+    const unsigned full = 0xffffffffu;
+    const int T = P.scan_threads, NT = blockDim.x, stride = T + 1, tid = threadIdx.x;
     const int run = blockIdx.x / kPsCluster;
     const int rank = (int)cl.block_rank();
     RunFields &F = P.fields[run];
@@ -161,80 +168,154 @@ __global__ void __cluster_dims__(kPsCluster, 1, 1) __launch_bounds__(kPsMaxThrea
     const int n = F.n, m = n - 1;
     const int L = (m + T * kPsCluster - 1) / (T * kPsCluster);
     const int g0 = rank * T * L;  // first unknown of this block's chunk
+    const int cnt = max(0, min(T * L, m - g0));
+    const double rho = D.rho;
     // right-hand side (dx^2 / eps0) (rho + rho_neutral), x_k = b_{k+1}
     const double te = kEps0Inv, w = P.w[run];
-    for (int l = threadIdx.x; l < T * L; l += T) {
-        const int g = g0 + l;
-        double v = 0.0;
-        if (g < m) {
-            const double r = te * (F.charge[g + 1] + F.neut[g + 1]);
-            v = r * w;
-        }
-        xs[(l % L) * stride + l / L] = v;
+    for (int l = tid; l < cnt; l += NT) {
+        if (P.assemble) assemble_cell(P.A, run, g0 + l + 1);
+        const double r = te * (F.charge[g0 + l + 1] + F.neut[g0 + l + 1]);
+        xs[(l % L) * stride + l / L] = r * w;
     }
-    if (threadIdx.x == 0) {  // powers by repeated products (a library pow is a long FP64 chain here)
-        double x = D.rho;
+    const bool ends = tid >= NT - 32;  // the last warp: the values at the ends of the vector
+    const int lane = tid & 31;
+    double b0 = 0.0, ex_old = 0.0;
+    if (ends) {
+        if (P.assemble && lane == 0) assemble_cell(P.A, run, 0);  // every block: the same values
+        __syncwarp();
+        const double r0 = te * (F.charge[0] + F.neut[0]);
+        b0 = r0 * w;
+        ex_old = *F.ex0;  // rewritten after the last barrier
+    }
+    if (tid == NT - 32) {  // powers by repeated products (a library pow is a long FP64 chain here)
+        double x = rho;
         for (int q = 0; q < L; q++) {
-            pw[q] = x;
-            x = x * D.rho;
+            W.pw[q] = x;
+            x = x * rho;
         }
-        const double aL = pw[L - 1];
+        const double aL = W.pw[L - 1];
         x = 1.0;
         int q = 0;
         while (q < kPsMaxTerms && x > 1e-20) {
-            wt[q++] = x;
+            W.wt[q++] = x;
             x = x * aL;
         }
-        s_nterms = q;
+        W.nterms = q;
     }
     __syncthreads();
-    const ScanScratch W{sa, sb, pw, wt, &s_tot, &s_pre, s_nterms};
-    scan_pass<false, true>(cl, xs, L, m, g0, 1.0, W);    // (I - S)^{-1}
-    scan_pass<false, false>(cl, xs, L, m, g0, D.rho, W);  // (I - rho S)^{-1}
-    scan_pass<true, false>(cl, xs, L, m, g0, D.rho, W);   // (I - rho S^T)^{-1}
-    scan_pass<true, true>(cl, xs, L, m, g0, 1.0, W);     // (I - S^T)^{-1}
-    cl.sync();  // every chunk final before the Woodbury entries are read across blocks
-    if (threadIdx.x < 3) {
-        const int g = threadIdx.x == 2 ? m - 1 : threadIdx.x;
+    // Thread t < T owns segment t, in the descending passes segment T - 1 - t, so that thread
+    // order is scan order either way; blocks are in scan order by rank.  Segments past the
+    // end of the vector are short or empty; in scan order they come last (descending:
+    // first), so no full-length weight ever crosses one.
+    {  // (I - S)^{-1}, then (I - rho S)^{-1}, ascending
+        double *seg = xs + tid;
+        const int len = tid < T ? max(0, min(L, cnt - tid * L)) : 0;
+        double y = 0.0;
+        for (int s = 0; s < len; s++) {
+            y = seg[s * stride] + y;
+            seg[s * stride] = y;
+        }
+        const double c1 = sum_carry<false>(cl, W, T, y);
+        y = 0.0;
+        for (int s = 0; s < len; s++) {
+            const double v = seg[s * stride] + c1;
+            y = v + rho * y;
+            seg[s * stride] = y;
+        }
+        const double c2 = decay_carry<false>(cl, W, T, y);
+        for (int s = 0; s < len; s++) seg[s * stride] = seg[s * stride] + W.pw[s] * c2;
+    }
+    __syncthreads();
+    {  // (I - rho S^T)^{-1}, then (I - S^T)^{-1}, descending
+        double *seg = xs + (T - 1 - tid);
+        const int len = tid < T ? max(0, min(L, cnt - (T - 1 - tid) * L)) : 0;
+        double y = 0.0;
+        for (int s = len - 1; s >= 0; s--) {
+            y = seg[s * stride] + rho * y;
+            seg[s * stride] = y;
+        }
+        const double c1 = decay_carry<true>(cl, W, T, y);
+        y = 0.0;
+        for (int s = len - 1; s >= 0; s--) {
+            const double v = seg[s * stride] + W.pw[len - 1 - s] * c1;
+            y = v + y;
+            seg[s * stride] = y;
+        }
+        const double c2 = sum_carry<true>(cl, W, T, y);
+        for (int s = len - 1; s >= 0; s--) seg[s * stride] = seg[s * stride] + c2;
+    }
+    cl.sync();  // every chunk final
+    // the element of unknown g, from the block that holds it
+    auto remote = [&](int g) {
         const int r = g / (T * L), l = g - r * T * L;
-        s_u[threadIdx.x] = cl.map_shared_rank(xs, r)[(l % L) * stride + l / L] * D.c_inv;
+        return cl.map_shared_rank(xs, r)[(l % L) * stride + l / L];
+    };
+    // The block's cells: phi index p0 .. p1-1 (block 0 holds phi_0 too).
+    const int p0 = rank == 0 ? 0 : g0 + 1, p1 = g0 + cnt + 1;
+    double u[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++) u[k] = remote(k == 2 ? m - 1 : k);
+    // The last warp's lanes: phi at 1, 2, n - 3, n - 2, n - 1 (phi_0 and Ex0 come from them)
+    // and at the two cells on either side of the block's.
+    int pe = 0;
+    double ve = 0.0;
+    if (ends && lane < 9) {
+        pe = lane < 2 ? lane + 1 : lane < 5 ? n - 5 + lane : lane < 7 ? p0 - 7 + lane : p1 - 7 + lane;
+        pe = pe < 0 ? pe + n : pe >= n ? pe - n : pe;
+        if (pe > 0) ve = remote(pe - 1);
+    }
+    auto arrival = cl.barrier_arrive();
+    double t[3];
+    for (int r = 0; r < 3; r++) {
+        const double s0 = u[0] * D.c_inv, s1 = u[1] * D.c_inv, s2 = u[2] * D.c_inv;
+        t[r] = D.K[3 * r] * s0 + D.K[3 * r + 1] * s1 + D.K[3 * r + 2] * s2;
+    }
+    const double fc = P.fcoef[run];
+    double ex0 = 0.0;
+    if (ends) {
+        double ph = (lane < 9 && pe > 0) ? phi_value(D, pe - 1, ve, t) : 0.0;
+        const double q1 = __shfl_sync(full, ph, 0), q2 = __shfl_sync(full, ph, 1), z3 = __shfl_sync(full, ph, 2),
+                     z2 = __shfl_sync(full, ph, 3), z1 = __shfl_sync(full, ph, 4);
+        const double phi0 = b0 - (D.w1 * q1 + D.w2 * q2 + D.w2 * z2 + D.w1 * z1);
+        const double e_m1 = -fc * (8 * (phi0 - z2) - q1 + z3) + ex_old;
+        const double e_0 = -fc * (8 * (q1 - z1) - q2 + z2) + ex_old;
+        ex0 = ex_old + -(e_m1 + e_0) * 0.5;
+        if (lane >= 5 && lane < 9) s_halo[lane - 5] = pe > 0 ? ph : phi0;
+        if (lane == 0) {
+            s_phi0 = phi0;
+            s_ex0 = ex0;
+        }
+    }
+    cl.barrier_wait(std::move(arrival));  // no block reads another's vector any more
+    for (int l = tid; l < cnt; l += NT) {
+        double *p = &xs[(l % L) * stride + l / L];
+        const double v = phi_value(D, g0 + l, *p, t);
+        *p = v;
+        F.phi[g0 + l + 1] = v;
+    }
+    if (rank == 0 && tid == NT - 32) {
+        F.phi[0] = s_phi0;
+        *F.ex0 = ex0;
     }
     __syncthreads();
-    double t[3];
-    for (int r = 0; r < 3; r++) t[r] = D.K[3 * r] * s_u[0] + D.K[3 * r + 1] * s_u[1] + D.K[3 * r + 2] * s_u[2];
-    for (int l = threadIdx.x; l < T * L; l += T) {
-        const int g = g0 + l;
-        if (g >= m) break;
-        const double z = xs[(l % L) * stride + l / L] * D.c_inv;
-        F.phi[g + 1] = z - (D.Y[3 * g] * t[0] + D.Y[3 * g + 1] * t[1] + D.Y[3 * g + 2] * t[2]);
-    }
-    __threadfence();
-    cl.sync();  // phi[1..n-1] written; no block touches another's shared memory after this
-    if (rank == 0 && threadIdx.x == 0) {
-        double *phi = F.phi;
-        const double r0 = te * (F.charge[0] + F.neut[0]);
-        phi[0] = r0 * w - (D.w1 * __ldcg(phi + 1) + D.w2 * __ldcg(phi + 2) + D.w2 * __ldcg(phi + n - 2) +
-                           D.w1 * __ldcg(phi + n - 1));
-        __threadfence_block();
-        const double ex0 = *F.ex0;
-        const double e_m1 = efield_at(phi, n, P.fcoef[run], ex0, -1);
-        const double e_0 = efield_at(phi, n, P.fcoef[run], ex0, 0);
-        *F.ex0 = ex0 + -(e_m1 + e_0) * 0.5;
-        __threadfence();
-    }
-    cl.sync();  // phi[0] and the new Ex0 are visible to every block of the cluster
-    // E_x on the finest grid (EMFieldSolver::GetEfield), each block a contiguous share
-    const double ex0 = __ldcg(F.ex0), fc = P.fcoef[run];
-    const int share = (n + kPsCluster - 1) / kPsCluster;
-    const int i1 = min(n, (rank + 1) * share);
-    for (int i = rank * share + threadIdx.x; i < i1; i += T) {
-        const double e = efield_at(F.phi, n, fc, ex0, i);
+    // E_x on the finest grid (EMFieldSolver::GetEfield)
+    ex0 = s_ex0;
+    auto phi = [&](int p) {  // p0 - 2 <= p <= p1 + 1
+        if (p < p0) return s_halo[p - p0 + 2];
+        if (p >= p1) return s_halo[p - p1 + 2];
+        if (p == 0) return s_phi0;
+        const int l = p - 1 - g0;
+        return xs[(l % L) * stride + l / L];
+    };
+    if (rank > 0 && cnt == 0) return;
+    for (int i = p0 + tid; i < p1; i += NT) {
+        const double e = -fc * (8 * (phi(i + 1) - phi(i - 1)) - phi(i + 2) + phi(i - 2)) + ex0;
         F.efin[i] = e;
         if (P.f32) F.efin32[i] = (float)e;
     }
 }
 
-// Threads per block: segments of about 8 elements (a decaying pass then gathers three
+// Scan threads per block: segments of about 8 elements (a decaying pass then gathers three
 // carry terms), 32 to kPsMaxThreads threads.
 int scan_threads(int maxn) {
     const int m = maxn - 1;
@@ -254,8 +335,10 @@ size_t poisson_scan_smem(int maxn) {
 void launch_poisson_fast(const PoissonFastLaunch &L) {
     if (L.nruns == 0) return;
     const size_t smem = poisson_scan_smem(L.maxn);
+    PoissonFastLaunch P = L;
+    P.scan_threads = scan_threads(L.maxn);
     cudaFuncSetAttribute(k_poisson_scan, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    vx_launch(k_poisson_scan, L.nruns * kPsCluster, scan_threads(L.maxn), smem, L.stream, L);
+    vx_launch(k_poisson_scan, L.nruns * kPsCluster, std::max(P.assemble ? kPsMaxThreads : kPsMinThreads, P.scan_threads + 32), smem, L.stream, P);
 }
 
 }  // namespace vx

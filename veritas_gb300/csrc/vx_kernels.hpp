@@ -250,6 +250,11 @@ void launch_moments_poisson64(const PipeLaunch &K);
 // Y holds the m x 3 Woodbury columns (row-major), K the 3x3 capacitance factor.
 constexpr int kPsMaxThreads = 512, kPsCluster = 8;
 constexpr int kPsMaxSeg = 48;                                              // elements per thread
+// Sets whose cells are at most one per thread of a cluster: the solve assembles rho and J
+// itself (FP32 steps of 130 momenta: n = 1062 0.305 -> 0.294 ms, 4096 0.388 -> 0.369, 4096 in two
+// levels 0.490 -> 0.473); beyond, the chain through the patch tables is walked more than
+// once per thread and the wide launch is the faster (8192 in two levels 1.076 against 1.090 ms).
+constexpr int kPsAssembleMaxN = kPsMaxThreads * kPsCluster;
 constexpr int kPsMaxUnknowns = kPsMaxThreads * kPsCluster * kPsMaxSeg;     // n - 1 <= this
 struct PoissonFastDev {
     const double *Y;
@@ -264,6 +269,9 @@ struct PoissonFastLaunch {
     int nruns;
     int maxn;                  // largest n of the runs
     int f32;                   // also write the FP32 copy of E_x (precision-32 sets)
+    AsmLaunch A;               // assemble: rho and J are formed here, from the moments
+    int assemble;
+    int scan_threads;          // threads that own segments (set by the launcher)
     cudaStream_t stream;
 };
 void launch_poisson_fast(const PoissonFastLaunch &L);
