@@ -1281,19 +1281,19 @@ __global__ void k_mx_rhs(MaxwellLaunch L) {
     VX_PDL_WAIT();
     const int run = blockIdx.y;
     if (run >= L.nruns) return;
-    mx_rhs_cell(L, run, blockIdx.x * blockDim.x + threadIdx.x);
+    mx_rhs_cell(L, run, blockIdx.x * blockDim.x + threadIdx.x, blockIdx.z);
 }
 __global__ void k_mx_update(MaxwellLaunch L) {
     VX_PDL_WAIT();
     const int run = blockIdx.y;
     if (run >= L.nruns) return;
-    mx_update_cell(L, run, blockIdx.x * blockDim.x + threadIdx.x);
+    mx_update_cell(L, run, blockIdx.x * blockDim.x + threadIdx.x, blockIdx.z);
 }
 __global__ void k_mx_asq(MaxwellLaunch L) {
     VX_PDL_WAIT();
     const int run = blockIdx.y;
     if (run >= L.nruns) return;
-    mx_asq_cell(L, run, blockIdx.x * blockDim.x + threadIdx.x);
+    mx_asq_pair(L, run, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 void launch_maxwell(const MaxwellLaunch &L) {
@@ -1301,10 +1301,10 @@ void launch_maxwell(const MaxwellLaunch &L) {
         launch_maxwell32(L);
         return;
     }
-    dim3 g((L.maxnf + 255) / 256, L.nruns);
-    vx_launch(k_mx_rhs, g, 256, 0, L.stream, L);
-    vx_launch(k_mx_update, g, 256, 0, L.stream, L);
-    vx_launch(k_mx_asq, g, 256, 0, L.stream, L);
+    const dim3 g((L.maxnf + kMxThreads - 1) / kMxThreads, L.nruns, kMxFields);
+    vx_launch(k_mx_rhs, g, kMxThreads, 0, L.stream, L);
+    vx_launch(k_mx_update, g, kMxThreads, 0, L.stream, L);
+    vx_launch(k_mx_asq, dim3((2 * L.maxnf + kMxThreads - 1) / kMxThreads, L.nruns), kMxThreads, 0, L.stream, L);
 }
 
 // ---------------------------------------------------------------- CFL

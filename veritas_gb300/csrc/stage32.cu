@@ -205,7 +205,10 @@ __global__ void __launch_bounds__(kStageThreads, 5) k32_stage_fct(Stage32Launch 
     const MaxwellLaunch &X = L.mx;
     const long long mxn = (long long)X.nruns * X.maxnf;
     // p fluxes (Rectangle.cpp:1326-1394; E_x from the solve) | Maxwell right-hand side
-    for_cells(mxn, [&](long long e) { mx_rhs_cell(X, (int)(e / X.maxnf), (int)(e % X.maxnf)); });
+    for_cells(mxn * kMxFields, [&](long long e) {
+        const long long c = e / kMxFields;
+        mx_rhs_cell(X, (int)(c / X.maxnf), (int)(c % X.maxnf), (int)(e % kMxFields));
+    });
     for_warp_units(L.sync, F.nptiles, [&](int w) { pflux32(patches, F.ptiles[w], lane, F.fields, s, F.use_f0, F.strip_rows); });
     bar.sync();
     // coarse faces on coarse/fine interfaces, batch by batch
@@ -218,7 +221,10 @@ __global__ void __launch_bounds__(kStageThreads, 5) k32_stage_fct(Stage32Launch 
         ds_32(patches, t, tx, row, F.params32, s);
         f2_32(patches, t, tx, row, F.params32, s);
     });
-    for_cells(mxn, [&](long long e) { mx_update_cell(X, (int)(e / X.maxnf), (int)(e % X.maxnf)); });
+    for_cells(mxn * kMxFields, [&](long long e) {
+        const long long c = e / kMxFields;
+        mx_update_cell(X, (int)(c / X.maxnf), (int)(c % X.maxnf), (int)(e % kMxFields));
+    });
     bar.sync();
     // ghost cells of f2 (Mesh::PushData(2))
     for (int b = 0; b < L.nghost_b; b++) {
@@ -324,19 +330,19 @@ __global__ void k_mx_rhs32(MaxwellLaunch L) {
     VX_PDL_WAIT();
     const int run = blockIdx.y;
     if (run >= L.nruns) return;
-    mx_rhs_cell(L, run, blockIdx.x * blockDim.x + threadIdx.x);
+    mx_rhs_cell(L, run, blockIdx.x * blockDim.x + threadIdx.x, blockIdx.z);
 }
 __global__ void k_mx_update32(MaxwellLaunch L) {
     VX_PDL_WAIT();
     const int run = blockIdx.y;
     if (run >= L.nruns) return;
-    mx_update_cell(L, run, blockIdx.x * blockDim.x + threadIdx.x);
+    mx_update_cell(L, run, blockIdx.x * blockDim.x + threadIdx.x, blockIdx.z);
 }
 __global__ void k_mx_asq32(MaxwellLaunch L) {
     VX_PDL_WAIT();
     const int run = blockIdx.y;
     if (run >= L.nruns) return;
-    mx_asq_cell(L, run, blockIdx.x * blockDim.x + threadIdx.x);
+    mx_asq_pair(L, run, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 void launch_ghost32(const void *patches, const GhostOp *ops, int n, const GhostOp *rows, int nrows, int slot,
@@ -355,10 +361,10 @@ void launch_assemble32(const AsmLaunch &A) {
     vx_launch(k_assemble32, g, 256, 0, A.stream, A);
 }
 void launch_maxwell32(const MaxwellLaunch &L) {
-    dim3 g((L.maxnf + 255) / 256, L.nruns);
-    vx_launch(k_mx_rhs32, g, 256, 0, L.stream, L);
-    vx_launch(k_mx_update32, g, 256, 0, L.stream, L);
-    vx_launch(k_mx_asq32, g, 256, 0, L.stream, L);
+    const dim3 g((L.maxnf + kMxThreads - 1) / kMxThreads, L.nruns, kMxFields);
+    vx_launch(k_mx_rhs32, g, kMxThreads, 0, L.stream, L);
+    vx_launch(k_mx_update32, g, kMxThreads, 0, L.stream, L);
+    vx_launch(k_mx_asq32, dim3((2 * L.maxnf + kMxThreads - 1) / kMxThreads, L.nruns), kMxThreads, 0, L.stream, L);
 }
 
 }  // namespace vx

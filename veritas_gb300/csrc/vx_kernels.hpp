@@ -286,7 +286,7 @@ struct MaxwellLaunch {
     int step;
     const double *params;  // per-run stage parameter blocks
     const double *dxinv;   // per run: 1/dx0
-    int f32;               // precision-32 sets: also the FP32 per-cell A^2 (k_mx_update)
+    int f32;               // precision-32 sets: also the FP32 per-cell A^2 (with a^2 on the faces)
     int asq32_out = 0;     // the face a^2 step also writes the FP32 copy of a^2 (persistent form:
                            // nothing reads that copy between this step and the next stage)
     cudaStream_t stream;
