@@ -278,61 +278,73 @@ __device__ __forceinline__ int mom_windows(int np) { return (np + kMomOut - 1) /
 // Per unit and window: a bound F >= |f| for each column over the window's cells and the
 // column's stencil, as the high word of a double (0: the column's contributions are all
 // zero), and in word kMomCols whether the window is formed.  One block per unit, a warp per
-// row of f: reads f once (4 rows of halo with the sub-cell interpolation), 22 MB and 10 us
-// on the 4096 x 512 two-level workload.
-__global__ void __launch_bounds__(256) k64_mom_screen(MomLaunch M) {
+// row of f: reads f once (4 rows of halo with the sub-cell interpolation).  Loads of
+// kScreenWin windows are in flight together: 22 MB of the 4096 x 512 two-level workload
+// took 48 us with eight warps that waited for each window, 16 us now.
+constexpr int kScreenRows = kMomCols + 4, kScreenWin = 6;
+__global__ void __launch_bounds__(kScreenRows * 32) k64_mom_screen(MomLaunch M) {
     VX_PDL_WAIT();
     extern __shared__ unsigned s_bound[];  // [row][window], bit 31 on a column's own row: none of its cells count
     __shared__ unsigned s_max[kMomCols];   // per column: largest |f| of the cells that count
     __shared__ int s_field[kMomCols];
     const unsigned full = 0xffffffffu;
-    const int col0 = blockIdx.x * kMomCols, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int col0 = blockIdx.x * kMomCols, lane = threadIdx.x & 31, r = threadIdx.x >> 5;
     const P64 &P = ((const P64 *)M.patches)[M.colpatch[col0]];
     const int np = P.np, rtb = P.rtb, nwin = mom_windows(np), halo = rtb > 1 ? 2 : 0;
-    int ncol = 0;  // real columns: consecutive i, the padding at the end
-    while (ncol < kMomCols && M.colpatch[col0 + ncol] >= 0) ncol++;
+    // real columns: consecutive i, the padding at the end
+    const int ncol = __popc(__ballot_sync(full, lane < kMomCols && M.colpatch[col0 + min(lane, kMomCols - 1)] >= 0));
     const int i0 = M.colidx[col0] / rtb;
-    for (int r = wid; r < ncol + 2 * halo; r += 8) {
+    if (r < ncol + 2 * halo) {
         const int i = i0 - halo + r;
-        const bool own = r >= halo && r < halo + ncol;
+        const bool own = r >= halo && r < halo + ncol, nest = own && P.nested;
+        const double *f = P.f1 + pidx(i, 0, P.pitch);
+        const uint8_t *nested = nest ? P.nested + pidx(i, 0, P.pitch) : nullptr;
         unsigned top = 0;
-        for (int w = 0; w < nwin; w++) {
-            const int j = kMomOut * w - 1 + lane;
-            const double v = j <= np ? P.f1[pidx(i, j, P.pitch)] : 0.0;
-            const unsigned h = (unsigned)__double2hiint(v) & 0x7fffffffu;
-            const unsigned e = (h | (unsigned)__double2loint(v)) ? min(h + 1u, 0x7fffffffu) : 0u;
-            unsigned m = __reduce_max_sync(full, e);
-            if (own && P.nested) {
-                const bool counts = lane >= 1 && lane <= kMomOut && j < np && !P.nested[pidx(i, j, P.pitch)];
-                top = max(top, __reduce_max_sync(full, counts ? e : 0u));
-                if (!__any_sync(full, counts)) m |= 0x80000000u;
-            } else {
-                top = max(top, m);
+        for (int w0 = 0; w0 < nwin; w0 += kScreenWin) {
+            double v[kScreenWin];
+            bool counts[kScreenWin];
+#pragma unroll
+            for (int k = 0; k < kScreenWin; k++) {
+                const int j = kMomOut * (w0 + k) - 1 + lane;
+                v[k] = j <= np ? f[j] : 0.0;  // windows past the last: nothing
+                counts[k] = nest && lane >= 1 && lane <= kMomOut && j < np && !nested[j];
             }
-            if (lane == 0) s_bound[r * nwin + w] = m;
+#pragma unroll
+            for (int k = 0; k < kScreenWin; k++) {
+                const unsigned h = (unsigned)__double2hiint(v[k]) & 0x7fffffffu;
+                const unsigned e = (h | (unsigned)__double2loint(v[k])) ? min(h + 1u, 0x7fffffffu) : 0u;
+                unsigned m = __reduce_max_sync(full, e);
+                if (nest) {
+                    top = max(top, __reduce_max_sync(full, counts[k] ? e : 0u));
+                    if (!__any_sync(full, counts[k])) m |= 0x80000000u;
+                } else {
+                    top = max(top, m);
+                }
+                if (lane == 0 && w0 + k < nwin) s_bound[r * nwin + w0 + k] = m;
+            }
         }
         if (own && lane == 0) s_max[r - halo] = top;
     }
-    __syncthreads();
-    for (int c = threadIdx.x; c < ncol; c += 256) {
+    if (threadIdx.x < ncol) {
         bool fin = true;  // a field that is not finite makes every cell's current so
-        for (int k = 0; k < rtb; k++) fin = fin && isfinite(cell_asq(M.fields[P.run], (i0 + c + P.x_pos) * rtb + k));
-        s_field[c] = fin;
+        for (int k = 0; k < rtb; k++)
+            fin = fin && isfinite(cell_asq(M.fields[P.run], (i0 + (int)threadIdx.x + P.x_pos) * rtb + k));
+        s_field[threadIdx.x] = fin;
     }
     __syncthreads();
     constexpr unsigned kFar = 96u << 20;  // 2^96 in the exponent of a high word
     unsigned *out = M.screen + (size_t)blockIdx.x * M.maxnwin * kMomScreen;
-    for (int w = threadIdx.x; w < nwin; w += 256) {
-        unsigned form = 0;
-        for (int c = 0; c < kMomCols; c++) {
-            unsigned b = 0;
-            if (c < ncol && !(s_bound[(c + halo) * nwin + w] & 0x80000000u)) {
-                for (int r = c; r <= c + 2 * halo; r++) b = max(b, s_bound[r * nwin + w] & 0x7fffffffu);
-                if (!s_field[c] || (b && !(s_max[c] < 0x7ff00000u && b + kFar <= s_max[c]))) form = 1;
-            }
-            out[w * kMomScreen + c] = b;
+    // sixteen lanes per window: a column each
+    for (int w0 = 2 * r; w0 < nwin; w0 += 2 * kScreenRows) {
+        const int w = w0 + (lane >> 4), c = lane & 15;
+        unsigned b = 0;
+        bool form = false;
+        if (w < nwin && c < ncol && !(s_bound[(c + halo) * nwin + w] & 0x80000000u)) {
+            for (int q = c; q <= c + 2 * halo; q++) b = max(b, s_bound[q * nwin + w] & 0x7fffffffu);
+            form = !s_field[c] || (b && !(s_max[c] < 0x7ff00000u && b + kFar <= s_max[c]));
         }
-        out[w * kMomScreen + kMomCols] = form;
+        const unsigned any = __ballot_sync(full, form) & (0xffffu << (lane & 16));
+        if (w < nwin) out[w * kMomScreen + c] = c < kMomCols ? b : any != 0;
     }
 }
 
@@ -346,7 +358,7 @@ void launch_mom_screen64(const MomLaunch &M) {
     if (smem > 48 * 1024) cudaFuncSetAttribute(k64_mom_screen, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(M.ncols / kMomCols);
-    cfg.blockDim = dim3(256);
+    cfg.blockDim = dim3(kScreenRows * 32);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = M.stream;
     cudaLaunchAttribute attr[2];
@@ -883,6 +895,8 @@ __device__ __forceinline__ void poisson_solve(const PoissonLaunch &L, unsigned c
     double *tmp = F.efin;  // scratch until E_x is recomputed at the end
     const double te = kEps0Inv;
     const double w = L.w[run];
+    const bool fwd_chunks = PIPE || lu.L.nslots >= 0;
+    if (fwd_chunks) pois_stage_fwd(buf[0].f, lu.L, 0, kPoisBuf, n, threadIdx.x, blockDim.x);  // needs no moments
     if (PIPE) {
         pipe_rows(*K, run, 0, x, threadIdx.x, blockDim.x, 0, false);  // chunk 0's rows, all threads
     } else {
@@ -902,13 +916,12 @@ __device__ __forceinline__ void poisson_solve(const PoissonLaunch &L, unsigned c
     if (PIPE && K->trace && run == 0 && threadIdx.x == 0) K->trace[1 + 2 * K->trace_nch] = clock64();
     const int lane = threadIdx.x & 31;
     // ---- forward: rows ascending; chunk c stages rows [c*R, c*R + R + LA)
-    if (!PIPE && lu.L.nslots < 0) {
+    if (!fwd_chunks) {
         __syncthreads();
         if (threadIdx.x == 0) pois_rows_plain<false>(lu.L, 0, n, n, x, true);
         __syncthreads();
     } else {
         double V = 0.0, w1 = 0.0;
-        pois_stage_fwd(buf[0].f, lu.L, 0, kPoisBuf, n, threadIdx.x, blockDim.x);
         __syncthreads();
         if (threadIdx.x < 32 && lane < 4 && lane < n) V = pois_far(lu.L, x, lane);
         // warp 0 sweeps, the others stage the next chunk (pipelined: and gather its rows):
