@@ -78,8 +78,8 @@ __device__ __forceinline__ double cell_asq(const RunFields &F, int x) {
     return (ay * ay) + (az * az);
 }
 
-// One warp per coarse column i, kMomCols columns of one patch per block; a warp forms
-// its column's finest sub-columns k in pairs, the f stencil and the interpolation's
+// One warp per coarse column i, a unit's kMomCols columns of one patch (or a third of them)
+// per block; a warp forms its column's finest sub-columns k in pairs, the f stencil and the interpolation's
 // shared part once per cell for the pair.  The warp walks p in windows of 32 lanes
 // covering j0-1 .. j0+30: every lane computes the Lorentz factor at its p-face once
 // (shared with the neighbouring face through shuffles instead of the reference's four
@@ -97,19 +97,14 @@ __device__ __forceinline__ double cell_asq(const RunFields &F, int x) {
 // The coarse-column list is padded per patch to a multiple of kMomCols (padding: patch
 // -1), so the warps of a block share n_p and rtb and step through the windows together.
 constexpr int kMomOut = kMomWindow;  // outputs per window: j0 .. j0+28
-constexpr int kMomThreads = (kMomCols + 1) * 32;
+constexpr int kMomSmallPart = 5;     // columns per block of k64_moments for small sets
 
 // Two window buffers: the column warps fill one while the summing warp adds the other.
+template <int PART>
 struct MomSmem {
-    double cc[2][kMomCols][2][32], cj[2][kMomCols][2][32];
+    double cc[2][PART][2][32], cj[2][PART][2][32];
     int redo;
 };
-
-// Barrier of one moment unit's kMomThreads threads: barrier 0 in k64_moments (the whole
-// block), named barriers 1 and 2 for the two units a pipelined block carries.
-__device__ __forceinline__ void mom_sync(int bar) {
-    asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(kMomThreads) : "memory");
-}
 
 // One window of column i's sub-columns k0 .. k0+kg-1 (kg <= 2): lane L covers the p index
 // j = j0 - 1 + L; lanes 1 .. kMomOut return the charge and current contributions cc[q],
@@ -253,12 +248,13 @@ struct MomLane {
     bool on, two, cur;
     int w, q;
     double f0, f1;  // bounds of one contribution over F
-    __device__ __forceinline__ MomLane(const P64 &P, int kg, int lane) {
-        on = lane < 2 * kMomCols;
+    // of the unit's columns c0 .. c0 + nc - 1 alone
+    __device__ __forceinline__ MomLane(const P64 &P, int kg, int lane, int c0 = 0, int nc = kMomCols) {
         two = kg == 2;
-        cur = !two && lane >= kMomCols;
-        w = two ? lane >> 1 : (cur ? lane - kMomCols : lane);
-        if (!on) w = 0;
+        cur = !two && lane >= nc;
+        w = c0 + (two ? lane >> 1 : (cur ? lane - nc : lane));
+        on = lane < 2 * nc;
+        if (!on) w = c0;
         q = two ? lane & 1 : 0;
         const double c = P.rtb > 1 ? 8.0 : 1.0, j = (P.rtb > 1 ? 10.0 : 1.25) * P.dp;
         f0 = on ? (cur ? j : c) : 0.0;
@@ -371,16 +367,28 @@ void launch_mom_screen64(const MomLaunch &M) {
     cudaLaunchKernelEx(&cfg, k64_mom_screen, M);  // errors surface through cudaGetLastError
 }
 
-// One unit: the kMomCols columns of unit `unit` of the padded column list, formed by warps
-// 0 .. kMomCols - 1 and summed by warp kMomCols (wid: warp within the unit).
-template <bool FAST>
-__device__ __forceinline__ void moments_unit(const MomLaunch &M, int unit, int wid, int lane, MomSmem &S, int bar) {
+// One part of a unit: PART of the kMomCols columns of a unit of the padded column list, from
+// c0, formed by a warp each and summed by warp PART.  A block of all fifteen keeps every
+// FP64 unit of its SM in four warps' hands; where there are not enough units for every SM
+// (a set of at most two per SM), three blocks of five spread a unit over three SMs: 50 x 38
+// 63 -> 44 us, 2048 x 256 74 -> 61 us with the screen, but 6.65 -> 6.71 ms per step for the
+// 657 units of 4096 x 512 in two levels (the summing warps do the same for fewer columns).
+template <bool FAST, int PART>
+__global__ void __launch_bounds__((PART + 1) * 32, PART == kMomCols ? 2 : 5) k64_moments(MomLaunch M) {
+    VX_PDL_WAIT();
+    constexpr int kParts = kMomCols / PART, nc = PART;
+    static_assert(kMomCols % PART == 0, "parts of equal size");
+    __shared__ MomSmem<PART> S;
+    const int unit = blockIdx.x / kParts, c0 = (blockIdx.x % kParts) * PART;
+    const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int col0 = unit * kMomCols;
-    const bool summer = wid == kMomCols;  // the last warp adds; warps 0..kMomCols-1 form columns
-    const bool real = !summer && M.colpatch[col0 + wid] >= 0;  // warp-uniform
+    if (M.colpatch[col0 + c0] < 0) return;  // padding alone
+    const bool summer = wid == PART;
+    const int col = col0 + c0 + wid;
+    const bool real = !summer && M.colpatch[col] >= 0;  // warp-uniform
     const P64 &P = ((const P64 *)M.patches)[M.colpatch[col0]];  // the unit's patch
     const int rtb = P.rtb, nwin = mom_windows(P.np);
-    const int i = summer ? 0 : M.colidx[col0 + wid] / rtb;
+    const int i = real ? M.colidx[col] / rtb : 0;
     const RunFields &F = M.fields[P.run];
     const unsigned *screen = M.screen + (size_t)unit * M.maxnwin * kMomScreen;
     const double minv = 1 / P.mass;
@@ -393,7 +401,7 @@ __device__ __forceinline__ void moments_unit(const MomLaunch &M, int unit, int w
         double a[2] = {0.0, 0.0};
         for (int q = 0; q < kg; q++)
             if (real) a[q] = P.qq * cell_asq(F, (i + P.x_pos) * rtb + k0 + q);
-        const MomLane ml(P, kg, lane);
+        const MomLane ml(P, kg, lane, c0, nc);
         for (int pass = 0; pass < 2; pass++) {  // pass 1: every window, where pass 0 did not settle
             MomSum s;
             bool both = false;
@@ -407,7 +415,8 @@ __device__ __forceinline__ void moments_unit(const MomLaunch &M, int unit, int w
                 }
                 if (w == nwin) return;
                 both = __any_sync(full, s.split());
-                const double *pc = ml.cur ? S.cj[bf][ml.w][0] : S.cc[bf][ml.w][ml.q], *pj = S.cj[bf][ml.w][ml.q];
+                const int k = ml.w - c0;
+                const double *pc = ml.cur ? S.cj[bf][k][0] : S.cc[bf][k][ml.q], *pj = S.cj[bf][k][ml.q];
                 s.add(both, ml.two, [&](int t) { return pc[t]; }, [&](int t) { return pj[t]; });
                 next = w + 1;
             };
@@ -427,7 +436,7 @@ __device__ __forceinline__ void moments_unit(const MomLaunch &M, int unit, int w
                 }
                 prev = w;
                 bf ^= 1;
-                mom_sync(bar);
+                __syncthreads();
             }
             if (summer) {
                 if (prev >= 0) add_to(prev, bf ^ 1);
@@ -436,26 +445,27 @@ __device__ __forceinline__ void moments_unit(const MomLaunch &M, int unit, int w
                 if (lane == 0) S.redo = redo;
                 if (!redo) ml.store(M, P, col0, k0, s);
             }
-            mom_sync(bar);  // the next pair's first window reuses the buffers
+            __syncthreads();  // the next pair's first window reuses the buffers
             if (!S.redo) break;
-            mom_sync(bar);
+            __syncthreads();
         }
     }
-}
-
-template <bool FAST>
-__global__ void __launch_bounds__(kMomThreads, 2) k64_moments(MomLaunch M) {
-    VX_PDL_WAIT();
-    __shared__ MomSmem S;
-    moments_unit<FAST>(M, blockIdx.x, threadIdx.x >> 5, threadIdx.x & 31, S, 0);
 }
 
 void launch_moments64(const MomLaunch &M) {
     if (M.ncols == 0) return;
     launch_mom_screen64(M);
-    // M.ncols is a multiple of kMomCols (the list is padded per patch)
-    if (M.fast) vx_launch(k64_moments<true>, M.ncols / kMomCols, kMomThreads, 0, M.stream, M);
-    else vx_launch(k64_moments<false>, M.ncols / kMomCols, kMomThreads, 0, M.stream, M);
+    const int units = M.ncols / kMomCols;  // the list is padded per patch
+    int sms = 0, dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (units <= 2 * sms) {
+        auto kern = M.fast ? k64_moments<true, kMomSmallPart> : k64_moments<false, kMomSmallPart>;
+        vx_launch(kern, units * (kMomCols / kMomSmallPart), (kMomSmallPart + 1) * 32, 0, M.stream, M);
+    } else {
+        auto kern = M.fast ? k64_moments<true, kMomCols> : k64_moments<false, kMomCols>;
+        vx_launch(kern, units, (kMomCols + 1) * 32, 0, M.stream, M);
+    }
 }
 
 // ---------------------------------------------------------------- separable initial f
