@@ -19,7 +19,6 @@
 #include <cuda_runtime.h>
 #include "amr.hpp"
 #include "div64.cuh"
-#include "fast64.cuh"
 #include "vx_kernels.hpp"
 
 #ifdef VX_FP64_FAST
@@ -94,14 +93,21 @@ __device__ __forceinline__ void weno_values(double f1, double f2, double f3, dou
     double BL = f3 - f1;
     double AR = f2 - 2 * f3 + f4;
     double BR = f4 - f2;
+#ifdef VX_FP64_FAST
+    // with t = B / 2 the indicator is A (c43 A +- t) + t^2: four operations instead of six
+    const double tL = 0.5 * BL, tR = 0.5 * BR;
+    const double bL = __fma_rn(tL, tL, AL * __fma_rn(c43, AL, tL));
+    const double bR = __fma_rn(tR, tR, AR * __fma_rn(c43, AR, -tR));
+#else
     double bL = c43 * (AL * AL) + 0.5 * AL * BL + 0.25 * (BL * BL);
     double bR = c43 * (AR * AR) - 0.5 * AR * BR + 0.25 * (BR * BR);
+#endif
     const double mm = 1.0e-10;
     const double dL = mm + bL, dR = mm + bR;
     double wL, wR;
 #ifdef VX_FP64_FAST
     // oL / (oL + oR) with o = 0.5 / (mm + b)^2 is dR^2 / (dL^2 + dR^2)
-    wL = (dR * dR) * rcp_nr(dL * dL + dR * dR);
+    wL = (dR * dR) * rcp_ulp(dL * dL + dR * dR);
     wR = 1.0 - wL;
     constexpr bool plain = true;
 #else
@@ -123,7 +129,7 @@ __device__ __forceinline__ void weno_values(double f1, double f2, double f3, dou
     const double pr = wgt(wL0, wR0) ? wL0 : wR0, pl = wgt(wR0, wL0) ? wL0 : wR0;
     const double sw = wL0 + wR0;
 #ifdef VX_FP64_FAST
-    const double inv = rcp_nr(sw);
+    const double inv = rcp_ulp(sw);
     auto quot = [&](double a) { return a * inv; };
 #else
     // the mapped weights sum to 0.75 .. 1.25, each 0 .. 1.25: below 1e-250 (a weight of a

@@ -9,7 +9,6 @@
 #include <cuda_runtime.h>
 #include <algorithm>
 #include "div64.cuh"
-#include "fast64.cuh"
 #include "field_ops.cuh"
 #include "vx_kernels.hpp"
 
