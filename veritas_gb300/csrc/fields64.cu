@@ -10,6 +10,7 @@
 #include <algorithm>
 #include "div64.cuh"
 #include "field_ops.cuh"
+#include "poisson_lu.hpp"
 #include "vx_kernels.hpp"
 
 namespace vx {
@@ -639,11 +640,9 @@ __device__ __noinline__ void pois_rows_plain(const BandFactor &F, int lo, int hi
     }
 }
 
-// Stage the chunk of rows [r0, r1) of the upper factor and subtract the rows' far terms
-// (their solution values are known): threads t of nt; those with t2 >= 0 (of nt2) do the
-// FP64 work.
-__device__ void pois_stage_bwd(PoisBwdChunk &B, const BandFactor &F, int r0, int r1, double *x, int t, int nt, int t2,
-                               int nt2) {
+// Stage the factors of rows [r0, r1) of the upper factor (they need no solution value):
+// threads t of nt.
+__device__ void pois_stage_bwd(PoisBwdChunk &B, const BandFactor &F, int r0, int r1, int t, int nt) {
     const int base = r0 - kPoisLA, rows = r1 - base;
     for (int k = t; k < rows; k += nt) {
         double v[kBwdCols] = {0.0, 0.0, 0.0, 0.0, 0.0};
@@ -656,12 +655,51 @@ __device__ void pois_stage_bwd(PoisBwdChunk &B, const BandFactor &F, int r0, int
         if (k >= kPoisLA) B.diag[k - kPoisLA] = F.diag[base + k];
     }
     if (t == 0) B.c[3][0] = make_double2(0.0, 1.0);
-    if (t2 >= 0)
-        for (int k = t2; k < r1 - r0; k += nt2) {
-            const double v = pois_far(F, x, r0 + k);
-            x[r0 + k] = v;
-            B.rhs[k] = v;
-        }
+}
+// Their right-hand sides with the far terms subtracted (the solution values of the last
+// rows, which are known): threads t of nt, t < 0 takes no part.
+__device__ void pois_rhs_bwd(PoisBwdChunk &B, const BandFactor &F, int r0, int r1, double *x, int t, int nt) {
+    if (t < 0) return;
+    for (int k = t; k < r1 - r0; k += nt) {
+        const double v = pois_far(F, x, r0 + k);
+        x[r0 + k] = v;
+        B.rhs[k] = v;
+    }
+}
+
+// The last rows of the upper factor, where its far columns lie: the triangle in dense form.
+constexpr int kPoisTail = PoissonLU::Band::kTail;
+struct PoisTail {
+    double u[kPoisTail][kPoisTail], diag[kPoisTail], y[kPoisTail];  // y: rounded 1 / diag
+};
+__device__ void pois_stage_tail(PoisTail &T, const BandFactor &F, int t0, int t) {
+    if (t >= kPoisTail) return;
+    const int i = t0 + t;
+    for (int c = 0; c < kPoisTail; c++) T.u[t][c] = 0.0;
+    for (int d = 1; d <= 4 && t + d < kPoisTail; d++) T.u[t][t + d] = F.band[4 * i + d - 1];
+    for (int e = F.fptr[i]; e < F.fptr[i + 1]; e++) T.u[t][F.fcol[e] - t0] = F.fval[e];
+    T.diag[t] = F.diag[i];
+    T.y[t] = F.sweep[(size_t)i * kBwdCols + 3];
+}
+// Solved by warp 0, a row per lane: column by column from the last, which subtracts every
+// row's terms in descending column order as dgetrs does (a zero where the factor has no
+// entry changes nothing).  One thread with its operands in global memory took 8 us.
+__device__ void pois_tail(const PoisTail &T, int t0, double *x) {
+    constexpr unsigned act = (1u << kPoisTail) - 1;
+    const int l = threadIdx.x & 31;
+    if (l >= kPoisTail) return;
+    double s = x[t0 + l], mine = 0.0;
+    const double diag = T.diag[l], y = T.y[l];
+    for (int c = kPoisTail - 1; c >= 0; c--) {
+        const double u = T.u[l][c];
+        // the rounding of s / diag, in short where s is in range (the diagonal is of order one)
+        const unsigned h = ((unsigned)__double2hiint(s) & 0x7fffffffu) - 0x16800000u;
+        const double q = h < 0x52800000u ? div_rn(s, diag, y) : s / diag;
+        const double xc = __shfl_sync(act, q, c);
+        if (l == c) mine = q;
+        s = s - xc * u;
+    }
+    x[t0 + l] = mine;
 }
 
 // Forward sweep of one chunk, software-pipelined on lanes 0..7 of warp 0.  Row i's sum is
@@ -712,7 +750,7 @@ __device__ void pois_fwd_fast(const PoisFwdChunk &B, const BandFactor &F, int r0
         const int i = r0 + q;
         // row q+1's operands; a slot's row r >= step + 4 and the right-hand side x[i + 5]
         // are not yet overwritten by the sweep.  Rows past the chunk read the staged
-        // look-ahead rows, or past n the neutral entries pois_stage_band leaves there.
+        // look-ahead rows, or past n the neutral entries pois_stage_fwd leaves there.
         double coef_n = *cp;
         cp += cstep;
         if (q + 1 > lim || !has_coef) coef_n = 0.0;
@@ -896,6 +934,7 @@ __device__ __forceinline__ void poisson_solve(const PoissonLaunch &L, unsigned c
                                               const PipeLaunch *K) {
     PoisChunk *buf = (PoisChunk *)smem_raw;  // two chunk buffers, then the solution vector
     __shared__ int s_bad;
+    __shared__ PoisTail s_tail;
     const int run = blockIdx.x;
     RunFields &F = L.fields[run];
     const LUDev &lu = L.lu[run];
@@ -925,9 +964,15 @@ __device__ __forceinline__ void poisson_solve(const PoissonLaunch &L, unsigned c
     if (PIPE && K->trace && run == 0 && threadIdx.x == 0) K->trace[1 + 2 * K->trace_nch] = clock64();
     const int lane = threadIdx.x & 31;
     // ---- forward: rows ascending; chunk c stages rows [c*R, c*R + R + LA)
+    const int t0 = lu.U.sweep ? lu.U.far_pre_col : 0;
+    const bool tail = t0 > 0;
     if (!fwd_chunks) {
         __syncthreads();
         if (threadIdx.x == 0) pois_rows_plain<false>(lu.L, 0, n, n, x, true);
+        if (tail) {
+            pois_stage_tail(s_tail, lu.U, t0, threadIdx.x);
+            pois_stage_bwd(buf[nchunks & 1].b, lu.U, max(t0 - kPoisRows, 0), t0, threadIdx.x, blockDim.x);
+        }
         __syncthreads();
     } else {
         double V = 0.0, w1 = 0.0;
@@ -952,37 +997,31 @@ __device__ __forceinline__ void poisson_solve(const PoissonLaunch &L, unsigned c
                 if (PIPE) pipe_rows(*K, run, c + 1, x, threadIdx.x - 32, blockDim.x - 32, 1, true);
                 __syncthreads();
             }
+            if (tail) {  // beside the last chunk: what the backward sweep starts from
+                pois_stage_tail(s_tail, lu.U, t0, threadIdx.x - 32);
+                pois_stage_bwd(buf[nchunks & 1].b, lu.U, max(t0 - kPoisRows, 0), t0, threadIdx.x - 32, blockDim.x - 32);
+            }
             __syncthreads();  // the last chunk's
         }
     }
     if (PIPE && K->trace && run == 0 && threadIdx.x == 0) K->trace[2 + 2 * K->trace_nch] = clock64();
-    // ---- backward: the last rows (all of them if their far columns reach further down)
-    // one by one, then chunks of R rows, descending
+    // ---- backward: the last rows (all of them, one by one, if their far columns reach
+    // further down), then chunks of R rows, descending
     {
-        const int t0 = lu.U.sweep ? lu.U.far_pre_col : 0;
-        if (threadIdx.x == 0) {
-            pois_rows_plain<true>(lu.U, t0, n, n, x, true);
-            s_bad = 0;
-        }
+        if (!tail && threadIdx.x == 0) pois_rows_plain<true>(lu.U, 0, n, n, x, true);
+        if (tail && threadIdx.x < 32) pois_tail(s_tail, t0, x);
+        if (threadIdx.x == 0) s_bad = 0;
         __syncthreads();
         const int nbwd = (t0 + kPoisRows - 1) / kPoisRows;
-        // FP64 work of the staging warps stays off warp 0's sub-partition (warps 4m)
-        const int wg = (int)threadIdx.x >> 5;
-        const int t2 = (wg & 3) == 0 ? -1 : ((wg >> 2) * 3 + (wg & 3) - 1) * 32 + lane;
-        const int nt2 = ((int)blockDim.x >> 7) * 3 * 32;
-        if (nbwd > 0)
-            pois_stage_bwd(buf[0].b, lu.U, max(t0 - kPoisRows, 0), t0, x, threadIdx.x, blockDim.x, t2, nt2);
-        __syncthreads();
-        for (int c = 0; c < nbwd; c++) {
-            const int r1 = t0 - c * kPoisRows, r0 = max(r1 - kPoisRows, 0), cnt = r1 - r0;
-            PoisBwdChunk &B = buf[c & 1].b;
-            if (threadIdx.x < 32) pois_bwd_fast(B, r0, cnt, x);
-            else if (r0 > 0)
-                pois_stage_bwd(buf[(c + 1) & 1].b, lu.U, max(r0 - kPoisRows, 0), r0, x, threadIdx.x - 32,
-                               blockDim.x - 32, t2, nt2);
-            __syncthreads();
-            // every row of the chunk with IEEE division, from the rows above it
-            for (int q = threadIdx.x; q < cnt; q += blockDim.x) {
+        // chunk c's rows and buffer; the first chunk's factors are staged already
+        auto first = [&](int c) { return max(t0 - (c + 1) * kPoisRows, 0); };
+        auto rows = [&](int c) { return t0 - c * kPoisRows - first(c); };
+        auto buffer = [&](int c) -> PoisBwdChunk & { return buf[(c + nchunks) & 1].b; };
+        // every row of a swept chunk with IEEE division, from the rows above it
+        auto check = [&](int c, int t, int nt) {
+            const PoisBwdChunk &B = buffer(c);
+            const int r0 = first(c), cnt = rows(c);
+            for (int q = t; q < cnt; q += nt) {
                 const double *xr = x + r0 + q;
                 const int e = q + kPoisLA;
                 double s = B.rhs[q] - xr[3] * B.c[2][e].x;
@@ -990,17 +1029,58 @@ __device__ __forceinline__ void poisson_solve(const PoissonLaunch &L, unsigned c
                 s = s - xr[1] * B.c[0][e].x;
                 if (__double_as_longlong(s / B.diag[q]) != __double_as_longlong(xr[0])) s_bad = 1;
             }
+        };
+        // chunk c in IEEE division, row by row
+        auto redo = [&](int c) {
+            const PoisBwdChunk &B = buffer(c);
+            const int r0 = first(c), cnt = rows(c);
+            for (int q = threadIdx.x; q < cnt; q += blockDim.x) x[r0 + q] = B.rhs[q];
             __syncthreads();
-            if (s_bad) {  // uniform: redone in IEEE division (the next chunk's sweep reads x alone)
-                for (int q = threadIdx.x; q < cnt; q += blockDim.x) x[r0 + q] = B.rhs[q];
-                __syncthreads();
-                if (threadIdx.x == 0) {
-                    pois_rows_plain<true>(lu.U, r0, r1, n, x, false);
-                    s_bad = 0;
+            if (threadIdx.x == 0) {
+                pois_rows_plain<true>(lu.U, r0, r0 + cnt, n, x, false);
+                s_bad = 0;
+            }
+            __syncthreads();
+        };
+        // FP64 work of the other warps stays off warp 0's sub-partition (warps 4m)
+        const int wg = (int)threadIdx.x >> 5, others = (int)blockDim.x - 32;
+        const int t2 = (wg & 3) == 0 ? -1 : ((wg >> 2) * 3 + (wg & 3) - 1) * 32 + lane;
+        const int nt2 = ((int)blockDim.x >> 7) * 3 * 32;
+        if (nbwd > 0) pois_rhs_bwd(buffer(0), lu.U, first(0), first(0) + rows(0), x, t2, nt2);
+        __syncthreads();
+        // While warp 0 sweeps chunk c, the others check chunk c - 1 and then, in the buffer that
+        // leaves, stage chunk c + 1 (the check between the sweeps took 1.2 us of a chunk's 34).
+        // A chunk that fails is redone, and the sweep of the next one, which began from it.
+        int settled = -1;  // the last chunk done in IEEE division: not checked again
+        for (int c = 0; c < nbwd; c++) {
+            if (threadIdx.x < 32) {
+                pois_bwd_fast(buffer(c), first(c), rows(c), x);
+            } else {
+                if (c > 0 && c - 1 != settled && t2 >= 0) check(c - 1, t2, nt2);
+                pipe_bar(1, others);
+                if (c + 1 < nbwd && !s_bad) {
+                    pois_stage_bwd(buffer(c + 1), lu.U, first(c + 1), first(c), threadIdx.x - 32, others);
+                    pois_rhs_bwd(buffer(c + 1), lu.U, first(c + 1), first(c), x, t2, nt2);
                 }
+            }
+            __syncthreads();
+            if (s_bad) {  // uniform
                 __syncthreads();
+                redo(c - 1);
+                for (int q = threadIdx.x; q < rows(c); q += blockDim.x) x[first(c) + q] = buffer(c).rhs[q];
+                __syncthreads();
+                settled = --c;
+                continue;
             }
             if (trace) trace[1 + nchunks + c] = tick();
+        }
+        if (nbwd > 0) {
+            check(nbwd - 1, threadIdx.x, blockDim.x);
+            __syncthreads();
+            if (s_bad) {
+                __syncthreads();
+                redo(nbwd - 1);
+            }
         }
         if (trace)
             for (int c = nbwd; c < nchunks; c++) trace[1 + nchunks + c] = tick();
