@@ -63,6 +63,20 @@ __device__ __forceinline__ bool wgt(double a, double b) {
     return __double_as_longlong(a) > __double_as_longlong(b);
 }
 
+// x / 2 and 2 x, exact, on the exponent field instead of the FP64 unit (its multiplication
+// where the field is near an end of its range and x is not zero).  With the products these
+// save, faces of 2.83 M cells 275 -> 262 us in x, 295 -> 282 us in p.
+__device__ __forceinline__ double half_of(double x) {
+    const unsigned h = (unsigned)__double2hiint(x), e = h & 0x7ff00000u;
+    if (e > 0x00100000u && e < 0x7ff00000u) return __hiloint2double((int)(h - 0x00100000u), __double2loint(x));
+    return (h << 1 | (unsigned)__double2loint(x)) == 0 ? x : 0.5 * x;
+}
+__device__ __forceinline__ double twice(double x) {
+    const unsigned h = (unsigned)__double2hiint(x), e = h & 0x7ff00000u;
+    if (e != 0 && e < 0x7fe00000u) return __hiloint2double((int)(h + 0x00100000u), __double2loint(x));
+    return (h << 1 | (unsigned)__double2loint(x)) == 0 ? x : 2 * x;
+}
+
 // WENO-type upwind face value (Rectangle.cpp:980-1030; identical values to
 // Rectangle.cpp:943-977).  f1..f4 are the four cells left-to-right around the face.  The
 // smoothness weights do not depend on the velocity, so both upwind choices come out of one
@@ -83,24 +97,31 @@ __device__ __forceinline__ void weno_values(double f1, double f2, double f3, dou
     }
     const double c6 = 1.0 / 6;
     const double c43 = 4.0 / 3;
-    double fL = c6 * (-f1 + 5 * f2 + 2 * f3);
-    double fR = c6 * (2 * f2 + 5 * f3 - f4);
+#ifdef VX_FP64_FAST  // fused into the sums
+    const double d2 = 2 * f2, d3 = 2 * f3;
+#else
+    const double d2 = twice(f2), d3 = twice(f3);
+#endif
+    double fL = c6 * (-f1 + 5 * f2 + d3);
+    double fR = c6 * (d2 + 5 * f3 - f4);
     if (none == 1) {
         out_right = out_left = 0.5 * fL + 0.5 * fR;
         return;
     }
-    double AL = f1 - 2 * f2 + f3;
+    double AL = f1 - d2 + f3;
     double BL = f3 - f1;
-    double AR = f2 - 2 * f3 + f4;
+    double AR = f2 - d3 + f4;
     double BR = f4 - f2;
+    // with t = B / 2, exact as is every product with a power of two, B^2 / 4 is t^2 and A B / 2
+    // is A t in the same rounding
+    const double tL = half_of(BL), tR = half_of(BR);
 #ifdef VX_FP64_FAST
-    // with t = B / 2 the indicator is A (c43 A +- t) + t^2: four operations instead of six
-    const double tL = 0.5 * BL, tR = 0.5 * BR;
+    // the indicator is A (c43 A +- t) + t^2
     const double bL = __fma_rn(tL, tL, AL * __fma_rn(c43, AL, tL));
     const double bR = __fma_rn(tR, tR, AR * __fma_rn(c43, AR, -tR));
 #else
-    double bL = c43 * (AL * AL) + 0.5 * AL * BL + 0.25 * (BL * BL);
-    double bR = c43 * (AR * AR) - 0.5 * AR * BR + 0.25 * (BR * BR);
+    double bL = c43 * (AL * AL) + AL * tL + tL * tL;
+    double bR = c43 * (AR * AR) - AR * tR + tR * tR;
 #endif
     const double mm = 1.0e-10;
     const double dL = mm + bL, dR = mm + bR;
@@ -114,7 +135,8 @@ __device__ __forceinline__ void weno_values(double f1, double f2, double f3, dou
     // within 1e-10 .. 1e95 every intermediate of the short quotients is a normal number
     const bool plain = (unsigned)__double2hiint(dL) < 0x53a00000u && (unsigned)__double2hiint(dR) < 0x53a00000u;
     if (plain) {
-        const double oL = 0.5 * rcp_rn(dL * dL), oR = 0.5 * rcp_rn(dR * dR);
+        // twice the reference's o = 0.5 / d^2, whose quotients are the same
+        const double oL = rcp_rn(dL * dL), oR = rcp_rn(dR * dR);
         const double so = oL + oR, y = rcp_ulp(so);
         wL = div_rn(oL, so, y);
         wR = div_rn(oR, so, y);
