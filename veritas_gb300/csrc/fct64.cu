@@ -291,23 +291,36 @@ __global__ void k64_faces(const P64 *patches, const TileRef *tiles, const RunFie
 // kernels, and warps of vacuum are a third of a laser run's base patch.  With the same in
 // the passes below, 2.83 M cells: flux kernel 70 -> 66 us per direction, limiter R 87 -> 75,
 // limiter C and update 69 -> 54, f2 30 -> 27.
-__device__ __forceinline__ double stage_flux64(double *const *H, int id, const double *a, int s, double v,
-                                               double low) {
-    double x[5];
+// The stage is a template argument: with it at run time the products of later stages are
+// issued too, switched off lane by lane.
+template <int S>
+__device__ __forceinline__ double stage_flux64_s(double *const *H, int id, const double *a, double v, double low) {
+    double x[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
     unsigned long long any = bits(v) | bits(low);
 #pragma unroll
-    for (int k = 0; k < 5; k++) {
-        x[k] = k < s && !(s == 5 && k == 1) ? H[k][id] : 0.0;  // b_1 = 0 (Rectangle.cpp:1494)
-        any |= bits(x[k]);
-    }
+    for (int k = 0; k < S; k++)
+        if (!(S == 5 && k == 1)) {  // b_1 = 0 (Rectangle.cpp:1494)
+            x[k] = H[k][id];
+            any |= bits(x[k]);
+        }
+    x[S] = v;
     if (zeros(any)) return 0.0;
-    double h = a[0] * (s == 0 ? v : x[0]);
+    double h = a[0] * x[0];
 #pragma unroll
-    for (int k = 1; k < 6; k++) {
-        if (k > s || (s == 5 && k == 1)) continue;
-        h = h + a[k] * (k == s ? v : x[k < 5 ? k : 0]);
-    }
+    for (int k = 1; k <= S; k++)
+        if (!(S == 5 && k == 1)) h = h + a[k] * x[k];
     return h - a[6] * low;
+}
+__device__ __forceinline__ double stage_flux64(double *const *H, int id, const double *a, int s, double v,
+                                               double low) {
+    switch (s) {  // uniform
+        case 0: return stage_flux64_s<0>(H, id, a, v, low);
+        case 1: return stage_flux64_s<1>(H, id, a, v, low);
+        case 2: return stage_flux64_s<2>(H, id, a, v, low);
+        case 3: return stage_flux64_s<3>(H, id, a, v, low);
+        case 4: return stage_flux64_s<4>(H, id, a, v, low);
+        default: return stage_flux64_s<5>(H, id, a, v, low);
+    }
 }
 
 // High-order flux of a face from the velocities and values there and at its neighbours on
