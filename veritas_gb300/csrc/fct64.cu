@@ -34,6 +34,16 @@ namespace VX_FCT64_NS {
 
 using P64 = PatchT<double>;
 
+// The bits of a double.  Through an instruction the compiler does not look into: it turns
+// integer tests for a sign, zero or NaN on __double_as_longlong back into FP64 compares, of
+// which each takes the FP64 unit's time like any other FP64 instruction (2.83 M cells:
+// limiter R 75 -> 58 us, limiter C and update 65 -> 54 us).
+__device__ __forceinline__ long long as_bits(double x) {
+    long long b;
+    asm("mov.b64 %0, %1;" : "=l"(b) : "d"(x));
+    return b;
+}
+
 // The four cells around a face where the reconstruction needs no weights.
 // 2: all are +0.0, and so is the face value (every term of weno_face is +0.0).
 // 1: every |f| < 1e-14.  The smoothness indicators are then below 27 max|f|^2 < 2.7e-27,
@@ -60,7 +70,7 @@ __device__ __forceinline__ int weno_void(double f1, double f2, double f3, double
 // a > b and a < b for the mapped weights (positive, or NaN): on the bit patterns, where
 // any NaN makes the face value NaN whichever weight is picked.
 __device__ __forceinline__ bool wgt(double a, double b) {
-    return __double_as_longlong(a) > __double_as_longlong(b);
+    return as_bits(a) > as_bits(b);
 }
 
 // x / 2 and 2 x, exact, on the exponent field instead of the FP64 unit (its multiplication
@@ -181,24 +191,24 @@ __device__ __forceinline__ double vmin(double a, double b) { return (a < b) ? a 
 // FP64 unit is the limiter's bottleneck): x < 0 exactly when the sign bit is set and x is
 // neither -0 nor NaN; x > 0 when the sign bit is clear and x is neither +0 nor NaN.
 __device__ __forceinline__ double vmax0(double x) {
-    const long long b = __double_as_longlong(x);
+    const long long b = as_bits(x);
     const long long m = b & 0x7FFFFFFFFFFFFFFFLL;
     return (b < 0 && m != 0 && m <= 0x7FF0000000000000LL) ? 0.0 : x;
 }
 __device__ __forceinline__ double vmin0(double x) {
-    const long long b = __double_as_longlong(x);
+    const long long b = as_bits(x);
     return (b > 0 && b <= 0x7FF0000000000000LL) ? 0.0 : x;
 }
 // x > 0.0 (false for zeros and NaN) on the bit pattern
 __device__ __forceinline__ bool gt0(double x) {
-    const long long b = __double_as_longlong(x);
+    const long long b = as_bits(x);
     return b > 0 && b <= 0x7FF0000000000000LL;
 }
 
 
 // Both zeros (bits, of doubles or of several or-ed together), and finite.
 __device__ __forceinline__ unsigned long long bits(double x) {
-    return (unsigned long long)__double_as_longlong(x);
+    return (unsigned long long)as_bits(x);
 }
 __device__ __forceinline__ bool zeros(unsigned long long b) { return (b << 1) == 0; }
 __device__ __forceinline__ bool finite_hi(double x) {
@@ -288,11 +298,11 @@ __global__ void k64_faces(const P64 *patches, const TileRef *tiles, const RunFie
 // the earlier stages and its low-order flux (Rectangle.cpp:1396-1517).  RK coefficients
 // arrive pre-multiplied by dt.  Formed where the flux is: v need not be read again.  Zero
 // where they all are (vacuum), without the operations: FP64 instructions bound the flux
-// kernels, and warps of vacuum are a third of a laser run's base patch.  With the same in
-// the passes below, 2.83 M cells: flux kernel 70 -> 66 us per direction, limiter R 87 -> 75,
-// limiter C and update 69 -> 54, f2 30 -> 27.
+// kernels, and warps of vacuum are a third of a laser run's base patch (the same in the
+// passes below).
 // The stage is a template argument: with it at run time the products of later stages are
-// issued too, switched off lane by lane.
+// issued too, switched off lane by lane (2.83 M cells: x fluxes 102 .. 90 us at every stage,
+// with it 69 us on stage 0 to 101 us on stage 5).
 template <int S>
 __device__ __forceinline__ double stage_flux64_s(double *const *H, int id, const double *a, double v, double low) {
     double x[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
@@ -447,11 +457,13 @@ __global__ void k64_f2(const P64 *patches, const TileRef *tiles, const double *p
     P.f2[id] = v;
 }
 
-// vmin for limiter values (not negative, or NaN) on the bit patterns: b where either is NaN
+// vmin for limiter values on the bit patterns: b where either is NaN, else the lesser (-0
+// before +0; the limiter's values are not negative).
 __device__ __forceinline__ double vmin_r(double a, double b) {
-    const long long p = __double_as_longlong(a), q = __double_as_longlong(b);
-    if ((p | q) < 0) return vmin(a, b);
-    return (p < q && q <= 0x7FF0000000000000LL) ? a : b;
+    constexpr long long kAbs = 0x7FFFFFFFFFFFFFFFLL, kInf = 0x7FF0000000000000LL;
+    const long long p = as_bits(a), q = as_bits(b);
+    const bool nan = (p & kAbs) > kInf || (q & kAbs) > kInf;
+    return !nan && (p ^ ((p >> 63) & kAbs)) < (q ^ ((q >> 63) & kAbs)) ? a : b;
 }
 
 // Zalesak R+/R- on i in [-1,nx], j in [-1,np] (Rectangle.cpp:1536-1579).
@@ -480,7 +492,7 @@ __global__ void k64_limR(const P64 *patches, const TileRef *tiles) {
         int sign = 0;
 #pragma unroll
         for (int k = 0; k < 10; k++) {
-            const long long b = __double_as_longlong(v[k]);
+            const long long b = as_bits(v[k]);
             sign |= __double2hiint(v[k]);
             hi = b > hi ? b : hi;
             lo = b < lo ? b : lo;
@@ -501,7 +513,7 @@ __global__ void k64_limR(const P64 *patches, const TileRef *tiles) {
         // among them, takes the division as written.  Most cells of a smooth solution
         // skip the division; within 2^-600 .. 2^600 it takes the short form.
         auto ratio = [](double Q, double P) {
-            const long long q = __double_as_longlong(Q), p = __double_as_longlong(P);
+            const long long q = as_bits(Q), p = as_bits(P);
             if (q >= p && p < 0x7FF0000000000000LL && q <= 0x7FF0000000000000LL) return 1.0;
             const unsigned hq = (unsigned)(q >> 32) - 0x1a700000u, hp = (unsigned)(p >> 32) - 0x1a700000u;
             return vmin_r(1.0, hq < 0x4b000000u && hp < 0x4b000000u ? div_rn(Q, P, rcp_ulp(P)) : Q / P);
