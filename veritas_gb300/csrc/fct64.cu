@@ -115,7 +115,7 @@ __device__ __forceinline__ void weno_values(double f1, double f2, double f3, dou
     double fL = c6 * (-f1 + 5 * f2 + d3);
     double fR = c6 * (d2 + 5 * f3 - f4);
     if (none == 1) {
-        out_right = out_left = 0.5 * fL + 0.5 * fR;
+        out_right = out_left = half_of(fL) + half_of(fR);
         return;
     }
     double AL = f1 - d2 + f3;
@@ -264,8 +264,54 @@ __global__ void k64_gamma(const P64 *patches, const TileRef *tiles, const RunFie
     }
 }
 
+// The stage's antidiffusive flux of a face from its high-order flux `v` of stage s, those of
+// the earlier stages and its low-order flux (Rectangle.cpp:1396-1517).  RK coefficients
+// arrive pre-multiplied by dt.  Formed where the flux is: v need not be read again.  Zero
+// where they all are (vacuum), without the operations: FP64 instructions bound the flux
+// kernels, and warps of vacuum are a third of a laser run's base patch (the same in the
+// passes below).
+// The stage is a template argument: with it at run time the products of later stages are
+// issued too, switched off lane by lane (2.83 M cells: x fluxes 90 to 102 us at every stage,
+// with it 70 us on stage 0 to 90 us on stage 5).  The earlier stages' sum needs nothing of
+// this stage: of the p faces it is formed before the solve's E_x is known (p fluxes after
+// the solve 114 -> 87 us on the late stages).
+// history64: the earlier stages' part of the sum, S > 0.
+template <int S>
+__device__ __forceinline__ double history64_s(double *const *H, int id, const double *a) {
+    double x[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+    unsigned long long any = 0;
+#pragma unroll
+    for (int k = 0; k < S; k++)
+        if (!(S == 5 && k == 1)) {  // b_1 = 0 (Rectangle.cpp:1494)
+            x[k] = H[k][id];
+            any |= bits(x[k]);
+        }
+    if (zeros(any)) return 0.0;
+    double h = a[0] * x[0];
+#pragma unroll
+    for (int k = 1; k < S; k++)
+        if (!(S == 5 && k == 1)) h = h + a[k] * x[k];
+    return h;
+}
+__device__ __forceinline__ double history64(double *const *H, int id, const double *a, int s) {
+    switch (s) {  // uniform
+        case 0: return 0.0;
+        case 1: return history64_s<1>(H, id, a);
+        case 2: return history64_s<2>(H, id, a);
+        case 3: return history64_s<3>(H, id, a);
+        case 4: return history64_s<4>(H, id, a);
+        default: return history64_s<5>(H, id, a);
+    }
+}
+// The rest, from that sum.
+__device__ __forceinline__ double stage_flux64(double hist, const double *a, int s, double v, double low) {
+    if (zeros(bits(hist) | bits(v) | bits(low))) return 0.0;
+    return (s == 0 ? a[0] * v : hist + a[s] * v) - a[6] * low;
+}
+
 // Face velocities and reconstructed face values (Rectangle.cpp:1278-1312).
-__global__ void k64_faces(const P64 *patches, const TileRef *tiles, const RunFields *fields, int use_f0, int part) {
+__global__ void k64_faces(const P64 *patches, const TileRef *tiles, const RunFields *fields, const double *params,
+                          int step, int use_f0, int part) {
     VX_PDL_WAIT();
     VX_TILE_PROLOGUE
     const double *f = use_f0 ? P.f0 : P.f1;
@@ -283,53 +329,16 @@ __global__ void k64_faces(const P64 *patches, const TileRef *tiles, const RunFie
         P.fp[id] = weno_face(f[pidx(i, j - 2, pit)], f[pidx(i, j - 1, pit)], f[id], f[pidx(i, j + 1, pit)], gt0(am));
     }
     // The part of the p faces that does not need E_x, formed beside the Poisson solve: both
-    // upwind candidates (fp and, as scratch, Rp) and the velocity's second term (Rm; the
-    // limiter rewrites both later in the stage).  k64_pflux_pick goes on from these.
+    // upwind candidates (fp and, as scratch, Rp), the velocity's second term (Rm; the limiter
+    // rewrites both later in the stage) and, in FpDS, the earlier stages' part of the stage
+    // flux.  k64_pflux_pick goes on from these.
     if ((part & 4) && i >= -1 && i <= P.nx && j >= 0 && j <= P.np) {
         double vr, vl;
         weno_values<true>(f[pidx(i, j - 2, pit)], f[pidx(i, j - 1, pit)], f[id], f[pidx(i, j + 1, pit)], true, vr, vl);
         P.fp[id] = vr;
         P.Rp[id] = vl;
         P.Rm[id] = P.kp * (g[pidx(i + 1, j, pit)] - g[id]);
-    }
-}
-
-// The stage's antidiffusive flux of a face from its high-order flux `v` of stage s, those of
-// the earlier stages and its low-order flux (Rectangle.cpp:1396-1517).  RK coefficients
-// arrive pre-multiplied by dt.  Formed where the flux is: v need not be read again.  Zero
-// where they all are (vacuum), without the operations: FP64 instructions bound the flux
-// kernels, and warps of vacuum are a third of a laser run's base patch (the same in the
-// passes below).
-// The stage is a template argument: with it at run time the products of later stages are
-// issued too, switched off lane by lane (2.83 M cells: x fluxes 102 .. 90 us at every stage,
-// with it 69 us on stage 0 to 101 us on stage 5).
-template <int S>
-__device__ __forceinline__ double stage_flux64_s(double *const *H, int id, const double *a, double v, double low) {
-    double x[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-    unsigned long long any = bits(v) | bits(low);
-#pragma unroll
-    for (int k = 0; k < S; k++)
-        if (!(S == 5 && k == 1)) {  // b_1 = 0 (Rectangle.cpp:1494)
-            x[k] = H[k][id];
-            any |= bits(x[k]);
-        }
-    x[S] = v;
-    if (zeros(any)) return 0.0;
-    double h = a[0] * x[0];
-#pragma unroll
-    for (int k = 1; k <= S; k++)
-        if (!(S == 5 && k == 1)) h = h + a[k] * x[k];
-    return h - a[6] * low;
-}
-__device__ __forceinline__ double stage_flux64(double *const *H, int id, const double *a, int s, double v,
-                                               double low) {
-    switch (s) {  // uniform
-        case 0: return stage_flux64_s<0>(H, id, a, v, low);
-        case 1: return stage_flux64_s<1>(H, id, a, v, low);
-        case 2: return stage_flux64_s<2>(H, id, a, v, low);
-        case 3: return stage_flux64_s<3>(H, id, a, v, low);
-        case 4: return stage_flux64_s<4>(H, id, a, v, low);
-        default: return stage_flux64_s<5>(H, id, a, v, low);
+        if (step > 0) P.FpDS[id] = history64(P.FpH, id, params + param_base(P.run, step), step);
     }
 }
 
@@ -367,7 +376,7 @@ __global__ void k64_flux(const P64 *patches, const TileRef *tiles, const double 
         } else {
             low = P.FxL[id];
         }
-        P.FxDS[id] = stage_flux64(P.FxH, id, a, step, v, low);
+        P.FxDS[id] = stage_flux64(history64(P.FxH, id, a, step), a, step, v, low);
     }
     if ((part & 2) && i >= -1 && i <= P.nx && j >= 0 && j <= P.np && !(P.ifp && P.ifp[id])) {
         double am = P.ep[id], ap1 = P.ep[id + pit], am1 = P.ep[id - pit];
@@ -381,7 +390,7 @@ __global__ void k64_flux(const P64 *patches, const TileRef *tiles, const double 
         } else {
             low = P.FpL[id];
         }
-        P.FpDS[id] = stage_flux64(P.FpH, id, a, step, v, low);
+        P.FpDS[id] = stage_flux64(history64(P.FpH, id, a, step), a, step, v, low);
     }
 }
 
@@ -429,7 +438,7 @@ __global__ void k64_pflux_pick(const P64 *patches, const TileRef *tiles, const R
     } else {
         low = P.FpL[id];
     }
-    P.FpDS[id] = stage_flux64(P.FpH, id, a, step, v, low);
+    P.FpDS[id] = stage_flux64(step > 0 ? P.FpDS[id] : 0.0, a, step, v, low);
 }
 
 __device__ __forceinline__ bool active_face(const P64 &P, int i, int j) {
@@ -634,7 +643,8 @@ void VX_FCT64_LAUNCH(const FctLaunch &L, int sub) {
             vx_launch(k64_gamma, L.ntiles, blk.x, 0, L.stream, pp, L.tiles, L.fields, (int)blk.y);
             break;
         case kSubFaces:
-            vx_launch(k64_faces, L.ntiles, blk, 0, L.stream, pp, L.tiles, L.fields, L.use_f0, L.part ? L.part : 3);
+            vx_launch(k64_faces, L.ntiles, blk, 0, L.stream, pp, L.tiles, L.fields, L.params, L.step, L.use_f0,
+                      L.part ? L.part : 3);
             break;
         case kSubFlux:
             if (L.part == 8)

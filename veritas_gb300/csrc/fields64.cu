@@ -117,9 +117,11 @@ struct MomSmem {
 // of the quotient.
 __device__ __forceinline__ double fast_log_ratio(double Gn, double G) {
     const double s = Gn + G;
-    if (G != 0.0 && s != 0.0) {
+    // tests on the high words (a zero or a subnormal has exponent 0): no FP64 compares
+    constexpr unsigned kExp = 0x7ff00000u, kHundredth = 0x3f847ae1u;  // high word of 0.01
+    if (((unsigned)__double2hiint(G) & kExp) != 0 && ((unsigned)__double2hiint(s) & kExp) != 0) {
         const double z = (Gn - G) * rcp_ulp(s);
-        if (fabs(z) <= 0.01) {
+        if (((unsigned)__double2hiint(z) & 0x7fffffffu) < kHundredth) {
             const double z2 = z * z;
             const double poly = __fma_rn(z2, __fma_rn(z2, __fma_rn(z2, 1.0 / 7.0, 0.2), 1.0 / 3.0), 1.0);
             return (2.0 * z) * poly;
