@@ -719,7 +719,8 @@ __device__ void pois_tail(const PoisTail &T, int t0, double *x) {
 // load placed after the previous row's shuffle-dependent store would add its shared-memory
 // latency to every row of the chain.  The look-ahead reads at most two rows past the
 // chunk: the staged look-ahead rows, or past n the neutral entries pois_stage_fwd writes
-// there (zero coefficients, no slot row).  206 cycles per row.
+// there (zero coefficients, no slot row).  198 cycles per row (204 rolled, 206 and 204 unrolled by
+// three and four).
 __device__ void pois_fwd_fast(const PoisFwdChunk &B, const BandFactor &F, int r0, int cnt, int n, double *x,
                               double &V, double &w1) {
     // Only lanes 0..7 (band lanes 0..3, accumulator lanes 4..7) run the recurrence.
@@ -748,6 +749,7 @@ __device__ void pois_fwd_fast(const PoisFwdChunk &B, const BandFactor &F, int r0
     double vld = ld >= 0 ? x[ld] : 0.0;
     int tk = B.take[k0];
     double fb = (lane == 3 && r0 + 4 < n) ? x[r0 + 4] : 0.0;
+#pragma unroll 2
     for (int q = 0; q < cnt; q++) {
         const int i = r0 + q;
         // row q+1's operands; a slot's row r >= step + 4 and the right-hand side x[i + 5]
