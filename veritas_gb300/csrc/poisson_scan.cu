@@ -256,10 +256,12 @@ __global__ void __cluster_dims__(kPsCluster, 1, 1) __launch_bounds__(kPsMaxThrea
 #pragma unroll
     for (int k = 0; k < 3; k++) u[k] = remote(k == 2 ? m - 1 : k);
     // The last warp's lanes: phi at 1, 2, n - 3, n - 2, n - 1 (phi_0 and Ex0 come from them)
-    // and at the two cells on either side of the block's.
-    int pe = 0;
+    // and at the two cells on either side of the block's (a block without cells has no sides:
+    // its bounds lie past the vector's end).
+    const int nends = cnt > 0 ? 9 : 5;
+    int pe = 0;  // 0 .. n - 1
     double ve = 0.0;
-    if (ends && lane < 9) {
+    if (ends && lane < nends) {
         pe = lane < 2 ? lane + 1 : lane < 5 ? n - 5 + lane : lane < 7 ? p0 - 7 + lane : p1 - 7 + lane;
         pe = pe < 0 ? pe + n : pe >= n ? pe - n : pe;
         if (pe > 0) ve = remote(pe - 1);
@@ -273,7 +275,7 @@ __global__ void __cluster_dims__(kPsCluster, 1, 1) __launch_bounds__(kPsMaxThrea
     const double fc = P.fcoef[run];
     double ex0 = 0.0;
     if (ends) {
-        double ph = (lane < 9 && pe > 0) ? phi_value(D, pe - 1, ve, t) : 0.0;
+        double ph = (lane < nends && pe > 0) ? phi_value(D, pe - 1, ve, t) : 0.0;
         const double q1 = __shfl_sync(full, ph, 0), q2 = __shfl_sync(full, ph, 1), z3 = __shfl_sync(full, ph, 2),
                      z2 = __shfl_sync(full, ph, 3), z1 = __shfl_sync(full, ph, 4);
         const double phi0 = b0 - (D.w1 * q1 + D.w2 * q2 + D.w2 * z2 + D.w1 * z1);
