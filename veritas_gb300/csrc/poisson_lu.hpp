@@ -50,7 +50,7 @@ struct PoissonLU {
         // (1 / u_ii - y, u1) in the fifth's eight bytes.  Empty when a row does not fit
         // (far_pre_col is then -1).
         static constexpr int kCols = 5;
-        static constexpr int kTail = 8;  // rows solved one by one: the far columns are n-1 and n-2
+        static constexpr int kTail = 8;  // rows solved before the chunks: the far columns are n-1 and n-2
         std::vector<double> sweep;
         int far_pre_col = -1;
     };
