@@ -1292,7 +1292,7 @@ __device__ void pipe_summer(const PipeLaunch &K, int lane) {
 // scheduled in.  Same arithmetic as k64_moments + k_assemble + k_poisson.
 // The fast form's workers are called, the exact form's inlined: the kernel has 64 registers a
 // thread, and which way the sweeps keep theirs differs between the two (4096 x 512 in two
-// levels per step: fast 14.32 ms inlined, 13.40 called; exact 13.74 and 14.23).
+// levels per step: fast 14.32 ms inlined, 13.57 called; exact 13.76 and 14.23).
 template <bool FAST>
 __device__ __noinline__ void pipe_columns_call(const PipeLaunch &K, int *ticket, int g, int tid) {
     pipe_columns<FAST>(K, ticket, g, tid);
