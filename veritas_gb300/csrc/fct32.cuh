@@ -326,6 +326,11 @@ __device__ __forceinline__ void cupdate32(const P32 *patches, const TileRef t, i
     if (P.cmask && col) mask = *reinterpret_cast<const unsigned *>(P.cmask + id);  // four cells' bytes
     const V4 one{{1.0f, 1.0f, 1.0f, 1.0f}};
     V4 cx = one, cp = one;  // C is 1 outside the interior
+    // C of a face between two cells, from R of the upper (p, m) and the lower (l, lm) and its flux
+    auto face = [](float flux, float p, float m, float l, float lm) {
+        const bool up = flux > 0.0f;
+        return fminf(up ? p : l, up ? lm : m);
+    };
     if (i >= 0 && i < P.nx) {
         const float *Rp = P.Rp, *Rm = P.Rm, *DX = P.FxDS, *DP = P.FpDS;
         const bool in = i >= 1, inn = i + 1 < P.nx;  // rows i and i + 1 have faces between cells
@@ -362,11 +367,6 @@ __device__ __forceinline__ void cupdate32(const P32 *patches, const TileRef t, i
             ep = Rp[id + eoff];
             em = Rm[id + eoff];
         }
-        // C of a face between two cells, from R of the upper (p, m) and the lower (l, lm) and its flux
-        auto face = [](float flux, float p, float m, float l, float lm) {
-            const bool up = flux > 0.0f;
-            return fminf(up ? p : l, up ? lm : m);
-        };
         float lp = __shfl_up_sync(full, rpc.v[3], 1), lm = __shfl_up_sync(full, rmc.v[3], 1);
         if (lane == 0) {
             lp = ep;
@@ -408,6 +408,17 @@ __device__ __forceinline__ void cupdate32(const P32 *patches, const TileRef t, i
                 P.Cx[id + e] = out ? 1.0f : cx.v[e];
                 P.Cp[id + e] = out ? 1.0f : cp.v[e];
             }
+        // Row j = 0 at the lower momentum edge: its faces move nothing, but the exchange passes
+        // their C on to finer faces that do, by the branch of the true flux.  Formed again for
+        // these alone: with the fluxes kept as loaded for every C the step of 38.6 M cells took
+        // 10.57 ms instead of 10.32.
+        const int e = -j;
+        if (e >= 0 && e < 4 && P.pm > 0 && ((mask >> (8 * e)) & kCStore) && i >= 1 && i < P.nx) {
+            const int k = id + e;
+            const float rp = P.Rp[k], rm = P.Rm[k];
+            P.Cx[k] = face(P.FxDS[k], rp, rm, P.Rp[k - pit], P.Rm[k - pit]);
+            P.Cp[k] = face(P.FpDS[k], rp, rm, P.Rp[k - 1], P.Rm[k - 1]);
+        }
     }
 }
 #undef VX_ROW32
