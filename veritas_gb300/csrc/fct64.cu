@@ -148,16 +148,18 @@ __device__ __forceinline__ void weno_values(double f1, double f2, double f3, dou
 #else
     // within 1e-10 .. 1e95 every intermediate of the short quotients is a normal number
     const bool plain = (unsigned)__double2hiint(dL) < 0x53a00000u && (unsigned)__double2hiint(dR) < 0x53a00000u;
+    bool hard = !plain;
     if (plain) {
         // twice the reference's o = 0.5 / d^2, whose quotients are the same
-        const double oL = rcp_rn(dL * dL), oR = rcp_rn(dR * dR);
+        const double oL = rcp_rn(dL * dL, hard), oR = rcp_rn(dR * dR, hard);
         const double so = oL + oR, y = rcp_ulp(so);
-        wL = div_rn(oL, so, y);
-        wR = div_rn(oR, so, y);
-    } else {
-        const double oL = 0.5 / (dL * dL), oR = 0.5 / (dR * dR);
-        wL = oL / (oL + oR);
-        wR = oR / (oL + oR);
+        wL = div_rn(oL, so, y, hard);
+        wR = div_rn(oR, so, y, hard);
+    }
+    if (hard) {
+        const double oL = div_call(0.5, dL * dL), oR = div_call(0.5, dR * dR);
+        wL = div_call(oL, oL + oR);
+        wR = div_call(oR, oL + oR);
     }
 #endif
     double wL0 = wL * (0.75 + wL * (wL - 0.5));
@@ -172,7 +174,9 @@ __device__ __forceinline__ void weno_values(double f1, double f2, double f3, dou
     // face between regions 1e60 apart) the residual would leave the normal range
     const double inv = rcp_ulp(sw);
     auto quot = [&](double a) {
-        return (plain && (unsigned)__double2hiint(a) >= 0x0c000000u) ? div_rn(a, sw, inv) : a / sw;
+        bool gen = !(plain && (unsigned)__double2hiint(a) >= 0x0c000000u);
+        const double q = div_rn(a, sw, inv, gen);
+        return gen ? div_call(a, sw) : q;
     };
 #endif
     const double w = quot(BOTH || right ? pr : pl);
@@ -264,7 +268,11 @@ __global__ void k64_gamma(const P64 *patches, const TileRef *tiles, const RunFie
     double p = P.pmin + P.dp * (double)(j + P.p_pos);
     for (int i = max(t.i0, -1); i < i1; i++) {
         double as = P.qq * a_sq_face(P, F, i);
-        P.gam[pidx(i, j, P.pitch)] = sqrt_rn(1.0 + ((p * p) + as) * P.g2);
+        const double x = 1.0 + ((p * p) + as) * P.g2;
+        bool hard = false;
+        double g = sqrt_rn(x, hard);
+        if (hard) g = sqrt_call(x);
+        P.gam[pidx(i, j, P.pitch)] = g;
     }
 }
 
@@ -529,7 +537,11 @@ __global__ void k64_limR(const P64 *patches, const TileRef *tiles) {
             const long long q = as_bits(Q), p = as_bits(P);
             if (q >= p && p < 0x7FF0000000000000LL && q <= 0x7FF0000000000000LL) return 1.0;
             const unsigned hq = (unsigned)(q >> 32) - 0x1a700000u, hp = (unsigned)(p >> 32) - 0x1a700000u;
-            return vmin_r(1.0, hq < 0x4b000000u && hp < 0x4b000000u ? div_rn(Q, P, rcp_ulp(P)) : Q / P);
+            bool gen = !(hq < 0x4b000000u && hp < 0x4b000000u);
+            double v = 0.0;
+            if (!gen) v = div_rn(Q, P, rcp_ulp(P), gen);
+            if (gen) v = div_call(Q, P);
+            return vmin_r(1.0, v);
         };
         if (up) rp = ratio(Qp, Pp);
         if (um) rm = ratio(Qm, Pm);

@@ -155,15 +155,17 @@ __device__ __forceinline__ double face_a(double f1, double f2, double f3, double
     // dL, dR are at least about 1e-20; below 2^600 (A below 1e45) the quotients take the short
     // form with the rounding of `/`
     double wL, wR;
-    if (__double2hiint(dL) < 0x65700000 && __double2hiint(dR) < 0x65700000) {
-        const double oL = div_rn(0.5, dL, rcp_ulp(dL)), oR = div_rn(0.5, dR, rcp_ulp(dR));
+    bool gen = !(__double2hiint(dL) < 0x65700000 && __double2hiint(dR) < 0x65700000);
+    if (!gen) {
+        const double oL = div_rn(0.5, dL, rcp_ulp(dL), gen), oR = div_rn(0.5, dR, rcp_ulp(dR), gen);
         const double o = add(oL, oR), y = rcp_ulp(o);
-        wL = div_rn(oL, o, y);
-        wR = div_rn(oR, o, y);
-    } else {
-        const double oL = 0.5 / dL, oR = 0.5 / dR;
-        wL = oL / add(oL, oR);
-        wR = oR / add(oL, oR);
+        wL = div_rn(oL, o, y, gen);
+        wR = div_rn(oR, o, y, gen);
+    }
+    if (gen) {
+        const double oL = div_call(0.5, dL), oR = div_call(0.5, dR);
+        wL = div_call(oL, add(oL, oR));
+        wR = div_call(oR, add(oL, oR));
     }
     return add(mul(wL, fL), mul(wR, fR));
 }

@@ -113,8 +113,7 @@ struct MomSmem {
 // ln(Gn / G) for the fast FP64 form.  Neighbouring nodes of a p grid differ by a factor
 // 1 + dp / gamma, so z = (Gn - G) / (Gn + G) is small and ln(Gn / G) = 2 atanh(z) =
 // 2 z (1 + z^2/3 + z^4/5 + z^6/7) to within z^8 / 9 < 1.2e-17 relative for |z| <= 0.01;
-// otherwise (and for G = 0 past the window's end, whose value is not used) the logarithm
-// of the quotient.
+// otherwise the logarithm of the quotient.
 __device__ __forceinline__ double fast_log_ratio(double Gn, double G) {
     const double s = Gn + G;
     // tests on the high words (a zero or a subnormal has exponent 0): no FP64 compares
@@ -156,20 +155,26 @@ __device__ __forceinline__ void mom_window(const P64 &P, const double *f, bool r
         cc[q] = 0.0;
         cj[q] = 0.0;
         if (real) {
-            double G = 0.0, V = 0.0;
+            double G = 1.0, V = 0.0;  // 1 past the last node: those lanes' logarithms are not used
             if (j <= np + 1) {
-                if (FAST) {
-                    const double g = sqrt_rn(__fma_rn(__fma_rn(p, p, a[q]), P.g2, 1.0));
-                    G = __fma_rn(c1, p, g);
-                } else {
-                    double g = sqrt_rn(1.0 + ((p * p) + a[q]) * P.g2);
-                    G = g + c1 * p;
-                }
+                const double x = FAST ? __fma_rn(__fma_rn(p, p, a[q]), P.g2, 1.0) : 1.0 + ((p * p) + a[q]) * P.g2;
+                bool hard = false;
+                const double g = sqrt_rn(x, hard);
+                G = FAST ? __fma_rn(c1, p, g) : g + c1 * p;
+                // after its first use, which covers the test; the fast form does without
+                if (!FAST && hard) G = sqrt_call(x) + c1 * p;
             }
             if (j <= np) V = rtb == 1 ? f3 : (FAST ? rel_pick_fma(P, k0 + q, a1, a2, a3, f3) : rel_pick(P, k0 + q, a1, a2, a3, f3)) + cor;
             const double Gn = __shfl_down_sync(full, G, 1);
-            // valid for lanes 0..30 (lane 31's Gn is its own G; beyond n_p + 1, G = 0)
-            const double L = FAST ? c2 * fast_log_ratio(Gn, G) : c2 * log(div_rn(Gn, G, rcp_ulp(G)));
+            // valid for lanes 0..30 (lane 31's Gn is its own G)
+            double L;
+            if (FAST) {
+                L = c2 * fast_log_ratio(Gn, G);
+            } else {
+                bool hard = false;
+                L = c2 * log(div_rn(Gn, G, rcp_ulp(G), hard));
+                if (hard) L = c2 * log(Gn / G);  // likewise
+            }
             const double Lm = __shfl_up_sync(full, L, 1);
             const double Lp = __shfl_down_sync(full, L, 1);
             const double Vm = __shfl_up_sync(full, V, 1);
@@ -685,23 +690,26 @@ __device__ void pois_stage_tail(PoisTail &T, const BandFactor &F, int t0, int t)
 }
 // Solved by warp 0, a row per lane: column by column from the last, which subtracts every
 // row's terms in descending column order as dgetrs does (a zero where the factor has no
-// entry changes nothing).  One thread with its operands in global memory took 8 us.
-__device__ void pois_tail(const PoisTail &T, int t0, double *x) {
+// entry changes nothing).  The quotients on the way are short ones; each lane then checks
+// its own against IEEE division, and if one differs the rows are solved again one by one.
+// One thread with its operands in global memory took 8 us.
+__device__ void pois_tail(const PoisTail &T, const BandFactor &F, int t0, double *x) {
     constexpr unsigned act = (1u << kPoisTail) - 1;
     const int l = threadIdx.x & 31;
     if (l >= kPoisTail) return;
-    double s = x[t0 + l], mine = 0.0;
+    double s = x[t0 + l], mine = 0.0, num = 0.0;
     const double diag = T.diag[l], y = T.y[l];
     for (int c = kPoisTail - 1; c >= 0; c--) {
-        const double u = T.u[l][c];
-        // the rounding of s / diag, in short where s is in range (the diagonal is of order one)
-        const unsigned h = ((unsigned)__double2hiint(s) & 0x7fffffffu) - 0x16800000u;
-        const double q = h < 0x52800000u ? div_rn(s, diag, y) : s / diag;
+        const double u = T.u[l][c], q = div_short(s, diag, y);
         const double xc = __shfl_sync(act, q, c);
-        if (l == c) mine = q;
+        if (l == c) {
+            mine = q;
+            num = s;
+        }
         s = s - xc * u;
     }
-    x[t0 + l] = mine;
+    if (!__any_sync(act, __double_as_longlong(num / diag) != __double_as_longlong(mine))) x[t0 + l] = mine;
+    else if (l == 0) pois_rows_plain<true>(F, t0, t0 + kPoisTail, t0 + kPoisTail, x, true);
 }
 
 // Forward sweep of one chunk, software-pipelined on lanes 0..7 of warp 0.  Row i's sum is
@@ -1013,7 +1021,7 @@ __device__ __forceinline__ void poisson_solve(const PoissonLaunch &L, unsigned c
     // further down), then chunks of R rows, descending
     {
         if (!tail && threadIdx.x == 0) pois_rows_plain<true>(lu.U, 0, n, n, x, true);
-        if (tail && threadIdx.x < 32) pois_tail(s_tail, t0, x);
+        if (tail && threadIdx.x < 32) pois_tail(s_tail, lu.U, t0, x);
         if (threadIdx.x == 0) s_bad = 0;
         __syncthreads();
         const int nbwd = (t0 + kPoisRows - 1) / kPoisRows;
@@ -1292,7 +1300,7 @@ __device__ void pipe_summer(const PipeLaunch &K, int lane) {
 // scheduled in.  Same arithmetic as k64_moments + k_assemble + k_poisson.
 // The fast form's workers are called, the exact form's inlined: the kernel has 64 registers a
 // thread, and which way the sweeps keep theirs differs between the two (4096 x 512 in two
-// levels per step: fast 14.32 ms inlined, 13.57 called; exact 13.76 and 14.23).
+// levels per step: fast 13.64 ms inlined, 13.42 called; exact 13.78 and 14.29).
 template <bool FAST>
 __device__ __noinline__ void pipe_columns_call(const PipeLaunch &K, int *ticket, int g, int tid) {
     pipe_columns<FAST>(K, ticket, g, tid);
