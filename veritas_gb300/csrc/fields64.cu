@@ -171,7 +171,7 @@ __device__ __forceinline__ void mom_window(const P64 &P, const double *f, bool r
             if (FAST) {
                 L = c2 * fast_log_ratio(Gn, G);
             } else {
-                bool hard = false;
+                bool hard = (unsigned)(exp_bits(G) - 963) > 120u;  // G beyond 2^-60 .. 2^60, or 0
                 L = c2 * log(div_rn(Gn, G, rcp_ulp(G), hard));
                 if (hard) L = c2 * log(Gn / G);  // likewise
             }
@@ -207,7 +207,9 @@ __device__ __forceinline__ void mom_window(const P64 &P, const double *f, bool r
 // Contributions are bounded from F >= |f| over the window's cells and stencil: charge
 // |V| <= 8 F with the sub-cell interpolation (its weights sum to less than 7), F without;
 // current |V L + (L+ - L-)(V+ - V-) / 48| <= 1.09 |V| max|L| with |L| <= dp (the logarithm
-// of the node ratio grows by c1 dp / gamma per cell).
+// of the node ratio grows by c1 dp / gamma per cell).  As computed, the ratio's cancellation
+// at negative p puts 4 gamma^2 2^-53 on top: below gamma = 1e6 that is lost in the bound's
+// margin, and beyond it (where the ratio comes to 1 / 0, too) every window is formed.
 struct MomSum {
     double lo0 = 0.0, hi0 = 0.0, lo1 = 0.0, hi1 = 0.0;
     __device__ __forceinline__ bool split() const { return !(lo0 == hi0 && lo1 == hi1); }
@@ -329,9 +331,11 @@ __global__ void __launch_bounds__(kScreenRows * 32) k64_mom_screen(MomLaunch M) 
         if (own && lane == 0) s_max[r - halo] = top;
     }
     if (threadIdx.x < ncol) {
-        bool fin = true;  // a field that is not finite makes every cell's current so
+        // gamma^2 - 1 < 1e12 over the column's nodes (false for a field that is not a number)
+        const double pe = fmax(fabs(P.pmin + P.dp * (P.p_pos - 1)), fabs(P.pmin + P.dp * (P.p_pos + np + 1)));
+        bool fin = true;
         for (int k = 0; k < rtb; k++)
-            fin = fin && isfinite(cell_asq(M.fields[P.run], (i0 + (int)threadIdx.x + P.x_pos) * rtb + k));
+            fin = fin && (pe * pe + P.qq * cell_asq(M.fields[P.run], (i0 + (int)threadIdx.x + P.x_pos) * rtb + k)) * P.g2 < 1e12;
         s_field[threadIdx.x] = fin;
     }
     __syncthreads();
