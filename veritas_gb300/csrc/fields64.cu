@@ -946,12 +946,11 @@ __device__ void pipe_rows(const PipeLaunch &K, int run, int c, double *x, int t,
 // instantiations let the compiler see x's address space: with one pointer chosen at run
 // time its loads and stores in the sweeps go through generic addressing.
 template <bool XS, bool PIPE>
-__device__ __forceinline__ void poisson_solve(const PoissonLaunch &L, unsigned char *smem_raw, double *x,
+__device__ __forceinline__ void poisson_solve(const PoissonLaunch &L, int run, unsigned char *smem_raw, double *x,
                                               const PipeLaunch *K) {
     PoisChunk *buf = (PoisChunk *)smem_raw;  // two chunk buffers, then the solution vector
     __shared__ int s_bad;
     __shared__ PoisTail s_tail;
-    const int run = blockIdx.x;
     RunFields &F = L.fields[run];
     const LUDev &lu = L.lu[run];
     const int n = F.n;
@@ -1117,8 +1116,9 @@ __device__ __forceinline__ void poisson_solve(const PoissonLaunch &L, unsigned c
 __global__ void __launch_bounds__(1024, 1) k_poisson(PoissonLaunch L) {
     VX_PDL_WAIT();
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    if (L.x_in_smem) poisson_solve<true, false>(L, smem_raw, (double *)(smem_raw + 2 * sizeof(PoisChunk)), nullptr);
-    else poisson_solve<false, false>(L, smem_raw, L.fields[blockIdx.x].phi, nullptr);
+    const int run = blockIdx.x;
+    if (L.x_in_smem) poisson_solve<true, false>(L, run, smem_raw, (double *)(smem_raw + 2 * sizeof(PoisChunk)), nullptr);
+    else poisson_solve<false, false>(L, run, smem_raw, L.fields[run].phi, nullptr);
 }
 
 // ---- workers of the pipelined launch
@@ -1295,13 +1295,13 @@ __device__ void pipe_summer(const PipeLaunch &K, int lane) {
     }
 }
 
-// Moments, assembly and the exact solve in one launch.  Block r < nruns solves run r (its
-// forward sweep starts as soon as the moments of its first rows are summed, instead of
-// after the whole moments kernel); the next K.summers blocks carry four summing warps each
-// (pipe_summer); every other block carries up to kPipeGroups groups of column warps (pipe_columns).
-// Column warps wait for nothing outside their group, summing warps only for column
-// warps, the solve only for summing warps: every wait ends whatever order the blocks are
-// scheduled in.  Same arithmetic as k64_moments + k_assemble + k_poisson.
+// Moments, assembly and the exact solve in one launch, a block per SM.  A block solves one run
+// (its forward sweep starts as soon as the moments of its first rows are summed, instead of
+// after the whole moments kernel), carries four summing warps (pipe_summer), or up to
+// kPipeGroups groups of column warps (pipe_columns).  Column warps wait for nothing outside
+// their group, summing warps only for column warps, the solve only for summing warps; the
+// blocks' order (pipe_block) lets every wait end on any number of SMs.  Same arithmetic as
+// k64_moments + k_assemble + k_poisson.
 // The fast form's workers are called, the exact form's inlined: the kernel has 64 registers a
 // thread, and which way the sweeps keep theirs differs between the two (4096 x 512 in two
 // levels per step: fast 13.64 ms inlined, 13.42 called; exact 13.78 and 14.29).
@@ -1317,11 +1317,12 @@ template <bool FAST>
 __global__ void __launch_bounds__(1024, 1) k64_moments_poisson(PipeLaunch K) {
     VX_PDL_WAIT();
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    if ((int)blockIdx.x < K.P.nruns) {
+    const PipeBlock me = pipe_block((int)blockIdx.x, K.P.nruns, K.summers);
+    if (me.role == kPipeSolver) {
         if (K.P.x_in_smem)
-            poisson_solve<true, true>(K.P, smem_raw, (double *)(smem_raw + 2 * sizeof(PoisChunk)), &K);
-        else poisson_solve<false, true>(K.P, smem_raw, K.P.fields[blockIdx.x].phi, &K);
-    } else if ((int)blockIdx.x < K.P.nruns + K.summers) {
+            poisson_solve<true, true>(K.P, me.run, smem_raw, (double *)(smem_raw + 2 * sizeof(PoisChunk)), &K);
+        else poisson_solve<false, true>(K.P, me.run, smem_raw, K.P.fields[me.run].phi, &K);
+    } else if (me.role == kPipeSummer) {
         if (threadIdx.x < 4 * 32) {  // warps 0..3: one per sub-partition
             if constexpr (FAST) pipe_summer_call<FAST>(K, (int)threadIdx.x & 31);
             else pipe_summer<FAST>(K, (int)threadIdx.x & 31);

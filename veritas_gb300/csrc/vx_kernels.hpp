@@ -4,6 +4,7 @@
 
 #include <utility>
 
+#include "pipe_blocks.hpp"
 #include "vx_common.hpp"
 
 namespace vx {
@@ -184,7 +185,7 @@ void launch_poisson(const PoissonLaunch &L);
 constexpr int kPoisRowsHost = 256;  // rows per chunk of k_poisson (fields64.cu kPoisRows)
 
 // Moments, assembly and exact Poisson solve of an FP64 set in one launch
-// (k64_moments_poisson): blocks 0 .. nruns-1 solve, each following its run's moments as
+// (k64_moments_poisson): a block per run solves, following its run's moments as
 // they are completed; the other blocks are persistent workers.  Groups of kPipeCols column
 // warps take parts of items — an item is one p window of one moment unit's 15 columns (one
 // pair of sub-columns), a part kPipeCols of the columns — by ticket in the order the
