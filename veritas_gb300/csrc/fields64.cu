@@ -362,7 +362,7 @@ void launch_mom_screen64(const MomLaunch &M) {
         cudaMemsetAsync(M.screen, 1, (size_t)(M.ncols / kMomCols) * M.maxnwin * kMomScreen * sizeof(unsigned), M.stream);
         return;
     }
-    if (smem > 48 * 1024) cudaFuncSetAttribute(k64_mom_screen, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (smem > 48 * 1024) vx_allow_smem(k64_mom_screen);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(M.ncols / kMomCols);
     cfg.blockDim = dim3(kScreenRows * 32);
@@ -1369,7 +1369,7 @@ void launch_poisson(const PoissonLaunch &L) {
     const int base = 2 * (int)sizeof(PoisChunk);
     P.x_in_smem = (L.maxn <= kPoisSmemMaxN && base + 8 * L.maxn <= max_smem) ? 1 : 0;
     const int smem = base + (P.x_in_smem ? 8 * L.maxn : 0);
-    cudaFuncSetAttribute(k_poisson, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    vx_allow_smem(k_poisson);
     // 1024 threads x 64 registers take a whole SM's register file: no block of the FP64
     // face kernels that run beside the solve shares the SM, whose FP64 unit would
     // otherwise delay the solve's dependent chain (step 32.4 -> 28.1 ms on 4096 x 512)
@@ -1386,7 +1386,7 @@ void launch_moments_poisson64(const PipeLaunch &K0) {
     const int smem_solve = base + (K.P.x_in_smem ? 8 * K.P.maxn : 0);
     const int smem = std::max(smem_solve, 2 * (int)sizeof(int) * kPipeGroups);
     auto kern = K.M.fast ? k64_moments_poisson<true> : k64_moments_poisson<false>;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    vx_allow_smem(kern);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(K.P.nruns + K.summers + K.workers);
     cfg.blockDim = dim3(1024);

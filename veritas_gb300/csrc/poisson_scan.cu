@@ -339,7 +339,7 @@ void launch_poisson_fast(const PoissonFastLaunch &L) {
     const size_t smem = poisson_scan_smem(L.maxn);
     PoissonFastLaunch P = L;
     P.scan_threads = scan_threads(L.maxn);
-    cudaFuncSetAttribute(k_poisson_scan, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    vx_allow_smem(k_poisson_scan);
     vx_launch(k_poisson_scan, L.nruns * kPsCluster, std::max(P.assemble ? kPsMaxThreads : kPsMinThreads, P.scan_threads + 32), smem, L.stream, P);
 }
 

@@ -32,6 +32,18 @@ inline void vx_launch(void (*kernel)(KP...), dim3 grid, dim3 block, size_t smem,
     cfg.numAttrs = g_launch_pdl ? 1 : 0;
     cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);  // errors surface through cudaGetLastError
 }
+// Lets `kernel` take all the dynamic shared memory an SM has beside its static.  Always the
+// same value: the limit belongs to the kernel, not to a launch, so a launch that set its own
+// size would take it from a larger one that another thread's engine is about to make.
+template <typename K>
+inline void vx_allow_smem(K *kernel) {
+    int dev = 0, optin = 0;
+    cudaFuncAttributes a{};
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    cudaFuncGetAttributes(&a, kernel);
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)a.sharedSizeBytes);
+}
 // Without the attribute: for the launch-set table kernels, queued from the host behind a
 // running step's graph (nothing to overlap with there).
 template <typename... KP, typename... A>
