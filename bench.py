@@ -42,13 +42,13 @@ MEASURED = ROOT / "MEASURED_PEAKS.json"
 
 # Compulsory DRAM bytes per padded cell of each profiled kernel (each plane read or
 # written once; stage-0 variants, which is what the profile launches).
-KERNEL_BYTES = {"gamma": 8, "faces": 48, "flux": 88, "ds_f2": 32, "limR": 48, "limC": 48, "update": 48,
+KERNEL_BYTES = {"gamma": 8, "faces": 48, "flux": 88, "ds_f2": 32, "limR": 48, "update": 48,
                 "moments": 24, "assemble": 0}
 # Algorithmic FP64 operations per padded cell (a division counts as one operation).
-KERNEL_FLOPS = {"gamma": 6, "faces": 125, "flux": 26, "ds_f2": 8, "limR": 34, "limC": 4, "update": 8,
+KERNEL_FLOPS = {"gamma": 6, "faces": 125, "flux": 26, "ds_f2": 8, "limR": 34, "update": 12,
                 "moments": 30, "assemble": 0}
 KERNEL_NAMES = {"gamma": "k64_gamma", "faces": "k64_faces", "flux": "k64_flux", "ds_f2": "k64_f2",
-                "limR": "k64_limR", "limC": "k64_limC", "update": "k64_update", "moments": "k64_moments",
+                "limR": "k64_limR", "update": "k64_cupdate", "moments": "k64_moments",
                 "assemble": "k_assemble", "poisson": "k_poisson", "maxwell": "k_maxwell*", "ghost": "k_ghost",
                 "iface": "k_iface", "csync": "k_csync", "moments_poisson": "k64_moments_poisson"}
 # The pipelined launch does the work of these three kernels (FP64 runs with the exact solve).

@@ -345,7 +345,8 @@ int vx_ctx_timer_end(vx_ctx *ctx, double *ms);
 
 /* Time the run's Vlasov kernels in isolation: reps back-to-back launches per kernel on
  * the context stream (after one untimed launch).  out_ms[k] receives the mean launch
- * time of kernel k in the order gamma, faces, flux, ds_f2, limR, limC, update,
+ * time of kernel k in the order gamma, faces, flux, ds_f2, limR, limC (0: the update's
+ * pass forms C), update,
  * moments (log table + ordered sums), assemble, poisson, maxwell, ghost, iface, csync
  * (all batches of each kind), moments_poisson (the pipelined moments + assembly + exact
  * solve launch; 0 where the run does not use it); *count is set to the number of entries

@@ -46,3 +46,16 @@ def test_autotune_times_the_step_and_changes_nothing(ctx, tmp_path, precision, f
         for ra, rb in zip(la, lb):
             assert (ra["f"][..., :2] == rb["f"][..., :2]).all()
     assert launches == 6 * SHAPES[precision] * KERNELS[precision]  # a warm-up and five timed
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [64, 32])
+def test_profile_times_the_update_of_the_step(ctx, precision):
+    """The step forms the limiter's C in the update's pass: that pass is timed, and no other."""
+    from veritas_gb300 import SolverManager
+
+    s = SolverManager(ctx, dataclasses.replace(problem_for("beam2"), precision=precision))
+    s.Advance(s.CalculateDt())
+    prof = s.profile_kernels(reps=1)
+    s.close()
+    assert prof["limC"] == 0.0 and prof["update"] > 0.0

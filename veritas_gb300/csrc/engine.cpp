@@ -646,9 +646,9 @@ std::vector<double> Engine::profile_kernels(Run &run, int reps) {
     };
     // stage-0 parameters with dt = 0 keep every kernel well defined
     // FP32 sets run the fused face + flux kernels: "faces" and "flux" time the x and p
-    // ones, "gamma" (folded into them) reads 0
-    for (int sub : {kSubGamma, kSubFaces, kSubFlux, kSubF2, kSubLimR, kSubLimC, kSubUpdate}) {
-        if (L.precision == kF32 && sub == kSubGamma) {
+    // ones, "gamma" (folded into them) reads 0; so does "limC", whose work is in the update's
+    for (int sub : {kSubGamma, kSubFaces, kSubFlux, kSubF2, kSubLimR, kSubLimC, kSubCUpdate}) {
+        if (sub == kSubLimC || (L.precision == kF32 && sub == kSubGamma)) {
             out.push_back(0.0);
             continue;
         }
