@@ -214,7 +214,7 @@ constexpr int kPipeErr = 0, kPipeTicket = 32, kPipeLeave = 64, kPipeQHead = 96, 
 // occupancy of an FP64 instruction are both about 64 cycles).  All 15 at a time held the
 // item for four times as long, which small sets and every forward sweep's first chunk wait
 // for: step of 50 x 38 in two levels 0.99 -> 0.78 ms, of 2048 x 256 3.94 -> 3.87 ms, 512 x
-// 128 with ions 68.3 -> 64.0 ms per 23 steps, 4096 x 512 in two levels the same.
+// 128 with ions 68.3 -> 64.0 ms per 22 steps and a regrid, 4096 x 512 in two levels the same.
 constexpr int kPipeCols = 4, kPipeParts = (kMomCols + kPipeCols - 1) / kPipeCols;
 // Groups per worker block: the second covers the first's loads and barriers (one, two,
 // four, eight: 4096 x 512 15.5, 14.95, 14.94, 14.94 ms, 512 x 128 68.4, 64.0, 64.8, 69.2);
